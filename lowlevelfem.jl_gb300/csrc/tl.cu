@@ -4,23 +4,31 @@
 // :2738-2910), with the hyperelastic laws in closed form (the reference
 // differentiates psi with Tensors.jl, ext/LowLevelFEMTensorsExt.jl:9-60).
 //
-// One CTA per element at a time.  Phase A (threads over integration points):
+// A CTA works on one element (k_tl_matrix) or on several small ones at once
+// (k_tl_packed, k_tl_force).  Phase A (threads over integration points):
 // Jacobian inverse, weight, interpolated F (or S, C), law -> PK2 stress S and
 // 6x6 Voigt tangent D, all kept in shared memory.  Phase B (per point):
 // physical gradients g, B(F) (6x3 per node) and T = w D B staged for all
 // nodes, then every thread accumulates the 3x3 blocks of its node pairs
-// (upper triangle; pairs processed in tiles of PPT per thread so the
+// (upper triangle; in k_tl_matrix in tiles of PPT per thread so the
 // accumulators stay in registers).  Blocks go to the same pair buffer and
 // element-ordered gather as the linear operators.
 // Arithmetic contract: identical, operation by operation, to the oracle's
 // TL restatement (intrinsics only; ln by the atanh series of the oracle).
 #include "common.cuh"
 
+#include <algorithm>
+
 namespace {
 
 constexpr int TL_THREADS = 128;
-constexpr int QD = 64;  // per-point record: wq, invJ[9], F or S [9], D[36], S[9] (tangent)
-enum { TL_KMAT = 0, TL_KGEO_S = 1, TL_KGEO_C = 2, TL_KTAN = 3 };
+constexpr int TLP_THREADS = 384;  // most threads of k_tl_packed: hex27's 378 node pairs
+// per-point record: wq, invJ[9], F or S [9], D[36], S[9] (tangent); an odd
+// stride, so that the threads of the point phase write to different banks
+constexpr int QD = 65;
+constexpr int QF = 19;  // the internal force's record: wq, invJ[9], P[9]
+// TL_FORCE: F in, first Piola-Kirchhoff stress out (internal force)
+enum { TL_KMAT = 0, TL_KGEO_S = 1, TL_KGEO_C = 2, TL_KTAN = 3, TL_FORCE = 4 };
 
 struct TLArgs {
   const double *xyz;
@@ -53,11 +61,13 @@ __device__ double tl_ln(double x) {
   return __fma_rn((double)e, 0.69314718055994530942, __dmul_rn(2.0, __dmul_rn(s, p)));
 }
 
-// S (3x3) and D (6x6 row-major) from C; false if det C <= 0.
+// S (3x3) and, WITH_D, D (6x6 row-major) from C; false if det C <= 0.
+template <bool WITH_D>
 __device__ bool tl_law(int law, const double *prm, const double C[3][3], double S[3][3], double *D) {
   if (law == LLF_LAW_CONSTANT_C) {
-    for (int a = 0; a < 6; ++a)
-      for (int b = 0; b < 6; ++b) D[a * 6 + b] = prm[b * 6 + a];
+    if constexpr (WITH_D)
+      for (int a = 0; a < 6; ++a)
+        for (int b = 0; b < 6; ++b) D[a * 6 + b] = prm[b * 6 + a];
     for (int i = 0; i < 3; ++i)
       for (int j = 0; j < 3; ++j) S[i][j] = 0.0;
     return true;
@@ -70,13 +80,14 @@ __device__ bool tl_law(int law, const double *prm, const double C[3][3], double 
     double trE = __dadd_rn(__dadd_rn(E[0][0], E[1][1]), E[2][2]);
     for (int i = 0; i < 3; ++i)
       for (int j = 0; j < 3; ++j) S[i][j] = __fma_rn(lam, i == j ? trE : 0.0, __dmul_rn(__dmul_rn(2.0, mu), E[i][j]));
-    for (int a = 0; a < 6; ++a)
-      for (int b = 0; b < 6; ++b) {
-        int I = VI[a], J = VJ[a], K = VI[b], L = VJ[b];
-        double v = __dmul_rn(lam, (I == J && K == L) ? 1.0 : 0.0);
-        v = __dadd_rn(v, __dmul_rn(mu, __dadd_rn((I == K && J == L) ? 1.0 : 0.0, (I == L && J == K) ? 1.0 : 0.0)));
-        D[a * 6 + b] = v;
-      }
+    if constexpr (WITH_D)
+      for (int a = 0; a < 6; ++a)
+        for (int b = 0; b < 6; ++b) {
+          int I = VI[a], J = VJ[a], K = VI[b], L = VJ[b];
+          double v = __dmul_rn(lam, (I == J && K == L) ? 1.0 : 0.0);
+          v = __dadd_rn(v, __dmul_rn(mu, __dadd_rn((I == K && J == L) ? 1.0 : 0.0, (I == L && J == K) ? 1.0 : 0.0)));
+          D[a * 6 + b] = v;
+        }
     return true;
   }
   double c00 = __dsub_rn(__dmul_rn(C[1][1], C[2][2]), __dmul_rn(C[1][2], C[2][1]));
@@ -99,13 +110,22 @@ __device__ bool tl_law(int law, const double *prm, const double C[3][3], double 
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j)
       S[i][j] = __fma_rn(t, Ci[i][j], __dmul_rn(mu, __dsub_rn(i == j ? 1.0 : 0.0, Ci[i][j])));
-  double m2 = __dsub_rn(mu, t);
-  for (int a = 0; a < 6; ++a)
-    for (int b = 0; b < 6; ++b) {
-      int I = VI[a], J = VJ[a], K = VI[b], L = VJ[b];
-      double sym = __dadd_rn(__dmul_rn(Ci[I][K], Ci[J][L]), __dmul_rn(Ci[I][L], Ci[J][K]));
-      D[a * 6 + b] = __fma_rn(lam, __dmul_rn(Ci[I][J], Ci[K][L]), __dmul_rn(m2, sym));
-    }
+  // C = F^T F is symmetric bit for bit (its products commute), so C^-1 and D
+  // are too: the upper triangle of D, mirrored
+  if constexpr (WITH_D) {
+    const double m2 = __dsub_rn(mu, t);
+#pragma unroll
+    for (int a = 0; a < 6; ++a)
+#pragma unroll
+      for (int b = a; b < 6; ++b) {
+        constexpr int WI[6] = {0, 1, 2, 1, 0, 0}, WJ[6] = {0, 1, 2, 2, 2, 1};
+        const int I = WI[a], J = WJ[a], K = WI[b], L = WJ[b];
+        const double sym = __dadd_rn(__dmul_rn(Ci[I][K], Ci[J][L]), __dmul_rn(Ci[I][L], Ci[J][K]));
+        const double v = __fma_rn(lam, __dmul_rn(Ci[I][J], Ci[K][L]), __dmul_rn(m2, sym));
+        D[a * 6 + b] = v;
+        D[b * 6 + a] = v;
+      }
+  }
   return true;
 }
 
@@ -121,18 +141,26 @@ __device__ __forceinline__ void pair_dec(int pi, int npe, int &a, int &b) {
 }
 
 // Phase A for one point: wq, invJ, and the tensors the mode needs.
-// Layout of rec: [0] wq, [1..9] invJ, [10..18] F (KMAT) or S, [19..54] D.
-__device__ void tl_point(const TLArgs &A, int mode, int q, const double *sX, const double *sT,
-                         double *rec) {
+// Layout of rec: [0] wq, [1..9] invJ, [10..18] F (KMAT, KTAN), S (KGEO) or
+// P (FORCE), [19..54] D, [55..63] S (KTAN).
+template <int mode>
+__device__ __forceinline__ void tl_point(const TLArgs &A, int q, const double *sX, const double *sT, double *rec) {
   const int npe = A.npe;
   const double *dNq = A.dN + (size_t)q * npe * 3;
   double J[3][3];
+#pragma unroll
   for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) {
-      double acc = 0.0;
-      for (int a = 0; a < npe; ++a) acc = __fma_rn(sX[a * 3 + i], __ldg(dNq + a * 3 + j), acc);
-      J[i][j] = acc;
-    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) J[i][j] = 0.0;
+  for (int a = 0; a < npe; ++a) {  // nine independent chains, each in node order
+    double d[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) d[j] = __ldg(dNq + a * 3 + j);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) J[i][j] = __fma_rn(sX[a * 3 + i], d[j], J[i][j]);
+  }
   double c00 = __dsub_rn(__dmul_rn(J[1][1], J[2][2]), __dmul_rn(J[1][2], J[2][1]));
   double c01 = -__dsub_rn(__dmul_rn(J[1][0], J[2][2]), __dmul_rn(J[1][2], J[2][0]));
   double c02 = __dsub_rn(__dmul_rn(J[1][0], J[2][1]), __dmul_rn(J[1][1], J[2][0]));
@@ -152,44 +180,79 @@ __device__ void tl_point(const TLArgs &A, int mode, int q, const double *sX, con
   // interpolated nodal tensor (column-major per node)
   const double *Nq = A.N + (size_t)q * npe;
   double Tq[3][3];
+#pragma unroll
   for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) {
-      double acc = 0.0;
-      for (int a = 0; a < npe; ++a) acc = __fma_rn(__ldg(Nq + a), sT[9 * a + 3 * j + i], acc);
-      Tq[i][j] = acc;
-    }
-  if (mode == TL_KGEO_S) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) Tq[i][j] = 0.0;
+  for (int a = 0; a < npe; ++a) {
+    const double na = __ldg(Nq + a);
+#pragma unroll
     for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) Tq[i][j] = __fma_rn(na, sT[9 * a + 3 * j + i], Tq[i][j]);
+  }
+  if (mode == TL_KGEO_S) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
       for (int j = 0; j < 3; ++j) rec[10 + 3 * i + j] = Tq[i][j];
     return;
   }
   double C[3][3];
-  if (mode == TL_KMAT || mode == TL_KTAN) {
+  if (mode != TL_KGEO_C) {
+#pragma unroll
     for (int I = 0; I < 3; ++I)
+#pragma unroll
       for (int J2 = 0; J2 < 3; ++J2) {
         double acc = 0.0;
+#pragma unroll
         for (int k = 0; k < 3; ++k) acc = __fma_rn(Tq[k][I], Tq[k][J2], acc);
         C[I][J2] = acc;
       }
-    for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j) rec[10 + 3 * i + j] = Tq[i][j];  // F
   } else {
+#pragma unroll
     for (int i = 0; i < 3; ++i)
+#pragma unroll
       for (int j = 0; j < 3; ++j) C[i][j] = Tq[i][j];
   }
+  constexpr bool with_d = mode == TL_KMAT || mode == TL_KTAN;
+  if (with_d)
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) rec[10 + 3 * i + j] = Tq[i][j];  // F
   double S[3][3];
-  if (!tl_law(A.law, A.prm, C, S, rec + 19)) atomicOr(A.status, ST_NONFINITE);
-  if (mode == TL_KGEO_C)
+  if (!tl_law<with_d>(A.law, A.prm, C, S, rec + 19)) {
+    atomicOr(A.status, ST_NONFINITE);
+#pragma unroll
     for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j) rec[10 + 3 * i + j] = S[i][j];
-  if (mode == TL_KTAN)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) S[i][j] = 0.0;
+  }
+  if (mode == TL_FORCE) {
+#pragma unroll
     for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j) rec[55 + 3 * i + j] = S[i][j];
+#pragma unroll
+      for (int J2 = 0; J2 < 3; ++J2) {
+        double s = 0.0;
+#pragma unroll
+        for (int K = 0; K < 3; ++K) s = __fma_rn(Tq[i][K], S[K][J2], s);
+        rec[10 + 3 * i + J2] = s;  // P
+      }
+  }
+  if (mode == TL_KGEO_C || mode == TL_KTAN) {
+    constexpr int at = mode == TL_KTAN ? 55 : 10;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) rec[at + 3 * i + j] = S[i][j];
+  }
 }
 
-template <int MODE, int PPT>
+template <int MODE>
 __global__ void __launch_bounds__(TL_THREADS) k_tl_matrix(TLArgs A) {
   extern __shared__ double sm[];
+  constexpr int PPT = 4;                   // node pairs per thread of a tile
   const int npe = A.npe, nip = A.nip;
   double *sX = sm;                         // npe*3
   double *sT = sX + npe * 3;               // npe*9
@@ -205,7 +268,7 @@ __global__ void __launch_bounds__(TL_THREADS) k_tl_matrix(TLArgs A) {
       sX[t] = A.xyz[(size_t)A.conn[e * npe + t / 3] * 3 + t % 3];
     for (int t = threadIdx.x; t < npe * 9; t += blockDim.x) sT[t] = A.T[(size_t)e * npe * 9 + t];
     __syncthreads();
-    for (int q = threadIdx.x; q < nip; q += blockDim.x) tl_point(A, MODE, q, sX, sT, qd + (size_t)q * QD);
+    for (int q = threadIdx.x; q < nip; q += blockDim.x) tl_point<MODE>(A, q, sX, sT, qd + (size_t)q * QD);
     __syncthreads();
     double *Ke = A.out + (size_t)e * npe * npe * BS;  // [column node][row node][block]
     const int tile = blockDim.x * PPT;
@@ -331,60 +394,189 @@ __global__ void __launch_bounds__(TL_THREADS) k_tl_matrix(TLArgs A) {
   }
 }
 
-// Internal force: element vectors fe[e][a][i].
-template <int MODE>  // 0: T = F with law, 1: T = P
-__global__ void __launch_bounds__(TL_THREADS) k_tl_force(TLArgs A) {
+// The same element matrices for elements of up to 384 node pairs, E of them
+// per CTA (e0 .. e0+E-1), so that the lanes of every phase are filled: the
+// FP64 pipe, which bounds this kernel, is spent per warp instruction, however
+// few lanes take part.  One element per 128-thread CTA used 36 lanes of hex8's
+// pair loop and 8 of its point phase.  Phases: the points of all elements,
+// then the physical gradients at all points, then per point B(F) (with
+// T = w D B and S g, which depend on one node only, staged once per node
+// instead of once per pair) and the node pairs, one per thread.  hex8,
+// 29,760 elements: 4.14 -> 1.71 ms (31,000 FP64 lane operations per element
+// at 608 G/s take 1.5 ms).
+// Shared memory (doubles): sX [E npe 3] | qd [E nip QD] | sG [E nip npe 3] |
+// stage [E npe 39], which starts as sT [E npe 9].
+template <int MODE>
+__global__ void __launch_bounds__(TLP_THREADS, 2) k_tl_packed(TLArgs A, int E) {
   extern __shared__ double sm[];
   const int npe = A.npe, nip = A.nip;
+  constexpr bool MAT = (MODE == TL_KMAT || MODE == TL_KTAN);
+  constexpr int BS = MAT ? 9 : 1;
   double *sX = sm;
-  double *sT = sX + npe * 3;
-  double *qd = sT + npe * 9;  // per point: wq, invJ[9], P[9]
-  for (int64_t e = blockIdx.x; e < A.nel; e += gridDim.x) {
-    for (int t = threadIdx.x; t < npe * 3; t += blockDim.x)
-      sX[t] = A.xyz[(size_t)A.conn[e * npe + t / 3] * 3 + t % 3];
-    for (int t = threadIdx.x; t < npe * 9; t += blockDim.x) sT[t] = A.T[(size_t)e * npe * 9 + t];
+  double *qd = sX + (size_t)E * npe * 3;
+  double *sG = qd + (size_t)E * nip * QD;
+  double *sS = sG + (size_t)E * nip * npe * 3;   // S g  [E npe 3]
+  double *sB = sS + (size_t)E * npe * 3;         // B    [E npe 18]
+  double *sTb = sB + (size_t)E * npe * 18;       // w D B [E npe 18]
+  double *sT = sS;
+  // this thread's node pair
+  const int el = threadIdx.x / A.npairs;
+  int a = 0, b = 0;
+  if (el < E) pair_dec(threadIdx.x - el * A.npairs, npe, a, b);
+  for (int64_t e0 = (int64_t)blockIdx.x * E; e0 < A.nel; e0 += (int64_t)gridDim.x * E) {
+    const int ne = (int)(A.nel - e0 < E ? A.nel - e0 : E);
+    for (int t = threadIdx.x; t < ne * npe * 3; t += blockDim.x)
+      sX[t] = A.xyz[(size_t)A.conn[e0 * npe + t / 3] * 3 + t % 3];
+    for (int t = threadIdx.x; t < ne * npe * 9; t += blockDim.x) sT[t] = A.T[(size_t)e0 * npe * 9 + t];
     __syncthreads();
-    for (int q = threadIdx.x; q < nip; q += blockDim.x) {
-      double *rec = qd + (size_t)q * QD;
-      tl_point(A, MODE == 0 ? TL_KMAT : TL_KGEO_S, q, sX, sT, rec);
-      // rec[10..18] holds F (MODE 0) or the interpolated P (MODE 1)
-      if (MODE == 0) {
-        double F[3][3], C[3][3], S[3][3], D[36];
-        for (int i = 0; i < 3; ++i)
-          for (int j = 0; j < 3; ++j) F[i][j] = rec[10 + 3 * i + j];
-        for (int I = 0; I < 3; ++I)
-          for (int J2 = 0; J2 < 3; ++J2) {
-            double acc = 0.0;
-            for (int k = 0; k < 3; ++k) acc = __fma_rn(F[k][I], F[k][J2], acc);
-            C[I][J2] = acc;
-          }
-        if (!tl_law(A.law, A.prm, C, S, D)) atomicOr(A.status, ST_NONFINITE);
-        for (int i = 0; i < 3; ++i)
-          for (int J2 = 0; J2 < 3; ++J2) {
+    for (int t = threadIdx.x; t < ne * nip; t += blockDim.x) {
+      const int k = t / nip;
+      if (A.emat && A.emat[e0 + k] < 0) continue;
+      tl_point<MODE>(A, t - k * nip, sX + (size_t)k * npe * 3, sT + (size_t)k * npe * 9, qd + (size_t)t * QD);
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < ne * nip * npe; t += blockDim.x) {
+      const int p = t / npe, q = p % nip;   // point of the CTA, of its element
+      const double *inv = qd + (size_t)p * QD + 1, *d = A.dN + ((size_t)q * npe + (t - p * npe)) * 3;
+      const double d0 = __ldg(d), d1 = __ldg(d + 1), d2 = __ldg(d + 2);
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        sG[(size_t)t * 3 + i] = __fma_rn(inv[6 + i], d2, __fma_rn(inv[3 + i], d1, __fma_rn(inv[i], d0, 0.0)));
+    }
+    const bool live = el < ne && !(A.emat && A.emat[e0 + el] < 0);
+    double acc[BS];
+#pragma unroll
+    for (int m = 0; m < BS; ++m) acc[m] = 0.0;
+    for (int q = 0; q < nip; ++q) {
+      __syncthreads();   // the gradients (q = 0), the pairs' reads of the last point
+      for (int t = threadIdx.x; t < ne * npe * 3; t += blockDim.x) {
+        const int n = t / 3, j = t - 3 * n, k = n / npe;   // node of the CTA, component, element
+        const double *rec = qd + ((size_t)k * nip + q) * QD;
+        const double *g = sG + (((size_t)k * nip + q) * npe + (n - k * npe)) * 3;
+        const double g0 = g[0], g1 = g[1], g2 = g[2];
+        if (MAT) {  // column j of B(F) (src/nonlinear.jl:2219-2242) and of w D B
+          const double *F = rec + 10 + 3 * j, *D = rec + 19;
+          const double v1 = F[0], v2 = F[1], v3 = F[2];
+          double Bc[6];
+          Bc[0] = __dmul_rn(v1, g0);
+          Bc[1] = __dmul_rn(v2, g1);
+          Bc[2] = __dmul_rn(v3, g2);
+          Bc[3] = __dadd_rn(__dmul_rn(v2, g2), __dmul_rn(v3, g1));
+          Bc[4] = __dadd_rn(__dmul_rn(v1, g2), __dmul_rn(v3, g0));
+          Bc[5] = __dadd_rn(__dmul_rn(v1, g1), __dmul_rn(v2, g0));
+          const double wq = rec[0];
+#pragma unroll
+          for (int I = 0; I < 6; ++I) {
             double s = 0.0;
-            for (int K = 0; K < 3; ++K) s = __fma_rn(F[i][K], S[K][J2], s);
-            rec[10 + 3 * i + J2] = s;  // P
+#pragma unroll
+            for (int J2 = 0; J2 < 6; ++J2) s = __fma_rn(D[I * 6 + J2], Bc[J2], s);
+            sB[(size_t)n * 18 + I * 3 + j] = Bc[I];
+            sTb[(size_t)n * 18 + I * 3 + j] = __dmul_rn(s, wq);
           }
+        }
+        if (MODE != TL_KMAT) {  // row j of S g
+          const double *S = rec + (MODE == TL_KTAN ? 55 : 10) + 3 * j;
+          sS[(size_t)n * 3 + j] = __fma_rn(S[2], g2, __fma_rn(S[1], g1, __fma_rn(S[0], g0, 0.0)));
+        }
+      }
+      __syncthreads();
+      if (live) {
+        const size_t na = (size_t)el * npe + a, nb = (size_t)el * npe + b;
+        if (MAT) {
+          const double *Ba = sB + na * 18, *Tb = sTb + nb * 18;
+#pragma unroll
+          for (int I = 0; I < 6; ++I) {
+            double x[3], y[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+              x[i] = Ba[I * 3 + i];
+              y[i] = Tb[I * 3 + i];
+            }
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+              for (int j = 0; j < 3; ++j) acc[i * 3 + j] = __fma_rn(x[i], y[j], acc[i * 3 + j]);
+          }
+        }
+        if (MODE != TL_KMAT) {  // geometric part
+          const double *ga = sG + (((size_t)el * nip + q) * npe + a) * 3, *tv = sS + nb * 3;
+          const double wq = qd[((size_t)el * nip + q) * QD];
+          const double v = __fma_rn(ga[2], tv[2], __fma_rn(ga[1], tv[1], __fma_rn(ga[0], tv[0], 0.0)));
+          if (MAT) {
+#pragma unroll
+            for (int i = 0; i < 3; ++i) acc[i * 3 + i] = __fma_rn(v, wq, acc[i * 3 + i]);
+          } else {
+            acc[0] = __fma_rn(v, wq, acc[0]);
+          }
+        }
+      }
+    }
+    if (live) {
+      double *Ke = A.out + (size_t)(e0 + el) * npe * npe * BS;  // [column node][row node][block]
+      double *ab = Ke + ((size_t)b * npe + a) * BS;   // block (a,b)
+      double *ba = Ke + ((size_t)a * npe + b) * BS;   // mirror (b,a)
+      if (MAT) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            const double v = (a == b && j < i) ? acc[j * 3 + i] : acc[i * 3 + j];
+            ab[i * 3 + j] = v;
+            if (a != b) ba[j * 3 + i] = v;
+          }
+      } else {
+        ab[0] = acc[0];
+        if (a != b) ba[0] = acc[0];
       }
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < npe * 3; t += blockDim.x) {
-      const int a = t / 3, i = t % 3;
-      double fe = 0.0;
+  }
+}
+
+// Internal force: element vectors fe[e][a][i], E elements per CTA (the
+// points of small elements fill whole warps: hex8 took 8 lanes of 128 one
+// element at a time).  A point's record holds only w, J^-1 and P, and a
+// thread makes the three components of a node, so that the node's physical
+// gradient is formed once per point.  hex8, 29,760 elements: 1.49 -> 0.25 ms;
+// hex125, 576 elements: 1.46 -> 0.68 ms.
+template <int MODE>  // TL_FORCE: T = F with law, TL_KGEO_S: T = P
+__global__ void __launch_bounds__(TL_THREADS) k_tl_force(TLArgs A, int E) {
+  extern __shared__ double sm[];
+  const int npe = A.npe, nip = A.nip;
+  double *sX = sm;
+  double *sT = sX + (size_t)E * npe * 3;
+  double *qd = sT + (size_t)E * npe * 9;
+  for (int64_t e0 = (int64_t)blockIdx.x * E; e0 < A.nel; e0 += (int64_t)gridDim.x * E) {
+    const int ne = (int)(A.nel - e0 < E ? A.nel - e0 : E);
+    for (int t = threadIdx.x; t < ne * npe * 3; t += blockDim.x)
+      sX[t] = A.xyz[(size_t)A.conn[e0 * npe + t / 3] * 3 + t % 3];
+    for (int t = threadIdx.x; t < ne * npe * 9; t += blockDim.x) sT[t] = A.T[(size_t)e0 * npe * 9 + t];
+    __syncthreads();
+    for (int t = threadIdx.x; t < ne * nip; t += blockDim.x) {
+      const int k = t / nip;
+      tl_point<MODE>(A, t - k * nip, sX + (size_t)k * npe * 3, sT + (size_t)k * npe * 9, qd + (size_t)t * QF);
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < ne * npe; t += blockDim.x) {
+      const int k = t / npe, a = t - k * npe;
+      double fe[3] = {0.0, 0.0, 0.0};
       for (int q = 0; q < nip; ++q) {
-        const double *rec = qd + (size_t)q * QD;
+        const double *rec = qd + ((size_t)k * nip + q) * QF;
         const double *d = A.dN + ((size_t)q * npe + a) * 3;
+        const double d0 = __ldg(d), d1 = __ldg(d + 1), d2 = __ldg(d + 2);
         double g[3];
-        for (int c = 0; c < 3; ++c) {
-          double s = 0.0;
-          for (int j = 0; j < 3; ++j) s = __fma_rn(rec[1 + 3 * j + c], __ldg(d + j), s);
-          g[c] = s;
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          g[c] = __fma_rn(rec[7 + c], d2, __fma_rn(rec[4 + c], d1, __fma_rn(rec[1 + c], d0, 0.0)));
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const double *P = rec + 10 + 3 * i;
+          const double v = __fma_rn(P[2], g[2], __fma_rn(P[1], g[1], __fma_rn(P[0], g[0], 0.0)));
+          fe[i] = __fma_rn(v, rec[0], fe[i]);
         }
-        double v = 0.0;
-        for (int J2 = 0; J2 < 3; ++J2) v = __fma_rn(rec[10 + 3 * i + J2], g[J2], v);
-        fe = __fma_rn(v, rec[0], fe);
       }
-      A.out[(size_t)e * npe * 3 + t] = fe;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) A.out[((size_t)e0 * npe + t) * 3 + i] = fe[i];
     }
     __syncthreads();
   }
@@ -501,7 +693,7 @@ __global__ void __launch_bounds__(TL_THREADS) k_tl_points_tc(TLArgs A, float *pd
       sX[t] = A.xyz[(size_t)A.conn[e * npe + t / 3] * 3 + t % 3];
     for (int t = threadIdx.x; t < npe * 9; t += blockDim.x) sT[t] = A.T[(size_t)e * npe * 9 + t];
     __syncthreads();
-    for (int q = threadIdx.x; q < nip; q += blockDim.x) tl_point(A, TL_KTAN, q, sX, sT, rec + (size_t)q * QD);
+    for (int q = threadIdx.x; q < nip; q += blockDim.x) tl_point<TL_KTAN>(A, q, sX, sT, rec + (size_t)q * QD);
     __syncthreads();
     float *out = pd + (size_t)e * nip * ps;
     for (int t = threadIdx.x; t < nip * ps; t += blockDim.x) {
@@ -713,10 +905,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tl_tangent_tc(TcArgs A) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
 }
 
-size_t tl_smem(int npe, int nip, bool matrix) {
-  size_t d = (size_t)npe * 3 + (size_t)npe * 9 + (size_t)nip * QD;
-  if (matrix) d += (size_t)npe * 3 + (size_t)npe * 18 * 2;
-  return d * sizeof(double);
+size_t tl_smem(int npe, int nip) {
+  return sizeof(double) * ((size_t)npe * 12 + (size_t)nip * QD + (size_t)npe * 39);
 }
 
 int fill_args(llf_ctx *ctx, llf_mesh *mesh, const double *T, int law, const double *params,
@@ -746,26 +936,52 @@ int fill_args(llf_ctx *ctx, llf_mesh *mesh, const double *T, int law, const doub
   return LLF_OK;
 }
 
+// Elements per CTA of k_tl_packed: the count whose node pairs fill their
+// warps best within TLP_THREADS threads and 110 KB of shared memory (two
+// CTAs per SM), the larger one of equals; 0 when one element does not fit.
+int packed_elements(const TLArgs &a, size_t per_elem) {
+  int best = 0;
+  double fill = 0.0;
+  for (int E = 1; E * a.npairs <= TLP_THREADS && E * per_elem <= 110 * 1024; ++E) {
+    const double f = (double)(E * a.npairs) / ((E * a.npairs + 31) / 32 * 32);
+    if (f >= fill) {
+      fill = f;
+      best = E;
+    }
+  }
+  return best;
+}
+
 template <int MODE>
 int launch_matrix(llf_ctx *ctx, TLArgs a, size_t smem) {
-  int ppt = (a.npairs + TL_THREADS - 1) / TL_THREADS;
-  ppt = ppt <= 1 ? 1 : (ppt <= 2 ? 2 : 4);
-  int per_sm = 1;
-  auto pick = [&](auto fn) -> int {
-    if (smem > 48 * 1024)
-      LLF_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    LLF_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, TL_THREADS, smem));
-    if (per_sm < 1) per_sm = 1;
-    int64_t grid = (int64_t)ctx->num_sms * per_sm;
-    if (grid > a.nel) grid = a.nel > 0 ? a.nel : 1;
-    KernelScope ks(ctx, MODE == TL_KMAT ? "k_tl_material" : (MODE == TL_KTAN ? "k_tl_tangent" : "k_tl_geometric"));
-    fn<<<(unsigned)grid, TL_THREADS, smem, ctx->stream>>>(a);
+  const char *name = MODE == TL_KMAT ? "k_tl_material" : (MODE == TL_KTAN ? "k_tl_tangent" : "k_tl_geometric");
+  const size_t per_elem = sizeof(double) * ((size_t)a.npe * 3 + (size_t)a.nip * QD + (size_t)a.nip * a.npe * 3 +
+                                            (size_t)a.npe * 39);
+  if (const int E = packed_elements(a, per_elem)) {
+    auto fn = k_tl_packed<MODE>;
+    const size_t sp = E * per_elem;
+    const int threads = (E * a.npairs + 31) / 32 * 32;
+    if (sp > 48 * 1024)
+      LLF_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp));
+    int per_sm = 1;
+    LLF_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, sp));
+    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->num_sms * std::max(per_sm, 1),
+                                                                (a.nel + E - 1) / E));
+    KernelScope ks(ctx, name);
+    fn<<<(unsigned)grid, threads, sp, ctx->stream>>>(a, E);
     LLF_CUDA_TRY(ctx, cudaGetLastError());
     return LLF_OK;
-  };
-  if (ppt == 1) return pick(k_tl_matrix<MODE, 1>);
-  if (ppt == 2) return pick(k_tl_matrix<MODE, 2>);
-  return pick(k_tl_matrix<MODE, 4>);
+  }
+  auto fn = k_tl_matrix<MODE>;
+  if (smem > 48 * 1024)
+    LLF_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per_sm = 1;
+  LLF_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, TL_THREADS, smem));
+  const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->num_sms * std::max(per_sm, 1), a.nel));
+  KernelScope ks(ctx, name);
+  fn<<<(unsigned)grid, TL_THREADS, smem, ctx->stream>>>(a);
+  LLF_CUDA_TRY(ctx, cudaGetLastError());
+  return LLF_OK;
 }
 
 int tl_matrix(llf_ctx *ctx, llf_mesh *mesh, llf_pattern *pat, int mode, const double *dT, int law,
@@ -775,7 +991,7 @@ int tl_matrix(llf_ctx *ctx, llf_mesh *mesh, llf_pattern *pat, int mode, const do
   TLArgs a{};
   int rc = fill_args(ctx, mesh, dT, law, params, nparams, a);
   if (rc) return rc;
-  size_t smem = tl_smem(mesh->npe, mesh->nip, true);
+  size_t smem = tl_smem(mesh->npe, mesh->nip);
   if (smem > 200 * 1024) return llf_fail(ctx, LLF_ERR_LIMIT, "element too large for the TL kernels");
   const bool mat = (mode == TL_KMAT || mode == TL_KTAN);
   const int BS = mat ? 9 : 1;
@@ -948,7 +1164,12 @@ int tl_internal_force_impl(llf_ctx *ctx, llf_mesh *mesh, const double *d_P, cons
     rc = fill_args(ctx, mesh, d_F, law, params, nparams, a);
   }
   if (rc) return rc;
-  size_t smem = tl_smem(mesh->npe, mesh->nip, false);
+  // elements per CTA: as many as fill the CTA's threads with points and nodes
+  const size_t per_elem = sizeof(double) * ((size_t)mesh->npe * 12 + (size_t)mesh->nip * QF);
+  const int E = std::max(1, std::min<int>(TL_THREADS / std::max(mesh->npe, mesh->nip),
+                                          (int)((100 * 1024) / per_elem)));
+  const size_t smem = E * per_elem;
+  if (smem > 200 * 1024) return llf_fail(ctx, LLF_ERR_LIMIT, "element too large for the TL kernels");
   double *fe = nullptr;
   LLF_CUDA_TRY(ctx, dalloc(ctx, &fe, (size_t)mesh->nel * mesh->npe * 3));
   a.out = fe;
@@ -957,14 +1178,14 @@ int tl_internal_force_impl(llf_ctx *ctx, llf_mesh *mesh, const double *d_P, cons
       LLF_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 1;
     LLF_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, TL_THREADS, smem));
-    int64_t grid = (int64_t)ctx->num_sms * (per_sm < 1 ? 1 : per_sm);
-    if (grid > a.nel) grid = a.nel > 0 ? a.nel : 1;
+    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->num_sms * std::max(per_sm, 1),
+                                                                (mesh->nel + E - 1) / E));
     KernelScope ks(ctx, "k_tl_force");
-    fn<<<(unsigned)grid, TL_THREADS, smem, ctx->stream>>>(a);
+    fn<<<(unsigned)grid, TL_THREADS, smem, ctx->stream>>>(a, E);
     LLF_CUDA_TRY(ctx, cudaGetLastError());
     return LLF_OK;
   };
-  rc = d_P ? go(k_tl_force<1>) : go(k_tl_force<0>);
+  rc = d_P ? go(k_tl_force<TL_KGEO_S>) : go(k_tl_force<TL_FORCE>);
   if (rc == LLF_OK) {
     LLF_CUDA_TRY(ctx, cudaMemsetAsync(d_f, 0, sizeof(double) * 3 * mesh->non, ctx->stream));
     rc = node_gather(ctx, mesh->d_conn, mesh->nel, mesh->npe, mesh->non, 3, fe, d_f);
