@@ -1082,7 +1082,7 @@ int llf_matrix_destroy(llf_ctx *ctx, llf_matrix *m) {
   if (!m) return LLF_OK;
   if (ctx) {
     dfree(ctx, m->d_nz); dfree(ctx, m->d_diag); dfree(ctx, m->d_colptr_s);
-    dfree(ctx, m->d_rowval_s); dfree(ctx, m->d_nzval_s);
+    dfree(ctx, m->d_rowval_s); dfree(ctx, m->d_nzval_s); dfree(ctx, m->d_keep);
     cudaStreamSynchronize(ctx->stream);
   }
   delete m;

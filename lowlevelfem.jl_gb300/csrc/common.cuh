@@ -183,6 +183,7 @@ struct StoredSpec {
   int64_t *rowval_s = nullptr;     // 1-based rows, total entries
   double *nzval_s = nullptr;
   unsigned *mismatch = nullptr;    // device: set when a column's stored count differs
+  uint2 *keep = nullptr;           // keep bits of the columns (llf_matrix::d_keep)
   double **nz_slot = nullptr;
   int64_t *cnt_fallback = nullptr;
   bool fell_back = false;
@@ -202,7 +203,27 @@ struct llf_matrix {
   int64_t *d_colptr_s = nullptr;  // ndof+1
   int64_t *d_rowval_s = nullptr;  // nnz_s
   double *d_nzval_s = nullptr;    // nnz_s
+  // written with a stored CSC that went into a kept layout: which structural
+  // entries of a column are stored.  Column c (structural start s) holds a
+  // pair of words per 64 entries at keep_pos(s, c): entry i of the 64 is bit
+  // i / 2 of word x (i even) or y (i odd).
+  uint2 *d_keep = nullptr;
 };
+
+// First keep word pair of column c, whose structural entries start at s, and
+// the pairs of a pattern: s / 64 + c leaves every column its ceil(len / 64).
+__host__ __device__ __forceinline__ int64_t keep_pos(int64_t s, int64_t c) { return (s >> 6) + c; }
+inline int64_t keep_words(int64_t nnz, int64_t ndof) { return (nnz >> 6) + ndof + 1; }
+#ifdef __CUDACC__
+// The stored entries among the 64 before entry i of them, and whether entry
+// i is stored (0 <= i < 64).
+__device__ __forceinline__ int keep_rank(uint2 w, int i, bool &kept) {
+  const int q = i >> 1, odd = i & 1;
+  const unsigned below = (1u << q) - 1u, ex = (w.x >> q) & 1u, ey = (w.y >> q) & 1u;
+  kept = odd ? ey : ex;
+  return __popc(w.x & below) + __popc(w.y & below) + (odd ? (int)ex : 0);
+}
+#endif
 
 // ---------------------------------------------------------------- helpers
 #define LLF_CUDA_TRY(ctx, expr)                                            \
@@ -290,9 +311,10 @@ int autotune_impl(llf_ctx *ctx, llf_mesh *mesh, llf_pattern *pat, int kind, int 
 int matrix_finalize(llf_ctx *ctx, llf_matrix *m, int64_t *counts, int64_t **ptr0_out = nullptr);
 // frees the pattern's stored layouts (assemble.cu)
 void pattern_free_layouts(llf_ctx *ctx, llf_pattern *pat);
-// The structural values of m, expanded from its stored CSC if the assembly
-// left them out (assemble.cu): the stored entries at their structural
-// positions, +0.0 at the others.  Allocates; a no-op when they exist.
+// The structural values of m, expanded from its stored values and keep bits
+// if the assembly left them out (assemble.cu): the stored entries at their
+// structural positions, +0.0 at the others.  Allocates; a no-op when they
+// exist.
 int matrix_ensure_nz(llf_ctx *ctx, const llf_matrix *m);
 // assemble_fp32.cu: precision form (FP32 quadrature, FP64 accumulation) into nz
 // aflag/ageo: per-element affine flag and invJ/det (null: quadrature form

@@ -162,6 +162,78 @@ k_spmv(const double *__restrict__ nz, const int64_t *__restrict__ colptr,
   }
 }
 
+// The same product from the stored values and their keep bits, for a matrix
+// whose assembly left the structural values out: entry i of a column is the
+// stored value at its rank among the column's kept entries, +0.0 when it is
+// not stored.  The lanes, the order of their sums and so the result's bits
+// are k_spmv's.  A warp's POPCs and selects (about 40 issue slots per step)
+// fit beside its P FP64 instructions, which take 64 each of an SM quarter.
+// hex27 40^3 (297.7 M entries): 0.97 ms; expanding the structural values
+// first and k_spmv took 2.55 + 0.83 ms.
+template <int P>
+__global__ void __launch_bounds__(CG_THREADS)
+k_spmv_kept(const double *__restrict__ vals, const int64_t *__restrict__ colptr_s, const uint2 *__restrict__ keep,
+            const int64_t *__restrict__ nptr, const int32_t *__restrict__ nadj, const double *__restrict__ x,
+            double *__restrict__ y, int64_t non) {
+  constexpr int NPW = 32 / SPMV_G;  // nodes per warp
+  const int lane = threadIdx.x & 31, g = lane % SPMV_G, wpb = blockDim.x >> 5;
+  const int64_t stride = (int64_t)gridDim.x * wpb * NPW;
+  for (int64_t B0 = ((int64_t)blockIdx.x * wpb + (threadIdx.x >> 5)) * NPW; B0 < non; B0 += stride) {
+    const int64_t B = B0 + lane / SPMV_G;
+    double acc[P];
+#pragma unroll
+    for (int j = 0; j < P; ++j) acc[j] = 0.0;
+    if (B < non) {
+      const int64_t r0 = nptr[B];
+      const int n = (int)(nptr[B + 1] - r0) * P;
+      const double *v[P];
+      const uint2 *kw[P];
+      uint2 w[P];
+#pragma unroll
+      for (int j = 0; j < P; ++j) {
+        v[j] = vals + (colptr_s[P * B + j] - 1);
+        kw[j] = keep + keep_pos((int64_t)P * P * r0 + (int64_t)j * n, P * B + j);
+        w[j] = n > 0 ? kw[j][0] : make_uint2(0u, 0u);
+      }
+      for (int k0 = 0; k0 < n; k0 += 64) {
+        uint2 nx[P];   // the next words, a block of entries ahead
+#pragma unroll
+        for (int j = 0; j < P; ++j) nx[j] = k0 + 64 < n ? kw[j][(k0 >> 6) + 1] : make_uint2(0u, 0u);
+        const int lim = n - k0 < 64 ? n - k0 : 64;
+#pragma unroll 2
+        for (int i = g; i < lim; i += SPMV_G) {
+          const int k = k0 + i;
+          const double xa = x[(int64_t)P * nadj[r0 + k / P] + k % P];
+          double a[P];
+#pragma unroll
+          for (int j = 0; j < P; ++j) {
+            bool kept;
+            const int r = keep_rank(w[j], i, kept);
+            a[j] = kept ? v[j][r] : 0.0;
+          }
+#pragma unroll
+          for (int j = 0; j < P; ++j) acc[j] = __fma_rn(a[j], xa, acc[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+          v[j] += __popc(w[j].x) + __popc(w[j].y);
+          w[j] = nx[j];
+        }
+      }
+    }
+#pragma unroll
+    for (int off = SPMV_G / 2; off > 0; off >>= 1)
+#pragma unroll
+      for (int j = 0; j < P; ++j) acc[j] = __dadd_rn(acc[j], __shfl_xor_sync(0xffffffffu, acc[j], off));
+    if (B < non && g < P) {
+      double t = acc[0];
+#pragma unroll
+      for (int j = 1; j < P; ++j) t = g == j ? acc[j] : t;
+      y[P * B + g] = t;
+    }
+  }
+}
+
 __global__ void k_diag_scale(const double *__restrict__ d, const double *__restrict__ x,
                              double *__restrict__ y, int64_t n) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -1727,23 +1799,42 @@ int pcg_noalloc_impl(llf_ctx *ctx, const llf_matrix *m, const double *d_b, doubl
   return llf_fail(ctx, LLF_ERR_UNSUPPORTED, "pdim must be 1, 2 or 3");
 }
 
-int spmv_impl(llf_ctx *ctx, const llf_matrix *m, const double *d_x, double *d_y) {
-  {
-    const int rc = matrix_ensure_nz(ctx, m);
-    if (rc != LLF_OK) return rc;
+namespace {
+// One warp per eight column nodes, one round of them per warp, so that the
+// block scheduler balances the nodes' uneven lists (hex27 40^3: 1.00 -> 0.93
+// ms, from the kept values 1.31 -> 0.97 ms, against four blocks per SM).
+template <int P>
+void launch_spmv(llf_ctx *ctx, const llf_matrix *m, const double *x, double *y) {
+  const llf_pattern *p = m->pat;
+  const int64_t non = p->ndof / P;
+  constexpr int per_block = CG_THREADS / SPMV_G;
+  const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((non + per_block - 1) / per_block, 1 << 30));
+  if (m->d_nz) {
+    KernelScope ks(ctx, "k_spmv");
+    k_spmv<P><<<grid, CG_THREADS, 0, ctx->stream>>>(m->d_nz, p->d_colptr, p->d_nptr, p->d_nadj, x, y, p->ndof);
+  } else {
+    KernelScope ks(ctx, "k_spmv_kept");
+    k_spmv_kept<P><<<grid, CG_THREADS, 0, ctx->stream>>>(m->d_nzval_s, m->d_colptr_s, m->d_keep, p->d_nptr, p->d_nadj,
+                                                         x, y, non);
   }
+}
+}  // namespace
+
+int spmv_impl(llf_ctx *ctx, const llf_matrix *m, const double *d_x, double *d_y) {
   const int64_t n = m->pat->ndof;
-  const unsigned grid = (unsigned)(ctx->num_sms * 4);
   if (m->diagonal_only) {
+    const unsigned grid = (unsigned)(ctx->num_sms * 4);
     KernelScope ks(ctx, "k_diag_scale");
     k_diag_scale<<<grid, CG_THREADS, 0, ctx->stream>>>(m->d_diag, d_x, d_y, n);
   } else {
-    KernelScope ks(ctx, "k_spmv");
-    const llf_pattern *p = m->pat;
-    switch (p->pdim) {
-      case 1: k_spmv<1><<<grid, CG_THREADS, 0, ctx->stream>>>(m->d_nz, p->d_colptr, p->d_nptr, p->d_nadj, d_x, d_y, n); break;
-      case 2: k_spmv<2><<<grid, CG_THREADS, 0, ctx->stream>>>(m->d_nz, p->d_colptr, p->d_nptr, p->d_nadj, d_x, d_y, n); break;
-      case 3: k_spmv<3><<<grid, CG_THREADS, 0, ctx->stream>>>(m->d_nz, p->d_colptr, p->d_nptr, p->d_nadj, d_x, d_y, n); break;
+    if (!m->d_nz && !m->d_keep) {
+      const int rc = matrix_ensure_nz(ctx, m);   // reports the missing values
+      if (rc != LLF_OK) return rc;
+    }
+    switch (m->pat->pdim) {
+      case 1: launch_spmv<1>(ctx, m, d_x, d_y); break;
+      case 2: launch_spmv<2>(ctx, m, d_x, d_y); break;
+      case 3: launch_spmv<3>(ctx, m, d_x, d_y); break;
       default: return llf_fail(ctx, LLF_ERR_UNSUPPORTED, "pdim must be 1, 2 or 3");
     }
   }
@@ -1835,7 +1926,7 @@ __global__ void k_fdm_check_diag(const double *__restrict__ d, const uint8_t *__
 
 void free_matrix_arrays(llf_ctx *ctx, llf_matrix *m) {
   dfree(ctx, m->d_nz); dfree(ctx, m->d_diag); dfree(ctx, m->d_colptr_s);
-  dfree(ctx, m->d_rowval_s); dfree(ctx, m->d_nzval_s);
+  dfree(ctx, m->d_rowval_s); dfree(ctx, m->d_nzval_s); dfree(ctx, m->d_keep);
 }
 
 template <int P>
