@@ -19,18 +19,13 @@
 //                 twice (block and mirror).  Both kernels leave the element
 //                 matrix whole in the layout Kf[element][column node b][row
 //                 node a][block];
-//   k_colgather   one warp per column node B: walks the elements around B in
-//                 ascending order; for each, the lanes read the element's
-//                 column b = local(B) — one contiguous run of npe blocks — and
-//                 add every block into a shared-memory accumulator of the
-//                 column at the row position the pattern's element-to-column
-//                 map gives.  Each entry is thus summed over its elements in
-//                 element order, the order SparseArrays.sparse combines the
-//                 reference's triplets (src/linear.jl:314-323).  The column is
-//                 written out coalesced together with its non-zero count, or,
-//                 when the pattern kept the stored layout of an earlier
-//                 assembly of the same operator and form, compacted straight
-//                 into it (dropzeros!, every column's count checked);
+//   k_colgather   (gather.cu) sums every entry over its elements in element
+//                 order, the order SparseArrays.sparse combines the
+//                 reference's triplets (src/linear.jl:314-323), and writes
+//                 the column with its non-zero count, or, when the pattern
+//                 kept the stored layout of an earlier assembly of the same
+//                 operator and form, compacted straight into it (dropzeros!,
+//                 every column's count checked);
 //   finalize      otherwise dropzeros! (src/linear.jl:324): scan of the
 //                 counts, then compaction into 1-based Int64 SparseMatrixCSC
 //                 arrays, whose column starts the pattern keeps.
@@ -534,258 +529,9 @@ k_elem_affine(ElemArgs A, int tab_n) {
   if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
-// Column-node gather.  T = double (FP64 form) or float (precision form);
-// FP64 sums in element order in both.  Per warp: the column's row-node list
-// (deg ints) and its accumulator (deg * P * P doubles) in shared memory.
-// Exact FP32 -> FP64 widening on the integer pipe (sign, exponent rebias,
-// mantissa shift; subnormals normalised by their leading-zero count; Inf and
-// NaN keep their payload): the precision form's gather widens every element
-// value, and GB300's FP64 pipe is kept for the additions.
-__device__ __forceinline__ double widen(double x) { return x; }
-__device__ __forceinline__ double widen(unsigned long long b) { return __longlong_as_double((long long)b); }
-// The gather holds FP64 values it only moves as their bit patterns (64-bit
-// integers), so that moving, selecting and storing them takes no FP64
-// instruction: GB300 spends its FP64 pipe per warp instruction.
-template <class T> struct GatherWord { using type = T; };
-template <> struct GatherWord<double> { using type = unsigned long long; };
-__device__ __forceinline__ unsigned long long value_bits(unsigned long long b) { return b; }
-__device__ __forceinline__ unsigned long long value_bits(float f) {
-  return (unsigned long long)__double_as_longlong(widen(f));
-}
-__device__ __forceinline__ double widen(float f) {
-  const unsigned u = __float_as_uint(f);
-  const unsigned e = (u >> 23) & 0xffu, m = u & 0x7fffffu;
-  if (e - 1u < 254u) {  // normal: in 32-bit halves, exponent + (1023 - 127), mantissa << 29
-    const unsigned hi = (u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u);
-    return __hiloint2double((int)hi, (int)(u << 29));
-  }
-  unsigned long long bits;
-  if (e != 0u) {
-    const unsigned long long ed = e == 0xffu ? 0x7ffull : (unsigned long long)(e + 896u);
-    bits = (ed << 52) | ((unsigned long long)m << 29);
-  } else if (m != 0u) {
-    const int p = 31 - __clz((int)m);
-    bits = ((unsigned long long)(p + 874) << 52) | (((unsigned long long)m << (52 - p)) & 0xfffffffffffffull);
-  } else {
-    bits = 0ull;
-  }
-  return __longlong_as_double((long long)(((unsigned long long)(u >> 31) << 63) | bits));
-}
-
-// The accumulator holds P planes, one per DoF column j of the column node,
-// ps doubles apart; plane j holds the column's entries (row node t,
-// component i) at P*t + i, the order they are written out in.
-template <int P, bool BLOCKVAL, bool FIRST, class W>
-__device__ __forceinline__ void add_block(double *acc, int t, const W *v, int ps) {
-  double *dst = acc + (size_t)t * P;
-  unsigned long long *dstb = reinterpret_cast<unsigned long long *>(dst);
-#pragma unroll
-  for (int i = 0; i < P; ++i)
-#pragma unroll
-    for (int j = 0; j < P; ++j) {
-      if (FIRST) {  // the first block of the position: its bits
-        dstb[j * ps + i] = BLOCKVAL ? value_bits(v[i * P + j]) : (i == j ? value_bits(v[0]) : 0ull);
-      } else {
-        const double x = BLOCKVAL ? widen(v[i * P + j]) : (i == j ? widen(v[0]) : 0.0);
-        dst[j * ps + i] = __dadd_rn(dst[j * ps + i], x);
-      }
-    }
-}
-
 // Non-zero test on the bit pattern (integer pipe): every value but +-0.
 __device__ __forceinline__ int nonzero_bits(double v) {
   return ((unsigned long long)__double_as_longlong(v) << 1) != 0ull;
-}
-
-// Column-node gather.  One warp per column node B: its accumulator
-// (deg*P*P doubles) lives in shared memory, starting at -0.0 (the identity
-// of IEEE addition).  The elements of B are walked in ascending order; lane
-// a reads block (a, b) of the element's column b = local(B) (one contiguous
-// run of npe blocks, 16-byte padded) and the block's row position from the
-// pattern's element-to-column map, both prefetched one element ahead, and
-// adds the block into the accumulator.  A byte per row position records
-// whether the position has a value yet: the first block that reaches a
-// position is stored, later ones are added, and positions that no element
-// reaches are written as -0.0 (the identity of IEEE addition).  Every entry
-// thus equals the reference's combination of its triplets (first value,
-// then + each later one), signed zeros included, with one FP64 addition per
-// contribution after the first only.  With init (values to accumulate into)
-// the accumulator starts from them and every block is added.  The column is
-// written out coalesced with its non-zero count: column (B,j) holds the
-// entries (row node t, component i) at P*t + i.
-// all_touched: every row position of a column receives a block (a gather
-// over the pattern's own element lists), so the marks are not read when the
-// column is written out.
-// With spec.ptr0 the column is compacted (dropzeros!) straight into the
-// stored CSC at the layout of an earlier assembly: each DoF column's
-// non-zeros go, in row order, to [ptr0[c], ptr0[c+1]) (writes stay inside
-// that range) and its keep bits to spec.keep, and a column whose count
-// differs sets *spec.mismatch; the structural values are then written only
-// if nz is given.
-template <int P, bool BLOCKVAL, class T>
-__global__ void k_colgather(const int64_t *__restrict__ nptr, const int64_t *__restrict__ n2e_ptr,
-                            const int2 *__restrict__ n2e, const uint16_t *__restrict__ pos,
-                            const T *__restrict__ Kf, int64_t cs, int npe, int64_t non, int max_deg,
-                            const double *__restrict__ init, double *__restrict__ nz,
-                            int64_t *__restrict__ cnt, const int32_t *__restrict__ list,
-                            const int32_t *__restrict__ nadj, StoredSpec spec, int all_touched,
-                            int first_marked) {
-  extern __shared__ double cg_smem[];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-  constexpr int BS = BLOCKVAL ? P * P : 1;
-  constexpr int BSTR = kf_bstride(P, BLOCKVAL, (int)sizeof(T));  // stored block stride
-  constexpr bool VEC = sizeof(T) == 4 && BSTR % 4 == 0;           // 16-byte block loads
-  using W = typename GatherWord<T>::type;
-  double *acc = cg_smem + (size_t)wib * max_deg * P * P;
-  unsigned long long *accb = reinterpret_cast<unsigned long long *>(acc);
-  const int ps = max_deg * P;  // accumulator plane stride
-  unsigned char *has = reinterpret_cast<unsigned char *>(cg_smem + (size_t)wpb * max_deg * P * P) +
-                       (size_t)wib * ((max_deg + 7) & ~7);
-  const int nw = (int)non, wstride = (int)gridDim.x * wpb;  // node counts fit int32 (nadj holds int32 nodes)
-  for (int w = (int)blockIdx.x * wpb + wib; w < nw; w += wstride) {
-    const int64_t B = list ? (int64_t)__ldg(list + w) : (int64_t)w;  // column node (non: nodes of the list)
-    const int64_t c0 = nptr[B];
-    const int deg = (int)(nptr[B + 1] - c0);
-    const int64_t s = n2e_ptr[B];
-    const int nb = (int)(n2e_ptr[B + 1] - s);
-    if (init) {  // accumulate into existing structural values (same layout as the output)
-      const double *src = init + (size_t)P * P * c0;
-      for (int idx = lane; idx < deg * P * P; idx += 32) {
-        const int j = idx / (P * deg), r = idx - j * P * deg;
-        accb[(size_t)j * ps + r] = reinterpret_cast<const unsigned long long *>(src)[idx];
-      }
-    } else if (!first_marked) {
-      for (int t = lane; t < deg; t += 32) has[t] = 0;
-    }
-    const bool store_first = init == nullptr;
-    __syncwarp();
-    if (npe <= 32) {
-      const bool act = lane < npe;
-      W cur[BSTR], nxt[BSTR];
-      unsigned tc = 0xffffu, tn = 0xffffu;
-      auto load_block = [&](const T *v, W *dst) {
-        if constexpr (VEC) {
-#pragma unroll
-          for (int m = 0; m < BSTR; m += 4) {
-            const float4 f = __ldg(reinterpret_cast<const float4 *>(v + m));
-            dst[m] = f.x; dst[m + 1] = f.y; dst[m + 2] = f.z; dst[m + 3] = f.w;
-          }
-        } else {
-          const W *vw = reinterpret_cast<const W *>(v);
-#pragma unroll
-          for (int m = 0; m < BS; ++m) dst[m] = vw[m];
-        }
-      };
-      if (nb > 0 && act) {
-        const int2 el = n2e[s];
-        load_block(Kf + ((size_t)el.x * npe + el.y) * cs + (size_t)lane * BSTR, cur);
-        tc = pos[s * npe + lane];
-      }
-      for (int k = 0; k < nb; ++k) {  // elements of B, ascending
-        if (k + 1 < nb && act) {
-          const int2 el = n2e[s + k + 1];
-          load_block(Kf + ((size_t)el.x * npe + el.y) * cs + (size_t)lane * BSTR, nxt);
-          tn = pos[(s + k + 1) * npe + lane];
-        }
-        if (act && tc != 0xffffu) {  // the lanes of one element hold distinct positions
-          if (first_marked) {  // the map marks each position's first block
-            if (store_first && (tc & 0x8000u))
-              add_block<P, BLOCKVAL, true>(acc, (int)(tc & 0x7fffu), cur, ps);
-            else
-              add_block<P, BLOCKVAL, false>(acc, (int)(tc & 0x7fffu), cur, ps);
-          } else if (store_first && !has[tc]) {
-            add_block<P, BLOCKVAL, true>(acc, (int)tc, cur, ps);
-            has[tc] = 1;
-          } else {
-            add_block<P, BLOCKVAL, false>(acc, (int)tc, cur, ps);
-          }
-        }
-        __syncwarp();
-#pragma unroll
-        for (int m = 0; m < BSTR; ++m) cur[m] = nxt[m];
-        tc = tn;
-      }
-    } else {
-      for (int k = 0; k < nb; ++k) {
-        const int2 el = n2e[s + k];
-        const T *col = Kf + ((size_t)el.x * npe + el.y) * cs;
-        for (int a = lane; a < npe; a += 32) {
-          const unsigned raw = pos[(s + k) * npe + a];
-          const unsigned t = (first_marked && raw != 0xffffu) ? (raw & 0x7fffu) : raw;
-          if (raw != 0xffffu) {
-            if (first_marked) {
-              if (store_first && (raw & 0x8000u))
-                add_block<P, BLOCKVAL, true>(acc, (int)t, reinterpret_cast<const W *>(col + (size_t)a * BSTR), ps);
-              else
-                add_block<P, BLOCKVAL, false>(acc, (int)t, reinterpret_cast<const W *>(col + (size_t)a * BSTR), ps);
-            } else if (store_first && !has[t]) {
-              add_block<P, BLOCKVAL, true>(acc, (int)t, reinterpret_cast<const W *>(col + (size_t)a * BSTR), ps);
-              has[t] = 1;
-            } else {
-              add_block<P, BLOCKVAL, false>(acc, (int)t, reinterpret_cast<const W *>(col + (size_t)a * BSTR), ps);
-            }
-          }
-        }
-        __syncwarp();
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < P; ++j) {
-      double *out = nz ? nz + (size_t)P * P * c0 + (size_t)j * P * deg : nullptr;
-      if (spec.ptr0) {
-        const int64_t o = spec.ptr0[B * P + j], oend = spec.ptr0[B * P + j + 1];
-        const int32_t *rn = nadj + c0;
-        const unsigned kp = (unsigned)keep_pos((int64_t)P * P * c0 + j * P * deg, B * P + j);
-        int run = 0;
-        const unsigned below = (1u << lane) - 1u;
-        // warp-uniform chunks of 64 entries, two consecutive ones per lane
-        for (int i0 = 0; i0 < P * deg; i0 += 64) {
-          const int idx = i0 + 2 * lane;
-          unsigned long long v[2] = {0ull, 0ull};   // value bits
-          bool keep[2];
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const bool valid = idx + h < P * deg;
-            if (valid) {
-              v[h] = (!store_first || all_touched || has[(idx + h) / P]) ? accb[(size_t)j * ps + idx + h]
-                                                                         : 0x8000000000000000ull;   // -0.0
-              if (nz) reinterpret_cast<unsigned long long *>(out)[idx + h] = v[h];
-            }
-            keep[h] = valid && (v[h] << 1) != 0ull;
-          }
-          const unsigned b0 = __ballot_sync(0xffffffffu, keep[0]), b1 = __ballot_sync(0xffffffffu, keep[1]);
-          if (lane == 0) spec.keep[kp + (i0 >> 6)] = make_uint2(b0, b1);
-          int64_t at = o + run + __popc(b0 & below) + __popc(b1 & below);   // the lanes before, both entries
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            if (keep[h]) {
-              if (at < oend) {
-                const int t = (idx + h) / P, i = (idx + h) % P;
-                spec.rowval_s[at] = (int64_t)P * rn[t] + i + 1;
-                reinterpret_cast<unsigned long long *>(spec.nzval_s)[at] = v[h];
-              }
-              ++at;
-            }
-          }
-          run += __popc(b0) + __popc(b1);
-        }
-        if (lane == 0 && (int64_t)run != oend - o) atomicOr(spec.mismatch, 1u);
-      } else {
-        int n = 0;
-        for (int idx = lane; idx < P * deg; idx += 32) {
-          const int t = idx / P, i = idx % P;
-          const unsigned long long v =
-              (!store_first || all_touched || has[t]) ? accb[(size_t)j * ps + idx] : 0x8000000000000000ull;
-          reinterpret_cast<unsigned long long *>(out)[idx] = v;
-          n += (v << 1) != 0ull;
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) n += __shfl_xor_sync(0xffffffffu, n, off);
-        if (lane == 0 && cnt) cnt[B * P + j] = n;
-      }
-    }
-    __syncwarp();
-  }
 }
 
 // ---------------------------------------------------------------- dropzeros
@@ -1010,208 +756,15 @@ int run_elem(llf_ctx *ctx, ElemArgs a) {
   return rc;
 }
 
-// Gather over explicit node -> element lists and element-to-column map (the
-// pattern's own, or those of another element set on the same nodes).
-// The column nodes of the pattern in two degree classes, once per pattern:
-// when at least 60 % of the nodes have a degree of at most 0.7 of the
-// largest, those nodes form the low class (ascending), the rest follow.
-// The low class then runs with a smaller accumulator and so with more warps
-// per SM (hex27: degree <= 75 against 125 for 7/8 of the nodes).  Each
-// column is summed the same way whichever launch takes it.
-static int gather_split(llf_ctx *ctx, llf_pattern *pat) {
-  if (pat->gather_split_done) return LLF_OK;
-  pat->gather_split_done = true;
-  const int64_t non = pat->mesh->non;
-  const int thr = pat->tune.gather_thr;   // percent of the largest degree
-  if (non < 1024 || pat->max_deg < 16 || thr <= 0) return LLF_OK;
-  std::vector<int64_t> h(non + 1);
-  LLF_CUDA_TRY(ctx, cudaMemcpyAsync(h.data(), pat->d_nptr, sizeof(int64_t) * (non + 1), cudaMemcpyDeviceToHost,
-                                    ctx->stream));
-  LLF_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-  std::vector<int64_t> hist(pat->max_deg + 1, 0);
-  for (int64_t b = 0; b < non; ++b) hist[h[b + 1] - h[b]]++;
-  int md_low = -1;
-  int64_t acc = 0;
-  for (int d = 0; d <= pat->max_deg; ++d) {
-    acc += hist[d];
-    if (acc >= (non * 6 + 9) / 10) { md_low = d; break; }
-  }
-  if (md_low < 1 || md_low * 100 > pat->max_deg * thr) return LLF_OK;
-  std::vector<int32_t> order;
-  order.reserve(non);
-  for (int64_t b = 0; b < non; ++b)
-    if (h[b + 1] - h[b] <= md_low) order.push_back((int32_t)b);
-  const int64_t n_low = (int64_t)order.size();
-  for (int64_t b = 0; b < non; ++b)
-    if (h[b + 1] - h[b] > md_low) order.push_back((int32_t)b);
-  LLF_CUDA_TRY(ctx, dalloc(ctx, &pat->d_gather_nodes, non));
-  LLF_CUDA_TRY(ctx, cudaMemcpyAsync(pat->d_gather_nodes, order.data(), sizeof(int32_t) * non, cudaMemcpyHostToDevice,
-                                    ctx->stream));
-  LLF_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-  pat->gather_n_low = n_low;
-  pat->gather_md_low = md_low;
-  return LLF_OK;
-}
-
-// Marks, once per pattern, the first block of every row position in the
-// pattern's element-to-column map: per column node B (a warp each), its
-// elements in ascending order, and the first element whose block reaches a
-// row position gets bit 15 of that map entry (positions fit 15 bits).  The
-// gather then stores that block and adds the later ones without keeping
-// per-position marks of its own.
-__global__ void k_mark_first(const int64_t *__restrict__ nptr, const int64_t *__restrict__ n2e_ptr,
-                             uint16_t *__restrict__ pos, int npe, int64_t non, int max_deg) {
-  extern __shared__ unsigned char mf_has[];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-  unsigned char *has = mf_has + (size_t)wib * ((max_deg + 7) & ~7);
-  for (int64_t B = (int64_t)blockIdx.x * wpb + wib; B < non; B += (int64_t)gridDim.x * wpb) {
-    const int deg = (int)(nptr[B + 1] - nptr[B]);
-    const int64_t s = n2e_ptr[B];
-    const int nb = (int)(n2e_ptr[B + 1] - s);
-    for (int t = lane; t < deg; t += 32) has[t] = 0;
-    __syncwarp();
-    for (int k = 0; k < nb; ++k) {
-      for (int a = lane; a < npe; a += 32) {  // the lanes of one element hold distinct positions
-        const unsigned raw = pos[(s + k) * npe + a];
-        if (raw < 0x8000u && !has[raw]) {
-          has[raw] = 1;
-          pos[(s + k) * npe + a] = (uint16_t)(raw | 0x8000u);
-        }
-      }
-      __syncwarp();
-    }
-  }
-}
-
-template <int P, bool BV, class T>
-int run_colgather(llf_ctx *ctx, llf_pattern *pat, const int64_t *n2e_ptr, const int2 *n2e, const uint16_t *pos,
-                  int npe, const T *Kf, int64_t cs, const double *init, double *nz, int64_t *cnt,
-                  int64_t B0 = 0, int64_t nB = -1, const StoredSpec *spec = nullptr) {
-  const StoredSpec sp = spec ? *spec : StoredSpec{};
-  // column nodes [B0, B0 + nB): the node-indexed arrays are offset, the
-  // offsets they hold (into n2e, pos, nz) stay absolute
-  if (nB < 0) nB = pat->mesh->non - B0;
-  if (pat->conn_version != pat->mesh->conn_version)
-    return llf_fail(ctx, LLF_ERR_STATE, "the mesh connectivity changed after the pattern was built; rebuild it");
-  // the pattern's own map: each position's first block marked (once)
-  bool first_marked = false;
-  const int mdm = pat->max_deg > 0 ? pat->max_deg : 1;
-  if (pos == pat->d_pos && mdm < 0x7fff) {
-    if (!pat->pos_first) {
-      const int mw = 4;
-      const size_t msm = (size_t)mw * ((mdm + 7) & ~7);
-      KernelScope ks(ctx, "k_mark_first");
-      k_mark_first<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((pat->mesh->non + mw - 1) / mw,
-                                                                    (int64_t)ctx->num_sms * 8)),
-                     mw * 32, msm, ctx->stream>>>(pat->d_nptr, pat->d_n2e_ptr, pat->d_pos, npe, pat->mesh->non, mdm);
-      LLF_CUDA_TRY(ctx, cudaGetLastError());
-      pat->pos_first = true;
-    }
-    first_marked = true;
-  }
-  auto fn = k_colgather<P, BV, T>;
-  // one launch over `count` column nodes (the list's, or [B0, B0 + count))
-  // with an accumulator of md row positions per warp
-  auto launch = [&](int md, const int32_t *list, int64_t b0, int64_t count) -> int {
-    if (count <= 0) return LLF_OK;
-    const size_t per_warp = (size_t)md * P * P * sizeof(double) + (size_t)((md + 7) & ~7);
-    int wpb = (int)std::min<size_t>(pat->tune.gather_wpb > 0 ? pat->tune.gather_wpb : 4, (200 * 1024) / per_warp);
-    if (wpb < 1) wpb = 1;
-    size_t smem = (size_t)wpb * per_warp;
-    if (smem > 200 * 1024)
-      return llf_fail(ctx, LLF_ERR_LIMIT, "a column node has too many neighbours for the gather buffer");
-    if (smem > 48 * 1024)
-      LLF_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 1;
-    LLF_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, wpb * 32, smem));
-    int64_t grid = (int64_t)ctx->num_sms * (per_sm < 1 ? 1 : per_sm);
-    int64_t need = (count + wpb - 1) / wpb;
-    if (grid > need) grid = need > 0 ? need : 1;
-    KernelScope ks(ctx, "k_colgather");
-    fn<<<(unsigned)grid, wpb * 32, smem, ctx->stream>>>(pat->d_nptr + b0, n2e_ptr + b0, n2e, pos, Kf, cs, npe, count,
-                                                        md, init, nz, cnt ? cnt + b0 * P : nullptr, list,
-                                                        pat->d_nadj, sp, n2e_ptr == pat->d_n2e_ptr ? 1 : 0,
-                                                        first_marked ? 1 : 0);
-    LLF_CUDA_TRY(ctx, cudaGetLastError());
-    return LLF_OK;
-  };
-  const int md = pat->max_deg > 0 ? pat->max_deg : 1;
-  if (B0 == 0 && nB == pat->mesh->non) {
-    int rc = gather_split(ctx, pat);
-    if (rc != LLF_OK) return rc;
-    if (pat->d_gather_nodes) {
-      rc = launch(pat->gather_md_low, pat->d_gather_nodes, 0, pat->gather_n_low);
-      if (rc == LLF_OK)
-        rc = launch(md, pat->d_gather_nodes + pat->gather_n_low, 0, pat->mesh->non - pat->gather_n_low);
-      return rc;
-    }
-  }
-  return launch(md, nullptr, B0, nB);
-}
-
 }  // namespace
 
 // ------------------------------------------------------------------ host
-template <class T>
-int gather_full_t(llf_ctx *ctx, llf_pattern *pat, const int64_t *n2e_ptr, const int2 *n2e, const uint16_t *pos,
-                  int npe, const T *Kf, int64_t cs, bool blockval, const double *init, double *nz, int64_t *cnt,
-                  StoredSpec *spec = nullptr);
-
-// The gather into a kept stored layout; if a column's count differs, the
-// usual gather (structural values and counts) follows.
-template <class T>
-int gather_spec_t(llf_ctx *ctx, llf_pattern *pat, const T *Kf, int64_t cs, bool blockval, StoredSpec *spec) {
-  int rc = gather_full_t<T>(ctx, pat, pat->d_n2e_ptr, pat->d_n2e, pat->d_pos, pat->mesh->npe, Kf, cs, blockval,
-                            nullptr, nullptr, nullptr, spec);
-  if (rc != LLF_OK) return rc;
-  unsigned mis = 1;
-  LLF_CUDA_TRY(ctx, cudaMemcpyAsync(&mis, spec->mismatch, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
-  LLF_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-  if (mis == 0) return LLF_OK;
-  spec->fell_back = true;
-  LLF_CUDA_TRY(ctx, dalloc(ctx, spec->nz_slot, pat->nnz));
-  return gather_full_t<T>(ctx, pat, pat->d_n2e_ptr, pat->d_n2e, pat->d_pos, pat->mesh->npe, Kf, cs, blockval,
-                          nullptr, *spec->nz_slot, spec->cnt_fallback, nullptr);
-}
-
-template <class T>
-int gather_full_t(llf_ctx *ctx, llf_pattern *pat, const int64_t *n2e_ptr, const int2 *n2e, const uint16_t *pos,
-                  int npe, const T *Kf, int64_t cs, bool blockval, const double *init, double *nz, int64_t *cnt,
-                  StoredSpec *spec) {
-  switch (pat->pdim * 2 + (blockval ? 1 : 0)) {
-    case 2: return run_colgather<1, false, T>(ctx, pat, n2e_ptr, n2e, pos, npe, Kf, cs, init, nz, cnt, 0, -1, spec);
-    case 3: return run_colgather<1, true, T>(ctx, pat, n2e_ptr, n2e, pos, npe, Kf, cs, init, nz, cnt, 0, -1, spec);
-    case 4: return run_colgather<2, false, T>(ctx, pat, n2e_ptr, n2e, pos, npe, Kf, cs, init, nz, cnt, 0, -1, spec);
-    case 5: return run_colgather<2, true, T>(ctx, pat, n2e_ptr, n2e, pos, npe, Kf, cs, init, nz, cnt, 0, -1, spec);
-    case 6: return run_colgather<3, false, T>(ctx, pat, n2e_ptr, n2e, pos, npe, Kf, cs, init, nz, cnt, 0, -1, spec);
-    case 7: return run_colgather<3, true, T>(ctx, pat, n2e_ptr, n2e, pos, npe, Kf, cs, init, nz, cnt, 0, -1, spec);
-  }
-  return llf_fail(ctx, LLF_ERR_UNSUPPORTED, "pdim must be 1, 2 or 3");
-}
-
-int gather_full(llf_ctx *ctx, llf_pattern *pat, const double *Kf, int64_t colstride, bool blockval,
-                double *nz, int64_t *cnt, const double *init, StoredSpec *spec) {
-  if (spec) return gather_spec_t<double>(ctx, pat, Kf, colstride, blockval, spec);
-  return gather_full_t<double>(ctx, pat, pat->d_n2e_ptr, pat->d_n2e, pat->d_pos, pat->mesh->npe, Kf, colstride,
-                               blockval, init, nz, cnt);
-}
-int gather_full32(llf_ctx *ctx, llf_pattern *pat, const float *Kf, int64_t colstride, bool blockval,
-                  double *nz, int64_t *cnt, const double *init, StoredSpec *spec) {
-  if (spec) return gather_spec_t<float>(ctx, pat, Kf, colstride, blockval, spec);
-  return gather_full_t<float>(ctx, pat, pat->d_n2e_ptr, pat->d_n2e, pat->d_pos, pat->mesh->npe, Kf, colstride,
-                              blockval, init, nz, cnt);
-}
-int gather_full_ext(llf_ctx *ctx, llf_pattern *pat, const int64_t *n2e_ptr, const int2 *n2e, const uint16_t *pos,
-                    int npe, const double *Kf, int64_t colstride, bool blockval, double *nz, int64_t *cnt) {
-  return gather_full_t<double>(ctx, pat, n2e_ptr, n2e, pos, npe, Kf, colstride, blockval, nullptr, nz, cnt);
-}
-
 // Structural values from the stored values and the keep bits, one warp per
-// DoF column, 64 entries at a time and two per lane (the bits' layout); an
-// entry that is not stored is +0.0.  Bound by HBM: nzval read, the
-// structural values written.  hex27 40^3 (297.7 M entries): 0.91 ms; the
-// binary search of every stored row in the column's node list that the bits
-// replace took 2.55 ms.
+// DoF column, 64 entries at a time (a word pair of the bits); an entry that
+// is not stored is +0.0.  Bound by HBM: nzval read, the structural values
+// written.  hex27 40^3 (297.7 M entries): 0.91 ms; the binary search of
+// every stored row in the column's node list that the bits replace took
+// 2.55 ms.
 __global__ void __launch_bounds__(256)
 k_expand_nz(const int64_t *__restrict__ colptr, int64_t ndof, const int64_t *__restrict__ colptr_s,
             const double *__restrict__ nzval_s, const uint2 *__restrict__ keep, double *__restrict__ nz) {
@@ -1221,17 +774,16 @@ k_expand_nz(const int64_t *__restrict__ colptr, int64_t ndof, const int64_t *__r
     const int len = (int)(colptr[c + 1] - s);
     const double *v = nzval_s + (colptr_s[c] - 1);
     const uint2 *kw = keep + keep_pos(s, c);
+    const unsigned below = (1u << lane) - 1u;
 #pragma unroll 4
     for (int l0 = 0; l0 < len; l0 += 64) {
       const uint2 w = kw[l0 >> 6];
-      const int l = l0 + 2 * lane;
-      bool k0, k1;
-      const int r = keep_rank(w, 2 * lane, k0);
-      keep_rank(w, 2 * lane + 1, k1);
-      const double a = k0 ? v[r] : 0.0, b = k1 ? v[r + k0] : 0.0;
+      const int l = l0 + lane, nx = __popc(w.x);
+      const double a = (w.x >> lane) & 1u ? v[__popc(w.x & below)] : 0.0;
+      const double b = (w.y >> lane) & 1u ? v[nx + __popc(w.y & below)] : 0.0;
       if (l < len) nz[s + l] = a;
-      if (l + 1 < len) nz[s + l + 1] = b;
-      v += __popc(w.x) + __popc(w.y);
+      if (l + 32 < len) nz[s + l + 32] = b;
+      v += nx + __popc(w.y);
     }
   }
 }
@@ -1711,15 +1263,7 @@ struct HostSlabSink : GatherSink {
         e_done = e_need;
       }
       if (nB > 0) {
-        switch (P * 2 + (blockval ? 1 : 0)) {
-          case 2: rc = run_colgather<1, false, T>(ctx, pat, pat->d_n2e_ptr, pat->d_n2e, pat->d_pos, pat->mesh->npe, Kf, cs, nullptr, nz, cnt, B0, nB); break;
-          case 3: rc = run_colgather<1, true, T>(ctx, pat, pat->d_n2e_ptr, pat->d_n2e, pat->d_pos, pat->mesh->npe, Kf, cs, nullptr, nz, cnt, B0, nB); break;
-          case 4: rc = run_colgather<2, false, T>(ctx, pat, pat->d_n2e_ptr, pat->d_n2e, pat->d_pos, pat->mesh->npe, Kf, cs, nullptr, nz, cnt, B0, nB); break;
-          case 5: rc = run_colgather<2, true, T>(ctx, pat, pat->d_n2e_ptr, pat->d_n2e, pat->d_pos, pat->mesh->npe, Kf, cs, nullptr, nz, cnt, B0, nB); break;
-          case 6: rc = run_colgather<3, false, T>(ctx, pat, pat->d_n2e_ptr, pat->d_n2e, pat->d_pos, pat->mesh->npe, Kf, cs, nullptr, nz, cnt, B0, nB); break;
-          case 7: rc = run_colgather<3, true, T>(ctx, pat, pat->d_n2e_ptr, pat->d_n2e, pat->d_pos, pat->mesh->npe, Kf, cs, nullptr, nz, cnt, B0, nB); break;
-          default: rc = llf_fail(ctx, LLF_ERR_UNSUPPORTED, "pdim must be 1, 2 or 3");
-        }
+        rc = gather_slab(ctx, pat, Kf, cs, blockval, nz, cnt, B0, nB);
         if (rc != LLF_OK) break;
         {
           KernelScope ks(ctx, "scan");

@@ -205,8 +205,8 @@ struct llf_matrix {
   double *d_nzval_s = nullptr;    // nnz_s
   // written with a stored CSC that went into a kept layout: which structural
   // entries of a column are stored.  Column c (structural start s) holds a
-  // pair of words per 64 entries at keep_pos(s, c): entry i of the 64 is bit
-  // i / 2 of word x (i even) or y (i odd).
+  // pair of words per 64 entries at keep_pos(s, c): entries 0..31 in word x,
+  // 32..63 in word y.
   uint2 *d_keep = nullptr;
 };
 
@@ -214,16 +214,6 @@ struct llf_matrix {
 // the pairs of a pattern: s / 64 + c leaves every column its ceil(len / 64).
 __host__ __device__ __forceinline__ int64_t keep_pos(int64_t s, int64_t c) { return (s >> 6) + c; }
 inline int64_t keep_words(int64_t nnz, int64_t ndof) { return (nnz >> 6) + ndof + 1; }
-#ifdef __CUDACC__
-// The stored entries among the 64 before entry i of them, and whether entry
-// i is stored (0 <= i < 64).
-__device__ __forceinline__ int keep_rank(uint2 w, int i, bool &kept) {
-  const int q = i >> 1, odd = i & 1;
-  const unsigned below = (1u << q) - 1u, ex = (w.x >> q) & 1u, ey = (w.y >> q) & 1u;
-  kept = odd ? ey : ex;
-  return __popc(w.x & below) + __popc(w.y & below) + (odd ? (int)ex : 0);
-}
-#endif
 
 // ---------------------------------------------------------------- helpers
 #define LLF_CUDA_TRY(ctx, expr)                                            \
@@ -337,6 +327,11 @@ int gather_full(llf_ctx *ctx, llf_pattern *pat, const double *Kf, int64_t colstr
                 double *nz, int64_t *cnt, const double *init = nullptr, StoredSpec *spec = nullptr);
 int gather_full32(llf_ctx *ctx, llf_pattern *pat, const float *Kf, int64_t colstride, bool blockval,
                   double *nz, int64_t *cnt, const double *init = nullptr, StoredSpec *spec = nullptr);
+// The gather of the column nodes [B0, B0 + nB) only (to-host slabs).
+int gather_slab(llf_ctx *ctx, llf_pattern *pat, const double *Kf, int64_t colstride, bool blockval, double *nz,
+                int64_t *cnt, int64_t B0, int64_t nB);
+int gather_slab(llf_ctx *ctx, llf_pattern *pat, const float *Kf, int64_t colstride, bool blockval, double *nz,
+                int64_t *cnt, int64_t B0, int64_t nB);
 // The same gather for another element set on the pattern's nodes (e.g.
 // boundary faces): its node -> element lists, element-to-column map and npe.
 int gather_full_ext(llf_ctx *ctx, llf_pattern *pat, const int64_t *n2e_ptr, const int2 *n2e, const uint16_t *pos,

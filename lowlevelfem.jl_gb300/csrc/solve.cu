@@ -168,7 +168,7 @@ k_spmv(const double *__restrict__ nz, const int64_t *__restrict__ colptr,
 // not stored.  The lanes, the order of their sums and so the result's bits
 // are k_spmv's.  A warp's POPCs and selects (about 40 issue slots per step)
 // fit beside its P FP64 instructions, which take 64 each of an SM quarter.
-// hex27 40^3 (297.7 M entries): 0.97 ms; expanding the structural values
+// hex27 40^3 (297.7 M entries): 0.87 ms; expanding the structural values
 // first and k_spmv took 2.55 + 0.83 ms.
 template <int P>
 __global__ void __launch_bounds__(CG_THREADS)
@@ -187,36 +187,33 @@ k_spmv_kept(const double *__restrict__ vals, const int64_t *__restrict__ colptr_
       const int64_t r0 = nptr[B];
       const int n = (int)(nptr[B + 1] - r0) * P;
       const double *v[P];
-      const uint2 *kw[P];
-      uint2 w[P];
+      const unsigned *kw[P];   // a word per 32 entries
+      unsigned w[P];
 #pragma unroll
       for (int j = 0; j < P; ++j) {
         v[j] = vals + (colptr_s[P * B + j] - 1);
-        kw[j] = keep + keep_pos((int64_t)P * P * r0 + (int64_t)j * n, P * B + j);
-        w[j] = n > 0 ? kw[j][0] : make_uint2(0u, 0u);
+        kw[j] = reinterpret_cast<const unsigned *>(keep + keep_pos((int64_t)P * P * r0 + (int64_t)j * n, P * B + j));
+        w[j] = n > 0 ? kw[j][0] : 0u;
       }
-      for (int k0 = 0; k0 < n; k0 += 64) {
-        uint2 nx[P];   // the next words, a block of entries ahead
+      for (int k0 = 0; k0 < n; k0 += 32) {
+        unsigned nx[P];   // the next words, a block of entries ahead
 #pragma unroll
-        for (int j = 0; j < P; ++j) nx[j] = k0 + 64 < n ? kw[j][(k0 >> 6) + 1] : make_uint2(0u, 0u);
-        const int lim = n - k0 < 64 ? n - k0 : 64;
+        for (int j = 0; j < P; ++j) nx[j] = k0 + 32 < n ? kw[j][(k0 >> 5) + 1] : 0u;
+        const int lim = n - k0 < 32 ? n - k0 : 32;
 #pragma unroll 2
         for (int i = g; i < lim; i += SPMV_G) {
           const int k = k0 + i;
           const double xa = x[(int64_t)P * nadj[r0 + k / P] + k % P];
+          const unsigned below = (1u << i) - 1u;
           double a[P];
 #pragma unroll
-          for (int j = 0; j < P; ++j) {
-            bool kept;
-            const int r = keep_rank(w[j], i, kept);
-            a[j] = kept ? v[j][r] : 0.0;
-          }
+          for (int j = 0; j < P; ++j) a[j] = (w[j] >> i) & 1u ? v[j][__popc(w[j] & below)] : 0.0;
 #pragma unroll
           for (int j = 0; j < P; ++j) acc[j] = __fma_rn(a[j], xa, acc[j]);
         }
 #pragma unroll
         for (int j = 0; j < P; ++j) {
-          v[j] += __popc(w[j].x) + __popc(w[j].y);
+          v[j] += __popc(w[j]);
           w[j] = nx[j];
         }
       }
