@@ -49,33 +49,51 @@ struct MixedBufs {
 };
 
 struct SegState {
-  double rho_prev, rho, alpha, res, res0, tol;
+  double rho, alpha, beta, res, res0, tol;   // beta: the next direction's rho / rho_prev
   long long it, maxiter;
   int done, breakdown;
   double rmax;  // mixed precision: true residual at the last reliable update
   int upd, pad;  // mixed precision: a reliable update is due
 };
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v = __dadd_rn(v, __shfl_xor_sync(0xffffffffu, v, off));
-  return v;
-}
-
-// Block-wide sum with a fixed tree; result valid in thread 0.
-__device__ __forceinline__ double block_sum(double v) {
-  __shared__ double ws[CG_THREADS / 32];
-  v = warp_sum(v);
+// Block-wide sums of CG_THREADS values with a fixed tree; results valid in
+// thread 0.  The tree is the xor tree of every warp (16, 8, ... 1), then of
+// the eight warps (4, 2, 1).  GB300 spends its FP64 pipe (16 SM cycles) per
+// warp instruction however few lanes hold distinct sums, so the first level
+// packs the halves of two warps into one (the values pass through shared
+// memory): 4 warps x 5 + 3 instead of 8 warps x 5 + 5 additions per sum.
+template <int N>
+__device__ __forceinline__ void block_sums(double (&v)[N]) {
+  static_assert(N == 1 || N == 2, "one or two sums");
+  __shared__ double sv[N][CG_THREADS], sw[N][CG_THREADS / 32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) ws[w] = v;
+#pragma unroll
+  for (int k = 0; k < N; ++k) sv[k][threadIdx.x] = v[k];
   __syncthreads();
-  double r = 0.0;
-  if (w == 0) {
-    r = lane < (int)(blockDim.x >> 5) ? ws[lane] : 0.0;
-    r = warp_sum(r);
+  if (w < 4 * N) {  // warps 4k .. 4k+3: sum k, each the halves of two warps
+    const int k = w >> 2, q = w & 3;
+    const double *s = sv[N == 1 ? 0 : k] + (2 * q + (lane >> 4)) * 32 + (lane & 15);
+    double t = __dadd_rn(s[0], s[16]);
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) t = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, off));
+    if ((lane & 15) == 0) sw[N == 1 ? 0 : k][2 * q + (lane >> 4)] = t;
   }
   __syncthreads();
-  return r;
+  if (w == 0) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      double t = lane < CG_THREADS / 32 ? sw[k][lane] : 0.0;
+#pragma unroll
+      for (int off = 4; off > 0; off >>= 1) t = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, off));
+      v[k] = t;
+    }
+  }
+  __syncthreads();
+}
+__device__ __forceinline__ double block_sum(double v) {
+  double s[1] = {v};
+  block_sums<1>(s);
+  return s[0];
 }
 
 // Products of the P columns of node B by x, summed over SPMV_G lanes: the
@@ -408,7 +426,6 @@ __device__ __forceinline__ void seg_set_alpha(const Seg &S, int s, double uc) {
 __device__ __forceinline__ bool seg_set_finish(const Seg &S, int s, double rr) {
   SegState &q = S.st[s];
   q.res = sqrt(rr);
-  q.rho_prev = q.rho;
   q.it += 1;
   if (q.res <= q.tol || q.it >= q.maxiter) {
     q.done = 1;
@@ -416,6 +433,13 @@ __device__ __forceinline__ bool seg_set_finish(const Seg &S, int s, double rr) {
     return true;
   }
   return false;
+}
+// The next rho, and beta from it and the last one: formed once by the block
+// that has rho (a division is about ten FP64 instructions, and the direction
+// kernels' blocks would each spend them in every warp).
+__device__ __forceinline__ void seg_set_rho(SegState &q, double rho) {
+  q.beta = rho / q.rho;
+  q.rho = rho;
 }
 
 __global__ void k_seg_start(Seg S, const double *part, double reltol, long long maxiter) {
@@ -426,8 +450,8 @@ __global__ void k_seg_start(Seg S, const double *part, double reltol, long long 
       q.res0 = sqrt(rr);
       q.res = q.res0;
       q.tol = reltol * q.res0;
-      q.rho_prev = 1.0;
-      q.rho = 0.0;
+      q.rho = 1.0;   // the first direction: beta = rho / 1
+      q.beta = 0.0;
       q.alpha = 0.0;
       q.it = 0;
       q.maxiter = maxiter;
@@ -461,7 +485,7 @@ __global__ void k_seg_rho(Seg S, const double *part) {
   for (int s = blockIdx.x; s < S.nseg; s += gridDim.x) {
     if (S.st[s].done) continue;
     double v = seg_total(S, s, part);
-    if (threadIdx.x == 0) S.st[s].rho = v;
+    if (threadIdx.x == 0) seg_set_rho(S.st[s], v);
   }
 }
 
@@ -469,7 +493,7 @@ __global__ void k_seg_dir(Seg S, const double *__restrict__ z, double *__restric
   for (int64_t ch = blockIdx.x; ch < S.nchunks; ch += gridDim.x) {
     const SegState &q = S.st[S.cseg[ch]];
     if (q.done) continue;
-    const double beta = q.rho / q.rho_prev;
+    const double beta = q.beta;
     const int64_t b = S.cbeg[ch], e = S.cend[ch];
 #pragma unroll
     for (int k = 0; k < CHUNK_PER_THREAD; ++k) {
@@ -483,8 +507,9 @@ __global__ void k_seg_dir(Seg S, const double *__restrict__ z, double *__restric
 // node column B (chunks start and end on node boundaries), the chunk's nodes
 // taken in the order S.perm gives (decreasing degree: the eight nodes of a
 // warp have lists of similar length, so few lanes idle in the FP64 products).
-// A column's sums do not depend on the order; the partial u.c takes its
-// nodes in that fixed order.  The block that brings in a segment's last
+// A column's sums do not depend on the order.  c is kept in shared memory as
+// well, and the partial u.c takes the chunk's DoFs as the update's sums do
+// (thread t: DoFs t, t + 256, t + 512), every lane busy.  The block that brings in a segment's last
 // chunk sums the partials (chunk order) and sets alpha = rho / u.c.
 template <int P>
 __global__ void __launch_bounds__(CG_THREADS)
@@ -492,11 +517,12 @@ k_seg_spmv(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ npt
            const int32_t *__restrict__ nadj, const double *__restrict__ u,
            const uint8_t *__restrict__ fixed, double *__restrict__ c, double *__restrict__ part) {
   constexpr int NPW = 32 / SPMV_G;  // nodes per warp
+  __shared__ double sC[CHUNK];
   const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5, w = threadIdx.x >> 5, g = lane % SPMV_G;
   for (int64_t ch = blockIdx.x; ch < S.nchunks; ch += gridDim.x) {
     if (S.st[S.cseg[ch]].done) continue;
-    double dot = 0.0;
-    const int64_t b0 = S.cbeg[ch] / P;
+    const int64_t b = S.cbeg[ch], b0 = b / P;
+    const int len = (int)(S.cend[ch] - b);
     const int nb = (int)(S.cend[ch] / P - b0);
     const int step = wpb * NPW;
     // this lane group's node of the round and of the next one, with its row
@@ -518,14 +544,21 @@ k_seg_spmv(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ npt
           const int64_t d = P * B + j;
           const double v = fixed[d] ? 0.0 : acc[j];
           c[d] = v;
-          dot = __fma_rn(u[d], v, dot);
+          sC[d - b] = v;
         }
       }
       B = Bn;
       q0 = q0n;
       q1 = q1n;
     }
-    double s = block_sum(dot);
+    __syncthreads();
+    double dot = 0.0;
+#pragma unroll
+    for (int k = 0; k < CHUNK_PER_THREAD; ++k) {
+      const int i = threadIdx.x + k * CG_THREADS;
+      if (i < len) dot = __fma_rn(u[b + i], sC[i], dot);
+    }
+    const double s = block_sum(dot);
     if (threadIdx.x == 0) part[ch] = s;
     const int sg = S.cseg[ch];
     if (arrive_last(S.arrive + sg, S.sfirst[sg + 1] - S.sfirst[sg])) {
@@ -593,18 +626,18 @@ k_seg_update_fused(Seg S, double *__restrict__ xw, double *__restrict__ r, const
         zr = __fma_rn(zi, r[i], zr);
       }
     }
-    const double s1 = block_sum(rr);
-    const double s2 = local_prec ? block_sum(zr) : 0.0;
+    double sums[2] = {rr, zr};
+    block_sums<2>(sums);
     if (threadIdx.x == 0) {
-      part[ch] = s1;
-      if (local_prec) part2[ch] = s2;
+      part[ch] = sums[0];
+      if (local_prec) part2[ch] = sums[1];
     }
     if (arrive_last(S.arrive + S.nseg + sg, S.sfirst[sg + 1] - S.sfirst[sg])) {
       const double trr = seg_total_l2(S, sg, part);
       const double tzr = local_prec ? seg_total_l2(S, sg, part2) : 0.0;
       if (threadIdx.x == 0) {
         const bool done = seg_set_finish(S, sg, trr);
-        if (local_prec && !done) S.st[sg].rho = tzr;
+        if (local_prec && !done) seg_set_rho(S.st[sg], tzr);
       }
     }
   }
@@ -856,7 +889,7 @@ k_seg_zr(Seg S, const float *__restrict__ zf, const double *__restrict__ r, doub
     const int sg = S.cseg[ch];
     if (arrive_last(S.arrive + 2 * S.nseg + sg, S.sfirst[sg + 1] - S.sfirst[sg])) {  // rho = z.r
       const double t = seg_total_l2(S, sg, part);
-      if (threadIdx.x == 0) S.st[sg].rho = t;
+      if (threadIdx.x == 0) seg_set_rho(S.st[sg], t);
     }
   }
 }
@@ -1305,7 +1338,7 @@ __global__ void __launch_bounds__(CG_THREADS) k_mx_dir(Seg S, const float *__res
   for (int64_t ch = blockIdx.x; ch < S.nchunks; ch += gridDim.x) {
     const SegState &q = S.st[S.cseg[ch]];
     if (q.done) continue;
-    const float beta = __double2float_rn(q.rho / q.rho_prev);
+    const float beta = __double2float_rn(q.beta);
     const int64_t b = S.cbeg[ch], e = S.cend[ch];
 #pragma unroll
     for (int k = 0; k < CHUNK_PER_THREAD; ++k) {
@@ -1412,11 +1445,10 @@ k_mx_update(Seg S, double *__restrict__ xw, float *__restrict__ r, const float *
         SegState &w = S.st[sg];
         const double res32 = sqrt(trr);
         w.it += 1;
-        w.rho_prev = w.rho;
         if (res32 <= w.tol || res32 <= MX_DELTA * w.rmax || w.it >= w.maxiter || !isfinite(res32)) {
           w.upd = 1;
         } else if (local_prec) {
-          w.rho = tzr;
+          seg_set_rho(w, tzr);
         }
       }
     }
@@ -1501,7 +1533,7 @@ k_mx_true(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ nptr
           atomicSub(S.active, 1);
         } else {
           q.rmax = q.res;
-          if (local_prec) q.rho = tzr;
+          if (local_prec) seg_set_rho(q, tzr);
         }
       }
     }
@@ -1525,7 +1557,7 @@ k_mx_zr(Seg S, const float *__restrict__ zf, const float *__restrict__ r, double
     const int sg = S.cseg[ch];
     if (arrive_last(S.arrive + 2 * S.nseg + sg, S.sfirst[sg + 1] - S.sfirst[sg])) {
       const double t = seg_total_l2(S, sg, part);
-      if (threadIdx.x == 0) S.st[sg].rho = t;
+      if (threadIdx.x == 0) seg_set_rho(S.st[sg], t);
     }
   }
 }
@@ -2081,7 +2113,7 @@ __global__ void __launch_bounds__(CG_THREADS) k_eng_dir(EngTab T, unsigned *ctr)
     const SegState &q = T.st[sl];
     if (q.done) continue;
     const EngSlot &S = T.slot[sl];
-    const double beta = q.rho / q.rho_prev;
+    const double beta = q.beta;
     const int64_t b = T.cbeg[ch], e = T.cend[ch];
 #pragma unroll
     for (int k = 0; k < CHUNK_PER_THREAD; ++k) {
@@ -2095,14 +2127,15 @@ __global__ void __launch_bounds__(CG_THREADS) k_eng_dir(EngTab T, unsigned *ctr)
 template <int P>
 __global__ void __launch_bounds__(CG_THREADS) k_eng_spmv(EngTab T, unsigned *ctr) {
   constexpr int NPW = 32 / SPMV_G;
+  __shared__ double sC[CHUNK];
   const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5, w = threadIdx.x >> 5, g = lane % SPMV_G;
   const int64_t nch = *T.nchunks;
   for (int64_t ch = eng_next(ctr); ch < nch; ch = eng_next(ctr)) {
     const int sl = T.cslot[ch];
     if (T.st[sl].done) continue;
     const EngSlot &S = T.slot[sl];
-    double dot = 0.0;
-    const int64_t b0 = T.cbeg[ch] / P;
+    const int64_t b = T.cbeg[ch], b0 = b / P;
+    const int len = (int)(T.cend[ch] - b);
     const int nb = (int)(T.cend[ch] / P - b0);
     const int step = wpb * NPW;
     auto node_of = [&](int r) -> int64_t { return b0 + (r < nb ? (int)S.perm[b0 + r] : 0); };
@@ -2122,12 +2155,19 @@ __global__ void __launch_bounds__(CG_THREADS) k_eng_spmv(EngTab T, unsigned *ctr
           const int64_t d = P * B + j;
           const double v = S.fixed[d] ? 0.0 : acc[j];
           S.c[d] = v;
-          dot = __fma_rn(S.u[d], v, dot);
+          sC[d - b] = v;
         }
       }
       B = Bn;
       q0 = q0n;
       q1 = q1n;
+    }
+    __syncthreads();
+    double dot = 0.0;
+#pragma unroll
+    for (int k = 0; k < CHUNK_PER_THREAD; ++k) {
+      const int i = threadIdx.x + k * CG_THREADS;
+      if (i < len) dot = __fma_rn(S.u[b + i], sC[i], dot);
     }
     const double s = block_sum(dot);
     if (threadIdx.x == 0) T.part3[ch] = s;
@@ -2176,11 +2216,11 @@ __global__ void __launch_bounds__(CG_THREADS) k_eng_update(EngTab T, unsigned *c
       S.z[i] = zi;
       zr = __fma_rn(zi, S.r[i], zr);
     }
-    const double s1 = block_sum(rr);
-    const double s2 = block_sum(zr);
+    double sums[2] = {rr, zr};
+    block_sums<2>(sums);
     if (threadIdx.x == 0) {
-      T.part[ch] = s1;
-      T.part2[ch] = s2;
+      T.part[ch] = sums[0];
+      T.part2[ch] = sums[1];
     }
     if (arrive_last(T.arrive + 2 * sl + 1, T.snch[sl])) {
       const double trr = eng_total(T, sl, T.part);
@@ -2188,10 +2228,9 @@ __global__ void __launch_bounds__(CG_THREADS) k_eng_update(EngTab T, unsigned *c
       if (threadIdx.x == 0) {
         SegState &w = T.st[sl];
         w.res = sqrt(trr);
-        w.rho_prev = w.rho;
         w.it += 1;
         if (w.res <= w.tol || w.it >= w.maxiter) w.done = 1;
-        else w.rho = tzr;
+        else seg_set_rho(w, tzr);
       }
     }
   }
