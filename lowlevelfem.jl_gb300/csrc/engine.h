@@ -10,7 +10,7 @@
 // over whatever the tables hold.  Systems are admitted and retired between
 // replays, so a request that arrives while others iterate joins the next
 // replay instead of waiting for the batch to drain.  Each system keeps its
-// own chunks (768 DoFs from its first DoF), scalars and reductions in chunk
+// own chunks (of chunk_dofs DoFs from its first DoF), scalars and reductions in chunk
 // order, so its iterates are those of a lone llf_pcg bit for bit.
 #pragma once
 #include <stdint.h>
@@ -33,6 +33,10 @@ struct Done {
   std::vector<double> x;   // the solution, fixed entries kept
 };
 
+// Marks a context whose kernels run beside those of other contexts (a
+// server's): its solves keep to launches that leave the SMs to others.
+void share_gpu(llf_ctx *ctx);
+
 // Set up the CG of K x = b (fixed entries of x0 prescribed; host arrays of
 // K's DoF count) on ctx's stream, with a local preconditioner (none, Jacobi,
 // block Jacobi).  Synchronises ctx's stream.  K must outlive the system.
@@ -41,7 +45,7 @@ int prepare(llf_ctx *ctx, const llf_matrix *K, const double *b, const double *x0
 void release(llf_ctx *ctx, System *sys);
 
 // An engine on ctx (its stream runs the iterations) for at most max_systems
-// systems of at most max_chunks chunks (768 DoFs) in total.
+// systems of at most max_chunks chunks in total.
 int create(llf_ctx *ctx, int max_systems, int64_t max_chunks, Engine **out);
 void destroy(Engine *e);
 

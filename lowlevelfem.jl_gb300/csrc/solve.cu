@@ -32,14 +32,25 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <mutex>
 
 namespace {
 
 constexpr int CG_THREADS = 256;
-constexpr int CHUNK = 768;  // DoFs per reduction chunk (a multiple of every pdim: chunks hold whole nodes)
+constexpr int CHUNK = 768;  // most DoFs per reduction chunk
 constexpr int CHUNK_PER_THREAD = CHUNK / CG_THREADS;  // a chunk's DoFs per thread of its block
 static_assert(CHUNK % CG_THREADS == 0, "a chunk is whole rounds of a block");
+// DoFs per chunk of a system of n DoFs (a multiple of every pdim: chunks hold
+// whole nodes): small systems are cut into chunks for every SM, down to 192
+// DoFs, whose sums still cost less than their products.  A function of the
+// system alone, so that its sums do not depend on what else is in a batch.
+constexpr int64_t CHUNKS_WANTED = 148;
+__host__ __device__ inline int chunk_dofs(int64_t n) {
+  const int64_t c = ((n + CHUNKS_WANTED - 1) / CHUNKS_WANTED + 5) / 6 * 6;
+  return (int)(c < 192 ? 192 : (c > CHUNK ? CHUNK : c));
+}
+inline int64_t chunk_count(int64_t n) { return (n + chunk_dofs(n) - 1) / chunk_dofs(n); }
 
 // Work vectors of the mixed-precision CG (FP32 matrix copy and vectors, the
 // FP64 right-hand side minus the prescribed values' product).
@@ -396,19 +407,24 @@ k_seg_init(Seg S, const double *__restrict__ b, const double *__restrict__ y,
   }
 }
 
-__device__ __forceinline__ double seg_total(const Seg &S, int s, const double *part) {
+// Sum of a system's n partials in a fixed order (thread t: t, t + 256, ...,
+// then block_sum), result valid in thread 0.
+template <class F>
+__device__ __forceinline__ double total_of(int64_t n, F part) {
   double v = 0.0;
-  for (int64_t ch = S.sfirst[s] + threadIdx.x; ch < S.sfirst[s + 1]; ch += blockDim.x) v = __dadd_rn(v, part[ch]);
+  for (int64_t k = threadIdx.x; k < n; k += blockDim.x) v = __dadd_rn(v, part(k));
   return block_sum(v);
+}
+__device__ __forceinline__ double seg_total(const Seg &S, int s, const double *part) {
+  const int64_t f = S.sfirst[s];
+  return total_of(S.sfirst[s + 1] - f, [&](int64_t k) { return part[f + k]; });
 }
 
 // The same sum read through L2 (partials written by other blocks of the
 // same launch).
 __device__ __forceinline__ double seg_total_l2(const Seg &S, int s, const double *part) {
-  double v = 0.0;
-  for (int64_t ch = S.sfirst[s] + threadIdx.x; ch < S.sfirst[s + 1]; ch += blockDim.x)
-    v = __dadd_rn(v, __ldcg(part + ch));
-  return block_sum(v);
+  const int64_t f = S.sfirst[s];
+  return total_of(S.sfirst[s + 1] - f, [&](int64_t k) { return __ldcg(part + f + k); });
 }
 
 // Segment state after the alpha reduction (u.c) / the residual reduction.
@@ -656,6 +672,405 @@ __global__ void k_keep_fixed(const double *__restrict__ x, const uint8_t *__rest
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     xc[i] = fixed[i] ? x[i] : 0.0;
+}
+
+// ---------------------------------------------------------------- resident CG
+// The whole iteration loop of systems of at most a few hundred chunks in one
+// cooperative kernel: one CTA per chunk, all resident, x, r, z, u and the
+// preconditioner of the chunk in registers, the chunk's node order, row
+// ranges and row nodes in shared memory.  The CTAs of one system meet three
+// times per iteration, each time at one word or word pair per chunk that every
+// CTA of the system polls: the new direction is written (the product reads it
+// from the other chunks), the partials of u.c, the partials of r.r and z.r.
+// Systems do not wait for one another.
+// What bounds the three launches per iteration that this replaces, for these
+// sizes, is latency: eight warps per SM in the product, and three launches
+// with two last-block reductions.  Here the FP64 pipe (16 SM cycles per warp
+// instruction) is what the phases between the meets cost, so no warp issues an
+// FP64 instruction that another one has issued: scalars are formed by one
+// thread, warps without work skip theirs.  Per iteration, with the launches
+// (after their own sums were packed) and here: 200x100 quad4 26.6 -> 14.2 us,
+// hex8 30^3 44 -> 27 us (the product's FP64 instructions alone take 13.8 us
+// of an interior chunk), tet10 heat, 90,945 nodes, 38 -> 20 us.
+// Every sum is formed as k_seg_spmv, k_seg_update_fused and seg_total form it
+// (256 virtual threads per chunk, then the chunks by 256 threads), whatever
+// the CTA size, so a solve gives the same bits as the launches and as the
+// serving engine.
+// Waits are bounded (RES_LIMIT_NS): a CTA that gives up sets *abort and
+// returns, every other one follows, and the host runs the launches instead
+// (x is written at the end only).
+constexpr unsigned long long RES_LIMIT_NS = 20000000000ull;   // 0: gives up at the first poll that fails
+
+// Meeting points: every chunk pushes its word pair {bits of the partial,
+// iteration} (or its word, the iteration whose direction is written) to a
+// place of its own in every chunk's row, and polls its own row: polling one
+// shared list made every SM read the same few L2 lines (7,400 cycles a meet
+// with 141 CTAs, 4,000 this way).  Row ch, column k at ch * nchunks + k.
+struct ResSync {
+  ulonglong2 *uc, *rr, *zr;
+  unsigned long long *dir;
+  unsigned *abort;
+  unsigned long long limit;   // ns
+};
+
+__device__ __forceinline__ unsigned long long res_now() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+// One 16-byte access each: value and iteration arrive together.
+__device__ __forceinline__ void res_put(ulonglong2 *p, double v, unsigned long long it) {
+  asm volatile("{\n\t.reg .b128 q;\n\tmov.b128 q, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], q;\n\t}"
+               ::"l"(p), "l"(__double_as_longlong(v)), "l"(it) : "memory");
+}
+__device__ __forceinline__ ulonglong2 res_get(const ulonglong2 *p) {
+  ulonglong2 v;
+  asm volatile("{\n\t.reg .b128 q;\n\tld.relaxed.gpu.global.b128 q, [%2];\n\tmov.b128 {%0, %1}, q;\n\t}"
+               : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void res_fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+// Polls until done() (a relaxed load) is true; false: gave up.
+template <class F>
+__device__ __forceinline__ bool res_poll(const ResSync &Y, F done) {
+  unsigned long long t0 = 0;
+  for (unsigned n = 0;; ++n) {
+    if (done()) return true;
+    if (Y.limit == 0) return false;
+    if ((n & 1023u) == 1023u) {
+      if (t0 == 0) t0 = res_now();
+      else if (res_now() - t0 > Y.limit || *(volatile const unsigned *)Y.abort) return false;
+    }
+  }
+}
+// The value of slot p of iteration it.
+__device__ __forceinline__ bool res_wait(const ulonglong2 *p, unsigned long long it, double &v, const ResSync &Y) {
+  return res_poll(Y, [&]() {
+    const ulonglong2 q = res_get(p);
+    v = __longlong_as_double((long long)q.x);
+    return q.y == it;
+  });
+}
+__device__ __forceinline__ bool res_wait_dir(const unsigned long long *p, unsigned long long it, const ResSync &Y) {
+  return res_poll(Y, [&]() {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v == it;
+  });
+}
+
+// block_sums' tree on the 256 values sv[0..255] of sum k: its first part by
+// warps 4k .. 4k+3, the last by any one warp, between two barriers.
+__device__ __forceinline__ void res_fold(const double *sv, double *sw, int w, int lane) {
+  const int q = w & 3;
+  const double *s = sv + (2 * q + (lane >> 4)) * 32 + (lane & 15);
+  double t = __dadd_rn(s[0], s[16]);
+#pragma unroll
+  for (int off = 8; off > 0; off >>= 1) t = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, off));
+  if ((lane & 15) == 0) sw[2 * q + (lane >> 4)] = t;
+}
+__device__ __forceinline__ double res_last(const double *sw, int lane) {
+  double t = lane < 8 ? sw[lane] : 0.0;
+#pragma unroll
+  for (int off = 4; off > 0; off >>= 1) t = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, off));
+  return t;
+}
+
+// The P columns of one node by u, the lane group's share (node_columns_at's
+// order).  u was written by other CTAs of this launch, so it is read through
+// plain loads (never the read-only path) after the acquire of the wait.
+template <int P>
+__device__ __forceinline__ void res_columns(const double *__restrict__ col, const int32_t *adj, const double *u, int n,
+                                            int g, double (&acc)[P]) {
+#pragma unroll
+  for (int j = 0; j < P; ++j) acc[j] = 0.0;
+  int k = g;
+  int32_t ra = k < n ? adj[k / P] : 0, rb = k + SPMV_G < n ? adj[(k + SPMV_G) / P] : 0;
+  for (; k + SPMV_G < n; k += 2 * SPMV_G) {
+    const int k2 = k + SPMV_G, kn = k + 2 * SPMV_G;
+    double v[P], v2[P];
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+      v[j] = __ldg(col + (int64_t)j * n + k);
+      v2[j] = __ldg(col + (int64_t)j * n + k2);
+    }
+    const double xa = __ldca(u + (int64_t)P * ra + k % P);
+    const double xb = __ldca(u + (int64_t)P * rb + k2 % P);
+    ra = kn < n ? adj[kn / P] : 0;
+    rb = kn + SPMV_G < n ? adj[(kn + SPMV_G) / P] : 0;
+#pragma unroll
+    for (int j = 0; j < P; ++j) acc[j] = __fma_rn(v2[j], xb, __fma_rn(v[j], xa, acc[j]));
+  }
+  if (k < n) {
+    const double xa = __ldca(u + (int64_t)P * ra + k % P);
+#pragma unroll
+    for (int j = 0; j < P; ++j) acc[j] = __fma_rn(__ldg(col + (int64_t)j * n + k), xa, acc[j]);
+  }
+}
+
+// Shared memory: u, c (then z), r of the chunk [3 CHUNK doubles] | values and
+// partial sums of two sums [2 x (256 + 8)] | scalars [4] | per position of the
+// node order: first row node (relative), row nodes, node and (from bit 16)
+// its fixed DoFs [CHUNK / P each, int] | row nodes of the chunk [adj_cap ints].
+constexpr int RES_SCALARS = 2 * (256 + 8) + 4;
+template <int P>
+constexpr size_t res_smem_fixed() {
+  return sizeof(double) * (3 * CHUNK + RES_SCALARS) + sizeof(int) * 3 * (CHUNK / P);
+}
+
+template <int P, int T>
+__global__ void __launch_bounds__(T, 1024 / T)
+k_cg_resident(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ nptr, const int32_t *__restrict__ nadj,
+              const uint8_t *__restrict__ fixed, const double *__restrict__ r0, const double *__restrict__ z0,
+              double *u, double *xw, const double *__restrict__ pinv, int mode, ResSync Y, int adj_cap) {
+  extern __shared__ double rsm[];
+  constexpr int NPT = (CHUNK + T - 1) / T, NODES = CHUNK / P;
+  constexpr bool PV = NPT * P <= 4;   // preconditioner in registers
+  double *sU = rsm, *sC = sU + CHUNK, *sR = sC + CHUNK;
+  double *sv0 = sR + CHUNK, *sv1 = sv0 + 256, *sw0 = sv1 + 256, *sw1 = sw0 + 8, *sq = sw1 + 8;
+  int *sFirst = reinterpret_cast<int *>(sq + 4), *sDeg = sFirst + NODES, *sNode = sDeg + NODES, *sAdj = sNode + NODES;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = threadIdx.x % SPMV_G;
+  const int64_t ch = blockIdx.x;
+  const int sg = S.cseg[ch];
+  SegState *st = S.st + sg;
+  if (st->done) return;   // the same for every CTA of the system
+  // sq: alpha, beta, rho, 1.0 when the loop ends
+  double res = st->res, tol = st->tol;         // thread 0's
+  long long iters = st->it, maxiter = st->maxiter;
+  int breakdown = 0;
+  if (threadIdx.x == 0) {
+    sq[0] = 0.0;
+    sq[1] = st->beta;
+    sq[2] = st->rho;
+    sq[3] = 0.0;
+  }
+  const int64_t first = S.sfirst[sg];
+  const int nch = (int)(S.sfirst[sg + 1] - first);
+  const int64_t b = S.cbeg[ch], B0 = b / P;
+  const int len = (int)(S.cend[ch] - b), nb = len / P;
+  const int64_t a0 = nptr[B0];
+  const int na = (int)(nptr[B0 + nb] - a0);
+  const bool adj_here = na <= adj_cap;
+  for (int p = threadIdx.x; p < nb; p += T) {
+    const int k = S.perm ? (int)S.perm[B0 + p] : p;
+    int fm = 0;
+#pragma unroll
+    for (int j = 0; j < P; ++j) fm |= fixed[b + P * k + j] ? 0x10000 << j : 0;
+    sNode[p] = k | fm;
+    sFirst[p] = (int)(nptr[B0 + k] - a0);
+    sDeg[p] = (int)(nptr[B0 + k + 1] - nptr[B0 + k]);
+  }
+  if (adj_here)
+    for (int k = threadIdx.x; k < na; k += T) sAdj[k] = nadj[a0 + k];
+  double x[NPT], r[NPT], z[NPT], d[NPT], pv[PV ? NPT : 1][P];
+  bool fx[NPT];
+#pragma unroll
+  for (int k = 0; k < NPT; ++k) {
+    const int i = threadIdx.x + k * T;
+    x[k] = r[k] = z[k] = d[k] = 0.0;
+    fx[k] = true;
+    if (PV)
+#pragma unroll
+      for (int j = 0; j < P; ++j) pv[PV ? k : 0][j] = 0.0;
+    if (i < len) {
+      x[k] = xw[b + i];
+      r[k] = r0[b + i];
+      z[k] = z0[b + i];
+      d[k] = u[b + i];
+      fx[k] = fixed[b + i] != 0;
+      if (PV && mode == LLF_PRECOND_BJACOBI) {
+#pragma unroll
+        for (int j = 0; j < P; ++j) pv[PV ? k : 0][j] = pinv[(b + i) * P + j];
+      } else if (PV) {
+        pv[PV ? k : 0][0] = pinv[b + i];
+      }
+    }
+  }
+  bool fail = false;
+  __syncthreads();
+  for (unsigned long long it = 1;; ++it) {
+    // u = z + beta u
+    const double beta = sq[1];
+#pragma unroll
+    for (int k = 0; k < NPT; ++k) {
+      const int i = threadIdx.x + k * T;
+      if (i < len) {
+        d[k] = __fma_rn(beta, d[k], z[k]);
+        sU[i] = d[k];
+        u[b + i] = d[k];
+      }
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < nch) res_fence();   // release: this chunk's direction
+    for (int k = threadIdx.x; k < nch; k += T)
+      asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(Y.dir + (first + k) * S.nchunks + ch), "l"(it) : "memory");
+    for (int k = threadIdx.x; k < nch && !fail; k += T)
+      fail = !res_wait_dir(Y.dir + ch * S.nchunks + first + k, it, Y);
+    if ((int)threadIdx.x < nch) res_fence();   // acquire: the other chunks' directions
+    if (__syncthreads_or(fail)) break;
+    // c = A u, SPMV_G lanes per node
+    for (int p0 = (w << 5) / SPMV_G; p0 < nb; p0 += T / SPMV_G) {   // the warp's first position
+      const int p = p0 + lane / SPMV_G;
+      const bool valid = p < nb;
+      const int deg = valid ? sDeg[p] : 0, at = valid ? sFirst[p] : 0;
+      double acc[P];
+      const double *col = nz + (int64_t)P * P * (a0 + at);
+      if (adj_here) res_columns<P>(col, sAdj + at, u, deg * P, g, acc);
+      else res_columns<P>(col, nadj + a0 + at, u, deg * P, g, acc);
+#pragma unroll
+      for (int off = SPMV_G / 2; off > 0; off >>= 1)
+#pragma unroll
+        for (int j = 0; j < P; ++j) acc[j] = __dadd_rn(acc[j], __shfl_xor_sync(0xffffffffu, acc[j], off));
+      if (valid && g == 0) {
+        const int k = sNode[p];
+#pragma unroll
+        for (int j = 0; j < P; ++j) sC[P * (k & 0xffff) + j] = (k >> (16 + j)) & 1 ? 0.0 : acc[j];
+      }
+    }
+    __syncthreads();
+    // the chunk's u.c: virtual thread t takes DoFs t, t + 256, t + 512
+    if (threadIdx.x < 256) {
+      double s = 0.0;
+      for (int i = threadIdx.x; i < len; i += 256) s = __fma_rn(sU[i], sC[i], s);
+      sv0[threadIdx.x] = s;
+    }
+    double cm[NPT];
+#pragma unroll
+    for (int k = 0; k < NPT; ++k) {
+      const int i = threadIdx.x + k * T;
+      cm[k] = i < len ? sC[i] : 0.0;
+    }
+    __syncthreads();
+    if (w < 4) res_fold(sv0, sw0, w, lane);
+    __syncthreads();
+    if (w == 0) {
+      const double s = __shfl_sync(0xffffffffu, res_last(sw0, lane), 0);
+      for (int k = lane; k < nch; k += 32) res_put(Y.uc + (first + k) * S.nchunks + ch, s, it);
+    }
+    // the system's u.c and alpha
+    if (threadIdx.x < 256) {
+      double s = 0.0;
+      for (int k = threadIdx.x; k < nch && !fail; k += 256) {
+        double v = 0.0;
+        fail = !res_wait(Y.uc + ch * S.nchunks + first + k, it, v, Y);
+        s = __dadd_rn(s, v);
+      }
+      sv0[threadIdx.x] = s;
+    }
+    if (__syncthreads_or(fail)) break;
+    if (w < 4) res_fold(sv0, sw0, w, lane);
+    __syncthreads();
+    if (w == 0) {
+      const double uc = res_last(sw0, lane);
+      if (lane == 0) {
+        if (!(uc > 0.0) || !isfinite(uc)) {
+          breakdown = 1;
+          sq[3] = 1.0;
+        } else {
+          sq[0] = sq[2] / uc;
+        }
+      }
+    }
+    __syncthreads();
+    if (sq[3] != 0.0) break;
+    // x += alpha u, r -= alpha c, z = M^-1 r
+    const double alpha = sq[0];
+#pragma unroll
+    for (int k = 0; k < NPT; ++k) {
+      const int i = threadIdx.x + k * T;
+      if (i < len) {
+        x[k] = __fma_rn(alpha, d[k], x[k]);
+        r[k] = __fma_rn(-alpha, cm[k], r[k]);
+        sR[i] = r[k];
+      }
+    }
+    if (mode == LLF_PRECOND_BJACOBI) __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NPT; ++k) {
+      const int i = threadIdx.x + k * T;
+      if (i < len) {
+        double zi;
+        if (mode == LLF_PRECOND_BJACOBI) {
+          const double *rn = sR + (i / P) * P;
+          zi = 0.0;
+#pragma unroll
+          for (int j = 0; j < P; ++j) zi = __fma_rn(PV ? pv[PV ? k : 0][j] : __ldg(pinv + (b + i) * P + j), rn[j], zi);
+        } else {
+          zi = __dmul_rn(PV ? pv[PV ? k : 0][0] : __ldg(pinv + b + i), r[k]);
+        }
+        z[k] = fx[k] ? 0.0 : zi;
+        sC[i] = z[k];
+      }
+    }
+    __syncthreads();
+    // the chunk's r.r (threads 0..255) and z.r (256..511, or the same threads)
+    if (threadIdx.x < 512) {
+      const int t = threadIdx.x & 255;
+      double s = 0.0;
+      const double *a = T > 256 && threadIdx.x >= 256 ? sC : sR;
+      for (int i = t; i < len; i += 256) s = __fma_rn(a[i], sR[i], s);
+      (T > 256 && threadIdx.x >= 256 ? sv1 : sv0)[t] = s;
+      if (T == 256) {
+        s = 0.0;
+        for (int i = t; i < len; i += 256) s = __fma_rn(sC[i], sR[i], s);
+        sv1[t] = s;
+      }
+    }
+    __syncthreads();
+    if (w < 8) res_fold(w < 4 ? sv0 : sv1, w < 4 ? sw0 : sw1, w, lane);
+    __syncthreads();
+    if (w < 2) {
+      const double s = __shfl_sync(0xffffffffu, res_last(w == 0 ? sw0 : sw1, lane), 0);
+      for (int k = lane; k < nch; k += 32) res_put((w == 0 ? Y.rr : Y.zr) + (first + k) * S.nchunks + ch, s, it);
+    }
+    // the system's r.r and z.r
+    if (threadIdx.x < 512) {
+      const int t = threadIdx.x & 255;
+      const bool second = T > 256 && threadIdx.x >= 256;
+      double s = 0.0, s2 = 0.0;
+      for (int k = t; k < nch && !fail; k += 256) {
+        double v = 0.0;
+        fail = !res_wait((second ? Y.zr : Y.rr) + ch * S.nchunks + first + k, it, v, Y);
+        s = __dadd_rn(s, v);
+        if (T == 256) {
+          fail = fail || !res_wait(Y.zr + ch * S.nchunks + first + k, it, v, Y);
+          s2 = __dadd_rn(s2, v);
+        }
+      }
+      (second ? sv1 : sv0)[t] = s;
+      if (T == 256) sv1[t] = s2;
+    }
+    if (__syncthreads_or(fail)) break;
+    if (w < 8) res_fold(w < 4 ? sv0 : sv1, w < 4 ? sw0 : sw1, w, lane);
+    __syncthreads();
+    if (w < 2) {   // the residual check beside the next rho and beta
+      const double s = res_last(w == 0 ? sw0 : sw1, lane);
+      if (threadIdx.x == 0) {
+        res = sqrt(s);
+        iters += 1;
+        if (res <= tol || iters >= maxiter) sq[3] = 1.0;
+      } else if (threadIdx.x == 32) {
+        sq[1] = s / sq[2];
+        sq[2] = s;
+      }
+    }
+    __syncthreads();
+    if (sq[3] != 0.0) break;
+  }
+  if (fail) atomicExch(Y.abort, 1u);
+  __syncthreads();
+  if (sq[3] == 0.0) return;   // gave up
+#pragma unroll
+  for (int k = 0; k < NPT; ++k) {
+    const int i = threadIdx.x + k * T;
+    if (i < len) xw[b + i] = x[k];
+  }
+  if (ch == first && threadIdx.x == 0) {
+    st->breakdown = breakdown;
+    st->res = res;
+    st->it = iters;
+    st->done = 1;
+  }
 }
 
 // IC(0) application z = (L L^T)^-1 r in FP32, one colour per launch, eight
@@ -997,13 +1412,111 @@ template <int P>
 int pcg_core(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double *d_x, const uint8_t *d_fixed,
              const Seg &S, double *r, double *z, double *u, double *c, double *xw, double *pinv,
              double *part, double *part2, double *part3, int precond, double reltol, int64_t maxiter, bool use_graph,
-             SegState *hst, const IcApply &ic = IcApply());
+             SegState *hst, const IcApply &ic = IcApply(), unsigned long long *sync = nullptr);
 int pcg_outcome(llf_ctx *ctx, int nseg, const SegState *hst, int64_t *iters, double *relres);
 template <int P>
 int pcg_mixed_core(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double *d_x, const uint8_t *d_fixed,
                    const Seg &S, const MixedBufs &B, double *xw, double *tmp, double *pinv, double *part,
                    double *part2, double *part3, int precond, double reltol, int64_t maxiter, bool use_graph,
                    SegState *hst, const IcApply &ic);
+
+constexpr int64_t RES_MAX_CHUNKS = 1024;
+// Words of the resident CG's meeting points for nch chunks (zeroed before
+// every launch): three word pairs and one word per pair of chunks, and the
+// abort flag; none for a solve that has too many chunks.
+inline int64_t res_sync_words(int64_t nch) { return nch > RES_MAX_CHUNKS ? 0 : 7 * nch * nch + 2; }
+
+// One resident CG per device at a time: two of them could each hold SMs that
+// the other waits for.  Another solve takes the launches meanwhile.
+std::mutex g_res_mutex[128];
+
+// Systems not done (one block).
+__global__ void k_count_active(Seg S) {
+  __shared__ int n;
+  if (threadIdx.x == 0) n = 0;
+  __syncthreads();
+  for (int g = threadIdx.x; g < S.nseg; g += blockDim.x)
+    if (!S.st[g].done) atomicAdd(&n, 1);
+  __syncthreads();
+  if (threadIdx.x == 0) *S.active = n;
+}
+
+template <int P, int T>
+int launch_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const double *r, const double *z, double *u,
+                    double *xw, const double *pinv, const uint8_t *fixed, int precond, unsigned long long *sync,
+                    bool *done) {
+  const llf_pattern *pat = m->pat;
+  const int64_t nch = S.nchunks;
+  cudaStream_t s = ctx->stream;
+  auto fn = k_cg_resident<P, T>;
+  // row nodes in shared memory as far as the CTA's share of the SM goes
+  const size_t fixed_b = res_smem_fixed<P>(), room = (size_t)(216 * 1024) / (1024 / T);
+  const int adj_cap = (int)std::min<int64_t>((int64_t)(CHUNK / P) * std::max(pat->max_deg, 1),
+                                             (int64_t)((room - fixed_b) / sizeof(int)));
+  const size_t smem = fixed_b + sizeof(int) * (size_t)adj_cap;
+  LLF_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per_sm = 0;
+  LLF_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, T, smem));
+  if ((int64_t)per_sm * ctx->num_sms < nch) return LLF_OK;
+  const int64_t words = res_sync_words(nch);
+  LLF_CUDA_TRY(ctx, cudaMemsetAsync(sync, 0, sizeof(unsigned long long) * words, s));
+  ulonglong2 *pairs = reinterpret_cast<ulonglong2 *>(sync);
+  const int64_t sq = nch * nch;
+  const char *lim = getenv("LLF_RESIDENT_WAIT_NS");   // tests: 0 makes the waits run out
+  const unsigned long long limit = lim ? strtoull(lim, nullptr, 10) : RES_LIMIT_NS;
+  ResSync Y{pairs, pairs + sq, pairs + 2 * sq, sync + 6 * sq, reinterpret_cast<unsigned *>(sync + 7 * sq), limit};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)nch);
+  cfg.blockDim = dim3(T);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  {
+    KernelScope k(ctx, "k_cg_resident");
+    if (cudaLaunchKernelEx(&cfg, fn, S, (const double *)m->d_nz, (const int64_t *)pat->d_nptr,
+                           (const int32_t *)pat->d_nadj, fixed, r, z, u, xw, pinv, precond, Y, adj_cap) != cudaSuccess) {
+      cudaGetLastError();   // not all CTAs can be resident here (a partitioned GPU)
+      return LLF_OK;
+    }
+  }
+  unsigned aborted = 1;
+  LLF_CUDA_TRY(ctx, cudaMemcpyAsync(&aborted, Y.abort, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+  LLF_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+  *done = aborted == 0;
+  if (*done) {
+    LLF_CUDA_TRY(ctx, cudaMemsetAsync(S.active, 0, sizeof(int), s));
+  } else {   // the launches start from the first direction; systems that finished stay done
+    LLF_CUDA_TRY(ctx, cudaMemsetAsync(u, 0, sizeof(double) * pat->ndof, s));
+    k_count_active<<<1, CG_THREADS, 0, s>>>(S);
+    LLF_CUDA_TRY(ctx, cudaGetLastError());
+  }
+  return LLF_OK;
+}
+
+// The resident CG when every chunk gets a CTA at once: the largest CTA whose
+// chunks still fit, one per SM (the product's loads then have all the warps
+// an SM holds, whatever the number of chunks), else two or four per SM.
+// *done = false: the caller runs the launches.
+template <int P>
+int run_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const double *r, const double *z, double *u,
+                 double *xw, const double *pinv, const uint8_t *fixed, int precond, unsigned long long *sync,
+                 bool *done) {
+  *done = false;
+  const int64_t nch = S.nchunks;
+  if (nch < 1 || nch > std::min<int64_t>(4 * ctx->num_sms, RES_MAX_CHUNKS) || ctx->shares_gpu || ctx->device < 0 || ctx->device >= 128)
+    return LLF_OK;
+  std::unique_lock<std::mutex> lock(g_res_mutex[ctx->device], std::try_to_lock);
+  if (!lock.owns_lock()) return LLF_OK;
+  if (nch <= ctx->num_sms)
+    return launch_resident<P, 1024>(ctx, m, S, r, z, u, xw, pinv, fixed, precond, sync, done);
+  if (nch <= 2 * (int64_t)ctx->num_sms)
+    return launch_resident<P, 512>(ctx, m, S, r, z, u, xw, pinv, fixed, precond, sync, done);
+  return launch_resident<P, 256>(ctx, m, S, r, z, u, xw, pinv, fixed, precond, sync, done);
+}
 
 // Buffers, chunking and preconditioner of the segmented PCG for one matrix
 // and one set of fixed DoFs, built once and reused by every solve with them
@@ -1020,6 +1533,7 @@ struct PcgPlan {
   double *part2 = nullptr, *part3 = nullptr;
   int *d_arrive = nullptr;
   int16_t *d_perm = nullptr;
+  unsigned long long *d_sync = nullptr;   // resident CG: res_sync_words(nch) words
   Ic0Factor icf;
   IcApply ic;
   int32_t *d_node_seg = nullptr;
@@ -1041,9 +1555,10 @@ struct PcgPlan {
     sf.assign(nseg + 1, 0);
     for (int g = 0; g < nseg; ++g) {
       sf[g] = (int64_t)cb.size();
-      for (int64_t i = seg_off[g]; i < seg_off[g + 1]; i += CHUNK) {
+      const int size = chunk_dofs(seg_off[g + 1] - seg_off[g]);
+      for (int64_t i = seg_off[g]; i < seg_off[g + 1]; i += size) {
         cb.push_back(i);
-        ce.push_back(std::min(i + CHUNK, seg_off[g + 1]));
+        ce.push_back(std::min(i + size, seg_off[g + 1]));
         cs.push_back(g);
       }
     }
@@ -1073,6 +1588,7 @@ struct PcgPlan {
     LLF_CUDA_TRY(ctx, dalloc(ctx, &part, nch));
     LLF_CUDA_TRY(ctx, dalloc(ctx, &part2, nch));
     LLF_CUDA_TRY(ctx, dalloc(ctx, &part3, nch));
+    if (!mixed && precond != LLF_PRECOND_IC0) LLF_CUDA_TRY(ctx, dalloc(ctx, &d_sync, res_sync_words(nch)));
     LLF_CUDA_TRY(ctx, dalloc(ctx, &d_arrive, 3 * (int64_t)nseg));
     LLF_CUDA_TRY(ctx, cudaMemsetAsync(d_arrive, 0, sizeof(int) * 3 * nseg, s));
     if (nch) {
@@ -1115,7 +1631,7 @@ struct PcgPlan {
     int rc = mixed ? pcg_mixed_core<P>(ctx, m, d_b, d_x, d_fixed, S, mb, xw, c, pinv, part, part2, part3, precond,
                                        reltol, maxiter, !ctx->profiling, hst.data(), ic)
                    : pcg_core<P>(ctx, m, d_b, d_x, d_fixed, S, r, z, u, c, xw, pinv, part, part2, part3, precond,
-                                 reltol, maxiter, !ctx->profiling, hst.data(), ic);
+                                 reltol, maxiter, !ctx->profiling, hst.data(), ic, d_sync);
     if (rc != LLF_OK) return rc;
     return pcg_outcome(ctx, nseg, hst.data(), iters, relres);
   }
@@ -1129,7 +1645,7 @@ struct PcgPlan {
     dfree(ctx, d_cb); dfree(ctx, d_ce); dfree(ctx, d_cs); dfree(ctx, d_sf); dfree(ctx, d_active);
     dfree(ctx, d_st); dfree(ctx, r); dfree(ctx, z); dfree(ctx, u); dfree(ctx, c); dfree(ctx, xw);
     dfree(ctx, pinv); dfree(ctx, part); dfree(ctx, part2); dfree(ctx, part3); dfree(ctx, d_arrive);
-    dfree(ctx, d_perm);
+    dfree(ctx, d_perm); dfree(ctx, d_sync);
     dfree(ctx, mb.nz32); dfree(ctx, mb.r); dfree(ctx, mb.z); dfree(ctx, mb.u); dfree(ctx, mb.c); dfree(ctx, mb.rb);
   }
 };
@@ -1154,7 +1670,7 @@ template <int P>
 int pcg_core(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double *d_x, const uint8_t *d_fixed,
              const Seg &S, double *r, double *z, double *u, double *c, double *xw, double *pinv,
              double *part, double *part2, double *part3, int precond, double reltol, int64_t maxiter, bool use_graph,
-             SegState *hst, const IcApply &ic) {
+             SegState *hst, const IcApply &ic, unsigned long long *sync) {
   const llf_pattern *pat = m->pat;
   const int64_t n = pat->ndof;
   const int64_t nch = S.nchunks;
@@ -1176,6 +1692,19 @@ int pcg_core(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double *d_x, 
   { KernelScope k(ctx, "k_seg_start"); k_seg_start<<<gseg, CG_THREADS, 0, s>>>(S, part, reltol, (long long)maxiter); }
   enqueue_first_prec<P>(ctx, S, m, pinv, precond, r, z, d_fixed, part, gch, gseg, ic);
   LLF_CUDA_TRY(ctx, cudaGetLastError());
+
+  if (sync && precond != LLF_PRECOND_IC0) {
+    bool done = false;
+    const int rc = run_resident<P>(ctx, m, S, r, z, u, xw, pinv, d_fixed, precond, sync, &done);
+    if (rc != LLF_OK) return rc;
+    if (done) {
+      { KernelScope k(ctx, "k_cg_merge"); k_cg_merge<<<gv, CG_THREADS, 0, s>>>(xw, d_fixed, d_x, n); }
+      LLF_CUDA_TRY(ctx, cudaGetLastError());
+      LLF_CUDA_TRY(ctx, cudaMemcpyAsync(hst, S.st, sizeof(SegState) * nseg, cudaMemcpyDeviceToHost, s));
+      LLF_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+      return LLF_OK;
+    }
+  }
 
   // capture a run of iterations once, replay until every segment is done
   const int per_graph = 16;
@@ -1723,8 +2252,9 @@ namespace {
 __global__ void k_na_chunks(int64_t *cb, int64_t *ce, int32_t *cs, int64_t *sf, int64_t n, int64_t nch) {
   for (int64_t ch = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; ch < nch;
        ch += (int64_t)gridDim.x * blockDim.x) {
-    cb[ch] = ch * CHUNK;
-    ce[ch] = (ch + 1) * CHUNK < n ? (ch + 1) * CHUNK : n;
+    const int64_t size = chunk_dofs(n);
+    cb[ch] = ch * size;
+    ce[ch] = (ch + 1) * size < n ? (ch + 1) * size : n;
     cs[ch] = 0;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1782,7 +2312,7 @@ int pcg_noalloc_typed(llf_ctx *ctx, const llf_matrix *m, const double *d_b, doub
   int *arrive = active + 1;
   double *part2 = (double *)(base + NA_OFF_PART2), *part3 = (double *)(base + NA_OFF_PART3);
   int16_t *perm = (int16_t *)(base + NA_OFF_PERM);
-  const int64_t nch = (n + CHUNK - 1) / CHUNK;
+  const int64_t nch = chunk_count(n);
   // the array keeps the previous call's contents: the active-system counter
   // and the three arrival counters must start at zero; every other region
   // is written before it is read
@@ -2087,10 +2617,8 @@ struct EngTab {
 };
 
 __device__ __forceinline__ double eng_total(const EngTab &T, int sl, const double *part) {
-  double v = 0.0;
-  const int64_t f = T.sfirst[sl], n = T.snch[sl];
-  for (int64_t k = threadIdx.x; k < n; k += blockDim.x) v = __dadd_rn(v, __ldcg(part + f + k));
-  return block_sum(v);
+  const int64_t f = T.sfirst[sl];
+  return total_of(T.snch[sl], [&](int64_t k) { return __ldcg(part + f + k); });
 }
 
 // The chunks of a launch are handed out in table order from a counter (one
@@ -2240,6 +2768,8 @@ __global__ void __launch_bounds__(CG_THREADS) k_eng_update(EngTab T, unsigned *c
 
 namespace llf_engine {
 
+void share_gpu(llf_ctx *ctx) { ctx->shares_gpu = true; }
+
 struct System {
   const llf_matrix *K = nullptr;
   int P = 1, precond = 0;
@@ -2281,7 +2811,7 @@ int prepare_t(llf_ctx *ctx, const llf_matrix *K, const double *hb, const double 
   sy->P = P;
   sy->precond = precond;
   sy->ndof = n;
-  const int64_t nch = (n + CHUNK - 1) / CHUNK;
+  const int64_t nch = chunk_count(n);
   sy->nch = nch;
   LLF_CUDA_TRY(ctx, dalloc(ctx, &sy->b, n));
   LLF_CUDA_TRY(ctx, dalloc(ctx, &sy->x, n));
@@ -2301,8 +2831,8 @@ int prepare_t(llf_ctx *ctx, const llf_matrix *K, const double *hb, const double 
   std::vector<int64_t> cb(nch), ce(nch), sf{0, nch};
   std::vector<int32_t> cs(nch, 0);
   for (int64_t k = 0; k < nch; ++k) {
-    cb[k] = k * CHUNK;
-    ce[k] = std::min<int64_t>((k + 1) * CHUNK, n);
+    cb[k] = k * chunk_dofs(n);
+    ce[k] = std::min<int64_t>((k + 1) * chunk_dofs(n), n);
   }
   int64_t *d_cb = nullptr, *d_ce = nullptr, *d_sf = nullptr;
   int32_t *d_cs = nullptr;
@@ -2376,8 +2906,8 @@ int upload_table(Engine *e) {
     snch[sl] = sy->nch;
     for (int64_t k = 0; k < sy->nch; ++k) {
       cslot.push_back(sl);
-      cbeg.push_back(k * CHUNK);
-      cend.push_back(std::min<int64_t>((k + 1) * CHUNK, sy->ndof));
+      cbeg.push_back(k * chunk_dofs(sy->ndof));
+      cend.push_back(std::min<int64_t>((k + 1) * chunk_dofs(sy->ndof), sy->ndof));
     }
   }
   const int64_t nch = (int64_t)cslot.size();
