@@ -67,7 +67,8 @@ __host__ __device__ constexpr int sym_l(int n) {
 // to +0.0 before the inverse (oracle: orc_geom_affine).  For affine elements
 // geo[e*10 + 0..8] = invJ (row-major) and geo[e*10 + 9] = det; flag[e] = 2
 // for axis-aligned ones, else 1.  Elements with a negative material index
-// get flag 0; the others with flag 0 are counted in *nonaffine (if given).
+// get flag 0; the others with flag 0 are counted in nonaffine[0] (if given),
+// and nonaffine[1] is set when an element is affine.
 template <int DIM>
 __global__ void k_affine_geometry(const double *__restrict__ xyz, const int32_t *__restrict__ conn,
                                   const int32_t *__restrict__ emat, int64_t nel, int npe,
@@ -126,6 +127,7 @@ __global__ void k_affine_geometry(const double *__restrict__ xyz, const int32_t 
         for (int k = 0; k < 9; ++k) geo[e * 10 + k] = inv[k];
         geo[e * 10 + 9] = det;
         f = aligned ? 2 : 1;
+        if (nonaffine) nonaffine[1] = 1ull;
       } else if (nonaffine) {
         atomicAdd(nonaffine, 1ull);
       }

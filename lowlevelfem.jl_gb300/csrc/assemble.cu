@@ -5,10 +5,14 @@
 //                 device mesh): which elements are affine images of the
 //                 reference element (and which of those are axis-aligned
 //                 bricks), with their J^-1 and det;
-//   k_elem_affine meshes whose elements are all affine: one CTA per element
-//                 at a time (persistent), the node-pair blocks formed from
-//                 the reference pair tables into a shared-memory image of the
-//                 element matrix, which one bulk store writes out;
+//   k_elem_packed small elements (up to 144 node pairs): several per CTA,
+//                 after k_affine_coeff has formed the affine ones'
+//                 coefficients;
+//   k_elem_affine larger elements of meshes whose elements are all affine:
+//                 one CTA per element at a time (persistent), the node-pair
+//                 blocks formed from the reference pair tables into a
+//                 shared-memory image of the element matrix, which one bulk
+//                 store writes out;
 //   k_elem_fp64   other meshes: one CTA per element at a time, element node
 //                 coordinates gathered into shared memory, the reference
 //                 shape gradients staged in shared memory for the CTA's
@@ -16,7 +20,7 @@
 //                 do not fit), Jacobian / inverse / physical gradients per
 //                 integration point (the affine form for affine elements),
 //                 then the upper-triangle node-pair blocks, each written
-//                 twice (block and mirror).  Both kernels leave the element
+//                 twice (block and mirror).  All three leave the element
 //                 matrix whole in the layout Kf[element][column node b][row
 //                 node a][block];
 //   k_colgather   (gather.cu) sums every entry over its elements in element
@@ -60,7 +64,7 @@ struct ElemArgs {
   const uint8_t *aflag;
   const double *ageo, *Rp, *Mp;
   int cta_cap;               // host side: CTAs per SM at most (0: as many as fit)
-  bool all_affine;           // host side: k_affine_geometry counted no non-affine element
+  bool all_affine, any_affine;  // host side: k_affine_geometry counted no non-affine element, met an affine one
 };
 
 __device__ __forceinline__ int pair_offset(int a, int npe) {
@@ -529,6 +533,300 @@ k_elem_affine(ElemArgs A, int tab_n) {
   if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
+// Several small elements per CTA (E of them: elements e0 .. e0+E-1 at a
+// time, persistent), one node pair per thread, for elements of at most
+// PACK_PAIRS node pairs, affine or not.  The FP64 pipe is spent per warp
+// instruction, and a CTA per element filled it badly: 36 of 64 lanes for
+// hex8's pairs (10 of 128 for tet4 and quad4), and about 28 instructions of
+// one warp for the coefficients of an affine element, where its pairs take 6
+// (hex8 conduction) to 102 (tet10 elasticity).  Here the coefficients come
+// from k_affine_coeff, a thread per element (6 warp instructions each), the
+// pairs of the E elements fill their warps, and a thread keeps its pair's
+// table row in registers.  The E element matrices are formed in a
+// shared-memory image of their Kf run and leave with one bulk store.
+// Elements that are not affine go through the points as in k_elem_fp64, all
+// E at once.  The arithmetic is k_elem_fp64's.
+// tet10 elasticity, 178,002 turned elements: 1.33 -> 0.92 ms and 0.09 ms of
+// coefficients (9.8 M pairs of 51 FP64 operations take 0.82 ms); hex8
+// conduction, 249,856 elements: 0.283 -> 0.088 + 0.020 ms.
+// Shared memory (doubles): image [E kelems] | coefficients [E AFF_PACK] |
+// flags [E ints] | QUAD: X [E npe DIM] | det w [E nip] | J^-1 [E nip 9] |
+// G, S [E nip npe gsw each].
+constexpr int PACK_PAIRS = 144, PACK_THREADS = 288;
+constexpr int AFF_PACK = 46;   // doubles per element: W 36, U 9 (or the other forms' coefficients)
+
+// Coefficients of the affine elements, one thread each, by the operations of
+// affine_coefficients / affine_stage_aligned: elasticity W [36] then U [9]
+// (2D: 9 and 1), axis-aligned elasticity alpha, beta, a, b; conduction c1 trV
+// [NS]; mass c1 det.
+template <int KIND, int DIM>
+__global__ void __launch_bounds__(128)
+k_affine_coeff(const double *__restrict__ ageo, const uint8_t *__restrict__ aflag, const int32_t *__restrict__ emat,
+               const double *__restrict__ mc1, const double *__restrict__ mc2, int64_t nel, double *__restrict__ coef,
+               unsigned *status) {
+  constexpr int NS = DIM == 3 ? 6 : 3, NA = DIM == 3 ? 3 : 1;
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nel; e += (int64_t)gridDim.x * blockDim.x) {
+    const int mat = emat ? emat[e] : 0, flag = aflag[e];
+    if (mat < 0 || !flag) continue;
+    const double *inv = ageo + (size_t)e * 10;
+    const double c1 = mc1[mat], c2 = KIND == KIND_ELASTIC ? mc2[mat] : 0.0, det = inv[9];
+    double *out = coef + (size_t)e * AFF_PACK;
+    if (!(det > 0.0)) atomicOr(status, ST_BAD_JACOBIAN);
+    const double cp = __dadd_rn(c1, c2), cm = __dsub_rn(c1, c2);
+    if (KIND == KIND_MASS) {
+      out[0] = __dmul_rn(c1, det);
+    } else if (flag == 2) {
+#pragma unroll
+      for (int n = 0; n < (KIND == KIND_ELASTIC ? NS : DIM); ++n) {
+        const int k = sym_k<DIM>(n), l = sym_l<DIM>(n);
+        const double V = __dmul_rn(det, __dmul_rn(inv[k * 3 + k], inv[l * 3 + l]));
+        if (KIND == KIND_HEAT) {
+          out[n] = __dmul_rn(c1, V);
+        } else if (n < DIM) {
+          out[n] = __dmul_rn(cp, V);
+          out[DIM + n] = __dmul_rn(c2, V);
+        } else {
+          out[DIM + n] = __dmul_rn(cp, V);
+          out[DIM + NA + n] = __dmul_rn(cm, V);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int n = 0; n < NS; ++n) {
+        const int k = sym_k<DIM>(n), l = sym_l<DIM>(n);
+        double V[NS];
+#pragma unroll
+        for (int m = 0; m < NS; ++m) {
+          const int i = sym_k<DIM>(m), j = sym_l<DIM>(m);
+          V[m] = k == l ? __dmul_rn(det, __dmul_rn(inv[k * 3 + i], inv[k * 3 + j]))
+                        : __dmul_rn(det, __fma_rn(inv[k * 3 + i], inv[l * 3 + j],
+                                                  __dmul_rn(inv[l * 3 + i], inv[k * 3 + j])));
+        }
+        double tr = __dadd_rn(V[0], V[1]);
+        if (DIM == 3) tr = __dadd_rn(tr, V[2]);
+        if (KIND == KIND_HEAT) {
+          out[n] = __dmul_rn(c1, tr);
+        } else {
+#pragma unroll
+          for (int m = 0; m < NS; ++m) {
+            const double v = __dmul_rn(cp, V[m]);
+            out[m * NS + n] = m < DIM ? __fma_rn(c2, tr, v) : v;
+          }
+        }
+      }
+      if (KIND == KIND_ELASTIC) {
+#pragma unroll
+        for (int t = 0; t < NA * NA; ++t) {
+          const int m = t / NA, n = t - m * NA;
+          const int i = sym_k<DIM>(DIM + m), j = sym_l<DIM>(DIM + m);
+          const int k = sym_k<DIM>(DIM + n), l = sym_l<DIM>(DIM + n);
+          out[NS * NS + t] = __dmul_rn(cm, __dmul_rn(det, __fma_rn(inv[k * 3 + i], inv[l * 3 + j],
+                                                                  -__dmul_rn(inv[l * 3 + i], inv[k * 3 + j]))));
+        }
+      }
+    }
+  }
+}
+
+template <int KIND, int DIM, bool QUAD>
+__global__ void __launch_bounds__(PACK_THREADS, QUAD ? 2 : 3)
+k_elem_packed(ElemArgs A, const double *__restrict__ coef, int E) {
+  extern __shared__ __align__(128) double smem_p[];
+  constexpr int NS = DIM == 3 ? 6 : 3, NA = DIM == 3 ? 3 : 1;
+  constexpr int BS = (KIND == KIND_ELASTIC) ? DIM * DIM : 1;
+  constexpr int P = (KIND == KIND_ELASTIC) ? DIM : 1;
+  constexpr int gsw = (KIND == KIND_MASS) ? 1 : DIM;
+  constexpr int NC = KIND == KIND_MASS ? 1 : (KIND == KIND_HEAT ? NS : NS * NS + NA * NA);  // coefficients used
+  const int npe = A.npe, nip = A.nip;
+  const int64_t kelems = (int64_t)npe * A.colstride;
+  double *sKe = smem_p, *sCo = sKe + E * kelems;
+  int *sFlag = reinterpret_cast<int *>(sCo + (size_t)E * AFF_PACK);   // -1 masked, 0 points, 1 affine, 2 aligned
+  double *sX = sCo + (size_t)E * AFF_PACK + (E + 1) / 2;
+  double *sWd = sX + (size_t)E * npe * DIM, *sInv = sWd + (size_t)E * nip;
+  double *G = sInv + (size_t)E * nip * 9, *S = G + (size_t)E * nip * npe * gsw;
+  // this thread's node pair and its table row
+  const int el = threadIdx.x / A.npairs, pi = threadIdx.x - el * A.npairs;
+  int a = 0, b = 0;
+  double sv[NS], av[NA];
+  if (el < E) {
+    pair_decode(pi, npe, a, b);
+    if (A.aflag) {
+      if (KIND == KIND_MASS) {
+        sv[0] = A.Mp[pi];
+      } else {
+#pragma unroll
+        for (int n = 0; n < NS; ++n) sv[n] = A.Rp[(size_t)pi * 9 + n];
+#pragma unroll
+        for (int n = 0; n < NA; ++n) av[n] = A.Rp[(size_t)pi * 9 + 6 + n];
+      }
+    }
+  }
+  for (int64_t e0 = (int64_t)blockIdx.x * E; e0 < A.nel; e0 += (int64_t)gridDim.x * E) {
+    const int ne = (int)(A.nel - e0 < E ? A.nel - e0 : E);
+    if ((int)threadIdx.x < ne) {
+      const int64_t e = e0 + threadIdx.x;
+      sFlag[threadIdx.x] = A.emat && A.emat[e] < 0 ? -1 : (A.aflag ? (int)A.aflag[e] : 0);
+    }
+    for (int t = threadIdx.x; coef && t < ne * NC; t += blockDim.x) {
+      const int k = t / NC, n = t - k * NC;
+      sCo[k * AFF_PACK + n] = coef[(size_t)(e0 + k) * AFF_PACK + n];
+    }
+    if (QUAD)
+      for (int t = threadIdx.x; t < ne * npe * DIM; t += blockDim.x)
+        sX[t] = A.xyz[(size_t)A.conn[e0 * npe + t / DIM] * 3 + t % DIM];
+    // the previous elements' store has read the image
+    if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    __syncthreads();
+    if (QUAD) {
+      for (int t = threadIdx.x; t < ne * nip; t += blockDim.x) {
+        const int k = t / nip, q = t - k * nip;
+        if (sFlag[k] != 0) continue;
+        double inv[9];
+        const double *dq = A.dN + (size_t)q * npe * 3;
+        const double det = geom_point<DIM>(sX + (size_t)k * npe * DIM, [&](int n, int j) { return __ldg(dq + n * 3 + j); },
+                                           npe, inv);
+        if (!(det > 0.0)) atomicOr(A.status, ST_BAD_JACOBIAN);
+        sWd[t] = __dmul_rn(det, __ldg(A.w + q));
+#pragma unroll
+        for (int n = 0; n < 9; ++n) sInv[(size_t)t * 9 + n] = inv[n];
+      }
+      __syncthreads();
+      for (int t = threadIdx.x; t < ne * nip * npe; t += blockDim.x) {
+        const int p = t / npe, k = p / nip, q = p - k * nip, n = t - p * npe;   // point, element, node
+        if (sFlag[k] != 0) continue;
+        const double wd = sWd[p];
+        if (KIND == KIND_MASS) {
+          S[t] = __dmul_rn(wd, __ldg(A.N + (size_t)q * npe + n));
+        } else {
+          const double *inv = sInv + (size_t)p * 9, *d = A.dN + ((size_t)q * npe + n) * 3;
+#pragma unroll
+          for (int i = 0; i < DIM; ++i) {
+            double acc = 0.0;
+#pragma unroll
+            for (int j = 0; j < DIM; ++j) acc = __fma_rn(inv[3 * j + i], __ldg(d + j), acc);
+            G[(size_t)t * DIM + i] = acc;
+            S[(size_t)t * DIM + i] = __dmul_rn(wd, acc);
+          }
+        }
+      }
+      __syncthreads();
+    }
+    const int flag = el < ne ? sFlag[el] : -1;
+    if (flag >= 0) {
+      const double *C = sCo + (size_t)el * AFF_PACK;
+      double blk[BS];
+      if (QUAD && flag == 0) {
+        const size_t p0 = (size_t)el * nip * npe;
+        if (KIND == KIND_ELASTIC) {
+          const int64_t e = e0 + el;
+          const int mat = A.emat ? A.emat[e] : 0;
+          const double c1 = A.c1[mat], c2 = A.c2[mat];
+          double O[DIM][DIM];
+#pragma unroll
+          for (int i = 0; i < DIM; ++i)
+#pragma unroll
+            for (int j = 0; j < DIM; ++j) O[i][j] = 0.0;
+          for (int q = 0; q < nip; ++q) {
+            const double *sa = S + (p0 + (size_t)q * npe + a) * DIM, *gb = G + (p0 + (size_t)q * npe + b) * DIM;
+            double s_[DIM], g_[DIM];
+#pragma unroll
+            for (int i = 0; i < DIM; ++i) { s_[i] = sa[i]; g_[i] = gb[i]; }
+#pragma unroll
+            for (int i = 0; i < DIM; ++i)
+#pragma unroll
+              for (int j = 0; j < DIM; ++j) O[i][j] = __fma_rn(s_[i], g_[j], O[i][j]);
+          }
+          if (a == b) {   // the upper triangle, mirrored
+#pragma unroll
+            for (int i = 0; i < DIM; ++i)
+#pragma unroll
+              for (int j = 0; j < i; ++j) O[i][j] = O[j][i];
+          }
+          double tr = __dadd_rn(O[0][0], O[1 % DIM][1 % DIM]);
+          if (DIM == 3) tr = __dadd_rn(tr, O[2 % DIM][2 % DIM]);
+#pragma unroll
+          for (int i = 0; i < DIM; ++i)
+#pragma unroll
+            for (int j = 0; j < DIM; ++j) {
+              double t = __fma_rn(c2, O[j][i], __dmul_rn(c1, O[i][j]));
+              if (i == j) t = __fma_rn(c2, tr, t);
+              blk[i * DIM + j] = t;
+            }
+        } else {
+          const double c1 = A.c1[A.emat ? A.emat[e0 + el] : 0];
+          double acc = 0.0;
+          for (int q = 0; q < nip; ++q) {
+            if (KIND == KIND_HEAT) {
+              const double *sa = S + (p0 + (size_t)q * npe + a) * DIM, *gb = G + (p0 + (size_t)q * npe + b) * DIM;
+#pragma unroll
+              for (int i = 0; i < DIM; ++i) acc = __fma_rn(sa[i], gb[i], acc);
+            } else {
+              acc = __fma_rn(S[p0 + (size_t)q * npe + a], __ldg(A.N + (size_t)q * npe + b), acc);
+            }
+          }
+          blk[0] = __dmul_rn(c1, acc);
+        }
+      } else if (KIND == KIND_MASS) {
+        blk[0] = __dmul_rn(C[0], sv[0]);
+      } else if (KIND == KIND_HEAT) {
+        double acc = 0.0;
+#pragma unroll
+        for (int n = 0; n < NS; ++n)
+          if (n < DIM || flag == 1) acc = __fma_rn(C[n], sv[n], acc);
+        blk[0] = acc;
+      } else if (flag == 2) {
+        double g = __dmul_rn(C[DIM], sv[0]);
+#pragma unroll
+        for (int n = 1; n < DIM; ++n) g = __fma_rn(C[DIM + n], sv[n], g);
+#pragma unroll
+        for (int i = 0; i < DIM; ++i) blk[i * DIM + i] = __fma_rn(C[i], sv[i], g);
+#pragma unroll
+        for (int m = 0; m < NA; ++m) {
+          const int i = sym_k<DIM>(DIM + m), j = sym_l<DIM>(DIM + m);
+          const double am = C[2 * DIM + m], s = sv[DIM + m];
+          if (a != b) {
+            const double h = __dmul_rn(C[2 * DIM + NA + m], av[m]);
+            blk[i * DIM + j] = __fma_rn(am, s, h);
+            blk[j * DIM + i] = __fma_rn(am, s, -h);
+          } else {
+            blk[i * DIM + j] = blk[j * DIM + i] = __dmul_rn(am, s);
+          }
+        }
+      } else {
+        double ks[NS];
+#pragma unroll
+        for (int m = 0; m < NS; ++m) {
+          double acc = 0.0;
+#pragma unroll
+          for (int n = 0; n < NS; ++n) acc = __fma_rn(C[m * NS + n], sv[n], acc);
+          ks[m] = acc;
+        }
+#pragma unroll
+        for (int i = 0; i < DIM; ++i) blk[i * DIM + i] = ks[i];
+#pragma unroll
+        for (int m = 0; m < NA; ++m) {
+          const int i = sym_k<DIM>(DIM + m), j = sym_l<DIM>(DIM + m);
+          double acc = 0.0;
+#pragma unroll
+          for (int n = 0; n < NA; ++n) acc = __fma_rn(C[NS * NS + m * NA + n], av[n], acc);
+          blk[i * DIM + j] = a != b ? __dadd_rn(ks[DIM + m], acc) : ks[DIM + m];
+          blk[j * DIM + i] = a != b ? __dsub_rn(ks[DIM + m], acc) : ks[DIM + m];
+        }
+      }
+      store_pair<P, BS>(sKe + (size_t)el * kelems, A.colstride, a, b, blk);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                   ::"l"(A.Kf + (size_t)e0 * kelems), "r"(sh_addr(sKe)), "r"((unsigned)(ne * kelems * 8))
+                   : "memory");
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+  }
+  if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+
 // Non-zero test on the bit pattern (integer pipe): every value but +-0.
 __device__ __forceinline__ int nonzero_bits(double v) {
   return ((unsigned long long)__double_as_longlong(v) << 1) != 0ull;
@@ -678,15 +976,15 @@ int launch_elem(llf_ctx *ctx, const ElemArgs &a, size_t smem, unsigned grid) {
   return LLF_OK;
 }
 
-// The staged affine kernel when every element is affine, the element has
-// enough node pairs to fill a CTA and two CTAs fit on an SM; *done = false
+// The staged affine kernel when every element is affine and two CTAs fit on
+// an SM; *done = false
 // otherwise.  Threads: the node pairs in as few rounds of at most 256 as
 // possible, rounded up to whole warps (hex27: 378 pairs, 2 rounds of 192).
 template <int KIND, int DIM>
 int run_elem_affine(llf_ctx *ctx, const ElemArgs &a, bool *done) {
   *done = false;
   const int npairs = a.npairs;
-  if (!a.all_affine || !a.aflag || npairs < 32) return LLF_OK;
+  if (!a.all_affine || !a.aflag) return LLF_OK;
   const int tab_n = KIND == KIND_MASS ? npairs : npairs * 9;
   const size_t smem = sizeof(double) * ((size_t)a.npe * a.colstride + ((tab_n + 1) & ~1) + AFF_DOUBLES) + 16;
   if (smem > 110 * 1024) return LLF_OK;
@@ -708,11 +1006,72 @@ int run_elem_affine(llf_ctx *ctx, const ElemArgs &a, bool *done) {
   return LLF_OK;
 }
 
+// Elements per CTA of k_elem_packed: as many as fill their warps best with
+// node pairs, the larger count of equals, within PACK_THREADS threads and
+// 72 KB of shared memory (three CTAs per SM); 0: one does not fit.
+int packed_count(int npairs, size_t per_elem) {
+  int best = 0;
+  double fill = 0.0;
+  for (int E = 1; E * npairs <= PACK_THREADS && E * per_elem <= 72 * 1024; ++E) {
+    const double f = (double)(E * npairs) / ((E * npairs + 31) / 32 * 32);
+    if (f >= fill) {
+      fill = f;
+      best = E;
+    }
+  }
+  return best;
+}
+
+// k_elem_packed for elements of at most PACK_PAIRS node pairs (two or more
+// fit a CTA); *done = false otherwise.  A mesh that would leave SMs idle puts
+// fewer elements in a CTA.
+template <int KIND, int DIM>
+int run_elem_packed(llf_ctx *ctx, const ElemArgs &a, bool *done) {
+  *done = false;
+  if (a.npairs > PACK_PAIRS) return LLF_OK;
+  const bool quad = !a.all_affine || !a.aflag;
+  const int gsw = (KIND == KIND_MASS) ? 1 : DIM;
+  const size_t per_elem = sizeof(double) * ((size_t)a.npe * a.colstride + AFF_PACK + 1 +
+                                            (quad ? (size_t)a.npe * DIM + (size_t)a.nip * 10 +
+                                                        2 * (size_t)a.nip * a.npe * gsw : 0));
+  int E = packed_count(a.npairs, per_elem);
+  if (E < 1) return LLF_OK;
+  E = (int)std::min<int64_t>(E, (a.nel + ctx->num_sms - 1) / ctx->num_sms);
+  double *coef = nullptr;
+  if (a.aflag && a.any_affine) {
+    LLF_CUDA_TRY(ctx, dalloc(ctx, &coef, (size_t)a.nel * AFF_PACK));
+    KernelScope ks(ctx, "k_affine_coeff");
+    k_affine_coeff<KIND, DIM><<<grid_1d(a.nel, 128, ctx->num_sms), 128, 0, ctx->stream>>>(
+        a.ageo, a.aflag, a.emat, a.c1, a.c2, a.nel, coef, a.status);
+    LLF_CUDA_TRY(ctx, cudaGetLastError());
+  }
+  const size_t smem = E * per_elem;
+  const int threads = (E * a.npairs + 31) / 32 * 32;
+  auto launch = [&](auto fn) -> int {
+    if (smem > 48 * 1024)
+      LLF_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 1;
+    LLF_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
+    if (per_sm < 1) per_sm = 1;
+    if (a.cta_cap > 0 && per_sm > a.cta_cap) per_sm = a.cta_cap;
+    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->num_sms * per_sm, (a.nel + E - 1) / E));
+    KernelScope ks(ctx, "k_elem_packed");
+    fn<<<(unsigned)grid, threads, smem, ctx->stream>>>(a, coef, E);
+    LLF_CUDA_TRY(ctx, cudaGetLastError());
+    return LLF_OK;
+  };
+  const int rc = quad ? launch(k_elem_packed<KIND, DIM, true>) : launch(k_elem_packed<KIND, DIM, false>);
+  dfree(ctx, coef);
+  *done = rc == LLF_OK;
+  return rc;
+}
+
 template <int KIND, int DIM>
 int run_elem(llf_ctx *ctx, ElemArgs a) {
   {
     bool done = false;
-    const int rc = run_elem_affine<KIND, DIM>(ctx, a, &done);
+    int rc = run_elem_packed<KIND, DIM>(ctx, a, &done);
+    if (rc == LLF_OK && !done) rc = run_elem_affine<KIND, DIM>(ctx, a, &done);
     if (rc != LLF_OK || done) return rc;
   }
   const int npe = a.npe, nip = a.nip;
@@ -984,9 +1343,9 @@ int assemble_impl(llf_ctx *ctx, llf_mesh *mesh, llf_pattern *pat, int kind, int 
         LLF_CUDA_TRY(ctx, dalloc(ctx, &mesh->d_aflag, mesh->nel));
         LLF_CUDA_TRY(ctx, dalloc(ctx, &mesh->d_ageo, (size_t)mesh->nel * 10));
       }
-      unsigned long long *nonaff = nullptr;   // elements in use that are not affine
-      LLF_CUDA_TRY(ctx, dalloc(ctx, &nonaff, 1));
-      LLF_CUDA_TRY(ctx, cudaMemsetAsync(nonaff, 0, sizeof(unsigned long long), s));
+      unsigned long long *nonaff = nullptr;   // elements in use that are not affine; whether one is
+      LLF_CUDA_TRY(ctx, dalloc(ctx, &nonaff, 2));
+      LLF_CUDA_TRY(ctx, cudaMemsetAsync(nonaff, 0, 2 * sizeof(unsigned long long), s));
       {
         KernelScope ks(ctx, "k_affine_geometry");
         const unsigned g = grid_1d(mesh->nel, 128, ctx->num_sms);
@@ -998,11 +1357,12 @@ int assemble_impl(llf_ctx *ctx, llf_mesh *mesh, llf_pattern *pat, int kind, int 
                                                  mesh->d_dN, mesh->d_nref, mesh->d_ageo, mesh->d_aflag, nonaff);
         LLF_CUDA_TRY(ctx, cudaGetLastError());
       }
-      unsigned long long h = 1;
-      LLF_CUDA_TRY(ctx, cudaMemcpyAsync(&h, nonaff, sizeof(h), cudaMemcpyDeviceToHost, s));
+      unsigned long long h[2] = {1, 1};
+      LLF_CUDA_TRY(ctx, cudaMemcpyAsync(h, nonaff, sizeof(h), cudaMemcpyDeviceToHost, s));
       LLF_CUDA_TRY(ctx, cudaStreamSynchronize(s));
       dfree(ctx, nonaff);
-      mesh->geo_all_affine = h == 0;
+      mesh->geo_all_affine = h[0] == 0;
+      mesh->geo_any_affine = h[1] != 0;
       mesh->geo_cached = mesh->geo_version;
       mesh->geo_cached_tables = mesh->tables_version;
     }
@@ -1039,6 +1399,7 @@ int assemble_impl(llf_ctx *ctx, llf_mesh *mesh, llf_pattern *pat, int kind, int 
     a.Mp = mesh->d_Mp;
     a.cta_cap = pat->tune.elem_cap;
     a.all_affine = all_affine;
+    a.any_affine = aflag && mesh->geo_any_affine;
     // element range [e0, e1): the element-indexed arrays are offset
     auto elems = [&](int64_t e0, int64_t e1) -> int {
       ElemArgs b = a;

@@ -99,10 +99,11 @@ struct llf_mesh {
   // affine geometry of the elements (assemble.cu), kept for the geometry
   // version and tables it was computed from: per element the flag and
   // J^-1, det (k_affine_geometry), and whether every element in use is affine
+  // and whether any is
   uint8_t *d_aflag = nullptr;
   double *d_ageo = nullptr;
   int geo_cached = -1, geo_cached_tables = -1;
-  bool geo_all_affine = false;
+  bool geo_all_affine = false, geo_any_affine = false;
   // affine-element tables (built-in rules, whose node coordinates are known;
   // null after llf_tables_upload): reference node coordinates [npe*3] and,
   // per upper-triangle node pair (a <= b, a-major), R_ab [9] and Mref_ab
