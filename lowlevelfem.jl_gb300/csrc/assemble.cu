@@ -5,9 +5,9 @@
 //                 device mesh): which elements are affine images of the
 //                 reference element (and which of those are axis-aligned
 //                 bricks), with their J^-1 and det;
-//   k_elem_packed small elements (up to 144 node pairs): several per CTA,
-//                 after k_affine_coeff has formed the affine ones'
-//                 coefficients;
+//   k_elem_packed elements of up to 384 node pairs: as many per CTA as fill
+//                 its threads (one hex27, ten hex8), after k_affine_coeff
+//                 has formed the affine ones' coefficients;
 //   k_elem_affine larger elements of meshes whose elements are all affine:
 //                 one CTA per element at a time (persistent), the node-pair
 //                 blocks formed from the reference pair tables into a
@@ -533,27 +533,38 @@ k_elem_affine(ElemArgs A, int tab_n) {
   if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
-// Several small elements per CTA (E of them: elements e0 .. e0+E-1 at a
-// time, persistent), one node pair per thread, for elements of at most
-// PACK_PAIRS node pairs, affine or not.  The FP64 pipe is spent per warp
-// instruction, and a CTA per element filled it badly: 36 of 64 lanes for
-// hex8's pairs (10 of 128 for tet4 and quad4), and about 28 instructions of
-// one warp for the coefficients of an affine element, where its pairs take 6
-// (hex8 conduction) to 102 (tet10 elasticity).  Here the coefficients come
-// from k_affine_coeff, a thread per element (6 warp instructions each), the
-// pairs of the E elements fill their warps, and a thread keeps its pair's
-// table row in registers.  The E element matrices are formed in a
-// shared-memory image of their Kf run and leave with one bulk store.
-// Elements that are not affine go through the points as in k_elem_fp64, all
-// E at once.  The arithmetic is k_elem_fp64's.
-// tet10 elasticity, 178,002 turned elements: 1.33 -> 0.92 ms and 0.09 ms of
-// coefficients (9.8 M pairs of 51 FP64 operations take 0.82 ms); hex8
-// conduction, 249,856 elements: 0.283 -> 0.088 + 0.020 ms.
-// Shared memory (doubles): image [E kelems] | coefficients [E AFF_PACK] |
-// flags [E ints] | QUAD: X [E npe DIM] | det w [E nip] | J^-1 [E nip 9] |
-// G, S [E nip npe gsw each].
-constexpr int PACK_PAIRS = 144, PACK_THREADS = 288;
-constexpr int AFF_PACK = 46;   // doubles per element: W 36, U 9 (or the other forms' coefficients)
+// One or more elements per CTA (E of them: elements e0 .. e0+E-1 at a time,
+// persistent), one node pair per thread, for elements of at most PACK_PAIRS
+// node pairs, affine or not.  The FP64 pipe bounds it and is spent per warp
+// instruction, and a 128-thread CTA per element filled it badly: 36 of 64
+// lanes for hex8's pairs (10 of 128 for tet4 and quad4), about 28
+// instructions of one warp for the coefficients of an affine element, where
+// its pairs take 6 (hex8 conduction) to 102 (tet10 elasticity), and by points
+// 27 lanes of one warp with 240 dependent operations each for a hex27's
+// Jacobians.  Here the coefficients come from k_affine_coeff, a thread per
+// element (6 warp instructions each), the pairs of the E elements fill their
+// warps, and a thread keeps its pair's table row in registers.  The E element
+// matrices are formed in a shared-memory image of their Kf run and leave with
+// one bulk store.  The next E elements' coefficients and coordinates are
+// copied in meanwhile (cp.async, two buffers).  Elements that are not affine
+// go through the points as in k_elem_fp64, all E at once, each entry of a
+// Jacobian in its own thread.  The arithmetic is k_elem_fp64's.
+// Measured, element kernel alone:
+//   tet10 elasticity, 178,002 turned: 1.33 -> 0.90 + 0.09 ms of coefficients
+//   (9.8 M pairs of 51 FP64 operations take 0.82 ms);
+//   hex27 elasticity, 64,000 boxes: 1.06 (k_elem_affine) -> 0.94 + 0.01 ms;
+//   hex27 elasticity, 4,522 curved: 1.41 (k_elem_fp64) -> 0.93 ms (operations
+//   0.80 ms); tet20, 10,368 curved: 4.41 -> 2.86 ms;
+//   hex8 conduction, 249,856 boxes: 0.283 -> 0.079 + 0.013 ms; hex27
+//   conduction, 64,000: 0.212 -> 0.202 + 0.009 ms boxes, 0.382 -> 0.275 +
+//   0.017 ms turned (without the two buffers 0.224 and 0.29).
+// Shared memory (doubles): image [E kelems] | coefficients [2][E NC] |
+// flags [2][E ints] | QUAD: X [2][E npe DIM] | det w [E nip] |
+// J^-1 [E nip 9] | G, S [E nip npe gsw each].
+constexpr int PACK_PAIRS = 384, PACK_THREADS = 384;
+// coefficients of an affine element
+template <int KIND, int DIM>
+constexpr int AFF_PACK = KIND == KIND_MASS ? 1 : (KIND == KIND_HEAT ? (DIM == 3 ? 6 : 3) : (DIM == 3 ? 45 : 10));
 
 // Coefficients of the affine elements, one thread each, by the operations of
 // affine_coefficients / affine_stage_aligned: elasticity W [36] then U [9]
@@ -570,7 +581,7 @@ k_affine_coeff(const double *__restrict__ ageo, const uint8_t *__restrict__ afla
     if (mat < 0 || !flag) continue;
     const double *inv = ageo + (size_t)e * 10;
     const double c1 = mc1[mat], c2 = KIND == KIND_ELASTIC ? mc2[mat] : 0.0, det = inv[9];
-    double *out = coef + (size_t)e * AFF_PACK;
+    double *out = coef + (size_t)e * AFF_PACK<KIND, DIM>;
     if (!(det > 0.0)) atomicOr(status, ST_BAD_JACOBIAN);
     const double cp = __dadd_rn(c1, c2), cm = __dsub_rn(c1, c2);
     if (KIND == KIND_MASS) {
@@ -628,21 +639,26 @@ k_affine_coeff(const double *__restrict__ ageo, const uint8_t *__restrict__ afla
   }
 }
 
+// 8-byte copy to shared memory, under way until the next cp.async wait
+__device__ __forceinline__ void copy_async8(double *dst, const double *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sh_addr(dst)), "l"(src) : "memory");
+}
+
 template <int KIND, int DIM, bool QUAD>
-__global__ void __launch_bounds__(PACK_THREADS, QUAD ? 2 : 3)
+__global__ void __launch_bounds__(PACK_THREADS, 2)
 k_elem_packed(ElemArgs A, const double *__restrict__ coef, int E) {
   extern __shared__ __align__(128) double smem_p[];
   constexpr int NS = DIM == 3 ? 6 : 3, NA = DIM == 3 ? 3 : 1;
   constexpr int BS = (KIND == KIND_ELASTIC) ? DIM * DIM : 1;
   constexpr int P = (KIND == KIND_ELASTIC) ? DIM : 1;
   constexpr int gsw = (KIND == KIND_MASS) ? 1 : DIM;
-  constexpr int NC = KIND == KIND_MASS ? 1 : (KIND == KIND_HEAT ? NS : NS * NS + NA * NA);  // coefficients used
+  constexpr int NC = AFF_PACK<KIND, DIM>;
   const int npe = A.npe, nip = A.nip;
   const int64_t kelems = (int64_t)npe * A.colstride;
-  double *sKe = smem_p, *sCo = sKe + E * kelems;
-  int *sFlag = reinterpret_cast<int *>(sCo + (size_t)E * AFF_PACK);   // -1 masked, 0 points, 1 affine, 2 aligned
-  double *sX = sCo + (size_t)E * AFF_PACK + (E + 1) / 2;
-  double *sWd = sX + (size_t)E * npe * DIM, *sInv = sWd + (size_t)E * nip;
+  double *sKe = smem_p, *sCo2 = sKe + E * kelems;
+  int *sFlag2 = reinterpret_cast<int *>(sCo2 + 2 * (size_t)E * NC);   // -1 masked, 0 points, 1 affine, 2 aligned
+  double *sX2 = sCo2 + 2 * (size_t)E * NC + E;
+  double *sWd = sX2 + (QUAD ? 2 * (size_t)E * npe * DIM : 0), *sInv = sWd + (size_t)E * nip;
   double *G = sInv + (size_t)E * nip * 9, *S = G + (size_t)E * nip * npe * gsw;
   // this thread's node pair and its table row
   const int el = threadIdx.x / A.npairs, pi = threadIdx.x - el * A.npairs;
@@ -661,30 +677,55 @@ k_elem_packed(ElemArgs A, const double *__restrict__ coef, int E) {
       }
     }
   }
-  for (int64_t e0 = (int64_t)blockIdx.x * E; e0 < A.nel; e0 += (int64_t)gridDim.x * E) {
+  // coefficients and coordinates of the elements from e0 on, under way into
+  // buffer h while the elements before are computed
+  auto fetch = [&](int64_t e0, int h) {
     const int ne = (int)(A.nel - e0 < E ? A.nel - e0 : E);
     if ((int)threadIdx.x < ne) {
       const int64_t e = e0 + threadIdx.x;
-      sFlag[threadIdx.x] = A.emat && A.emat[e] < 0 ? -1 : (A.aflag ? (int)A.aflag[e] : 0);
+      sFlag2[h * E + threadIdx.x] = A.emat && A.emat[e] < 0 ? -1 : (A.aflag ? (int)A.aflag[e] : 0);
     }
-    for (int t = threadIdx.x; coef && t < ne * NC; t += blockDim.x) {
-      const int k = t / NC, n = t - k * NC;
-      sCo[k * AFF_PACK + n] = coef[(size_t)(e0 + k) * AFF_PACK + n];
-    }
+    for (int t = threadIdx.x; coef && t < ne * NC; t += blockDim.x)
+      copy_async8(sCo2 + (size_t)h * E * NC + t, coef + (size_t)e0 * NC + t);
     if (QUAD)
       for (int t = threadIdx.x; t < ne * npe * DIM; t += blockDim.x)
-        sX[t] = A.xyz[(size_t)A.conn[e0 * npe + t / DIM] * 3 + t % DIM];
+        copy_async8(sX2 + (size_t)h * E * npe * DIM + t, A.xyz + (size_t)A.conn[e0 * npe + t / DIM] * 3 + t % DIM);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int64_t step = (int64_t)gridDim.x * E;
+  int h = 0;
+  if ((int64_t)blockIdx.x * E < A.nel) fetch((int64_t)blockIdx.x * E, 0);
+  for (int64_t e0 = (int64_t)blockIdx.x * E; e0 < A.nel; e0 += step, h ^= 1) {
+    const int ne = (int)(A.nel - e0 < E ? A.nel - e0 : E);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     // the previous elements' store has read the image
     if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     __syncthreads();
+    if (e0 + step < A.nel) fetch(e0 + step, h ^ 1);
+    const int *sFlag = sFlag2 + h * E;
+    const double *sX = sX2 + (size_t)h * E * npe * DIM, *sCo = sCo2 + (size_t)h * E * NC;
     if (QUAD) {
+      // J of every point, one entry per thread (its fma chain over the nodes),
+      // then the inverse, one point per thread, in place
+      for (int t = threadIdx.x; t < ne * nip * DIM * DIM; t += blockDim.x) {
+        const int p = t / (DIM * DIM), ij = t - p * DIM * DIM, k = p / nip, q = p - k * nip;
+        if (sFlag[k] != 0) continue;
+        const int i = ij / DIM, j = ij - i * DIM;
+        const double *x = sX + (size_t)k * npe * DIM + i, *d = A.dN + (size_t)q * npe * 3 + j;
+        double acc = 0.0;
+        for (int n = 0; n < npe; ++n) acc = __fma_rn(x[n * DIM], __ldg(d + n * 3), acc);
+        sInv[(size_t)p * 9 + 3 * i + j] = acc;
+      }
+      __syncthreads();
       for (int t = threadIdx.x; t < ne * nip; t += blockDim.x) {
         const int k = t / nip, q = t - k * nip;
         if (sFlag[k] != 0) continue;
-        double inv[9];
-        const double *dq = A.dN + (size_t)q * npe * 3;
-        const double det = geom_point<DIM>(sX + (size_t)k * npe * DIM, [&](int n, int j) { return __ldg(dq + n * 3 + j); },
-                                           npe, inv);
+        double J[3][3], inv[9];
+#pragma unroll
+        for (int i = 0; i < DIM; ++i)
+#pragma unroll
+          for (int j = 0; j < DIM; ++j) J[i][j] = sInv[(size_t)t * 9 + 3 * i + j];
+        const double det = jac_inverse<DIM>(J, inv);
         if (!(det > 0.0)) atomicOr(A.status, ST_BAD_JACOBIAN);
         sWd[t] = __dmul_rn(det, __ldg(A.w + q));
 #pragma unroll
@@ -713,7 +754,7 @@ k_elem_packed(ElemArgs A, const double *__restrict__ coef, int E) {
     }
     const int flag = el < ne ? sFlag[el] : -1;
     if (flag >= 0) {
-      const double *C = sCo + (size_t)el * AFF_PACK;
+      const double *C = sCo + (size_t)el * NC;
       double blk[BS];
       if (QUAD && flag == 0) {
         const size_t p0 = (size_t)el * nip * npe;
@@ -1008,11 +1049,11 @@ int run_elem_affine(llf_ctx *ctx, const ElemArgs &a, bool *done) {
 
 // Elements per CTA of k_elem_packed: as many as fill their warps best with
 // node pairs, the larger count of equals, within PACK_THREADS threads and
-// 72 KB of shared memory (three CTAs per SM); 0: one does not fit.
+// 108 KB of shared memory (two CTAs per SM); 0: one does not fit.
 int packed_count(int npairs, size_t per_elem) {
   int best = 0;
   double fill = 0.0;
-  for (int E = 1; E * npairs <= PACK_THREADS && E * per_elem <= 72 * 1024; ++E) {
+  for (int E = 1; E * npairs <= PACK_THREADS && E * per_elem <= 108 * 1024; ++E) {
     const double f = (double)(E * npairs) / ((E * npairs + 31) / 32 * 32);
     if (f >= fill) {
       fill = f;
@@ -1022,24 +1063,27 @@ int packed_count(int npairs, size_t per_elem) {
   return best;
 }
 
-// k_elem_packed for elements of at most PACK_PAIRS node pairs (two or more
-// fit a CTA); *done = false otherwise.  A mesh that would leave SMs idle puts
+// k_elem_packed for elements of at most PACK_PAIRS node pairs; *done = false
+// otherwise (from hex64's 2080 pairs on a thread has many pairs either way).  A mesh that would leave SMs idle puts
 // fewer elements in a CTA.
 template <int KIND, int DIM>
 int run_elem_packed(llf_ctx *ctx, const ElemArgs &a, bool *done) {
   *done = false;
-  if (a.npairs > PACK_PAIRS) return LLF_OK;
   const bool quad = !a.all_affine || !a.aflag;
+  // The mass matrix by points has one operation per pair and point and little
+  // shared memory; from 144 pairs on, an element per small CTA is as good
+  // (27,000 curved hex27: 1.012 against 1.038 ms here).
+  if (a.npairs > (KIND == KIND_MASS && quad ? 144 : PACK_PAIRS)) return LLF_OK;
   const int gsw = (KIND == KIND_MASS) ? 1 : DIM;
-  const size_t per_elem = sizeof(double) * ((size_t)a.npe * a.colstride + AFF_PACK + 1 +
-                                            (quad ? (size_t)a.npe * DIM + (size_t)a.nip * 10 +
+  const size_t per_elem = sizeof(double) * ((size_t)a.npe * a.colstride + 2 * AFF_PACK<KIND, DIM> + 1 +
+                                            (quad ? 2 * (size_t)a.npe * DIM + (size_t)a.nip * 10 +
                                                         2 * (size_t)a.nip * a.npe * gsw : 0));
   int E = packed_count(a.npairs, per_elem);
   if (E < 1) return LLF_OK;
   E = (int)std::min<int64_t>(E, (a.nel + ctx->num_sms - 1) / ctx->num_sms);
   double *coef = nullptr;
   if (a.aflag && a.any_affine) {
-    LLF_CUDA_TRY(ctx, dalloc(ctx, &coef, (size_t)a.nel * AFF_PACK));
+    LLF_CUDA_TRY(ctx, dalloc(ctx, &coef, (size_t)a.nel * AFF_PACK<KIND, DIM>));
     KernelScope ks(ctx, "k_affine_coeff");
     k_affine_coeff<KIND, DIM><<<grid_1d(a.nel, 128, ctx->num_sms), 128, 0, ctx->stream>>>(
         a.ageo, a.aflag, a.emat, a.c1, a.c2, a.nel, coef, a.status);

@@ -57,7 +57,8 @@ def _cauchy_green(A, m):
 # elements on the GPU's SMs and leave the last one partly filled
 ASM_CASES = {"hex8": ((11, 10, 11), 1, False), "tet4": ((8, 7, 7), 1, True), "tet10": ((5, 4, 5), 2, True),
              "quad4": ((49, 47), 1, False), "tri3": ((61, 59), 1, True), "tri6": ((29, 29), 2, True),
-             "quad9": ((28, 28), 2, False)}
+             "quad9": ((28, 28), 2, False), "hex27": ((7, 7, 7), 2, False), "tet20": ((4, 4, 5), 3, True),
+             "quad25": ((18, 18), 4, False)}
 
 
 def _shaped(llf, cells, order, simplex, shape):
