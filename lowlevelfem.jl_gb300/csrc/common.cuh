@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <functional>
+#include <atomic>
 #include <string>
 #include <vector>
 
@@ -210,6 +211,9 @@ struct llf_matrix {
   // pair of words per 64 entries at keep_pos(s, c): entries 0..31 in word x,
   // 32..63 in word y.
   uint2 *d_keep = nullptr;
+  // a product has run: llf_pcg_noalloc takes the matrix, from the stored
+  // values where the structural ones are not expanded
+  mutable std::atomic<bool> multiplied{false};
 };
 
 // First keep word pair of column c, whose structural entries start at s, and

@@ -191,18 +191,71 @@ k_spmv(const double *__restrict__ nz, const int64_t *__restrict__ colptr,
   }
 }
 
+// Stored values, stored column starts (1-based) and keep bits of a matrix
+// whose assembly left the structural values out; vals null otherwise.
+struct KeptCols {
+  const double *vals;
+  const int64_t *colptr_s;
+  const uint2 *keep;
+};
+
+// node_columns_at from the stored values: entry i of a column is the stored
+// value at its rank among the column's kept entries, +0.0 when it is not
+// stored.  The lanes, the order of their sums and so the bits are the same.
+template <int P>
+__device__ __forceinline__ void node_columns_kept(const KeptCols &K, const int32_t *__restrict__ nadj,
+                                                  const double *__restrict__ x, int64_t B, int64_t r0, int64_t r1,
+                                                  bool valid, int g, double (&acc)[P]) {
+#pragma unroll
+  for (int j = 0; j < P; ++j) acc[j] = 0.0;
+  if (valid) {
+    const int n = (int)(r1 - r0) * P;
+    const double *v[P];
+    const unsigned *kw[P];   // a word per 32 entries
+    unsigned w[P];
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+      v[j] = K.vals + (K.colptr_s[P * B + j] - 1);
+      kw[j] = reinterpret_cast<const unsigned *>(K.keep + keep_pos((int64_t)P * P * r0 + (int64_t)j * n, P * B + j));
+      w[j] = n > 0 ? kw[j][0] : 0u;
+    }
+    for (int k0 = 0; k0 < n; k0 += 32) {
+      unsigned nx[P];   // the next words, a block of entries ahead
+#pragma unroll
+      for (int j = 0; j < P; ++j) nx[j] = k0 + 32 < n ? kw[j][(k0 >> 5) + 1] : 0u;
+      const int lim = n - k0 < 32 ? n - k0 : 32;
+#pragma unroll 2
+      for (int i = g; i < lim; i += SPMV_G) {
+        const int k = k0 + i;
+        const double xa = x[(int64_t)P * nadj[r0 + k / P] + k % P];
+        const unsigned below = (1u << i) - 1u;
+        double a[P];
+#pragma unroll
+        for (int j = 0; j < P; ++j) a[j] = (w[j] >> i) & 1u ? v[j][__popc(w[j] & below)] : 0.0;
+#pragma unroll
+        for (int j = 0; j < P; ++j) acc[j] = __fma_rn(a[j], xa, acc[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < P; ++j) {
+        v[j] += __popc(w[j]);
+        w[j] = nx[j];
+      }
+    }
+  }
+#pragma unroll
+  for (int off = SPMV_G / 2; off > 0; off >>= 1)
+#pragma unroll
+    for (int j = 0; j < P; ++j) acc[j] = __dadd_rn(acc[j], __shfl_xor_sync(0xffffffffu, acc[j], off));
+}
+
 // The same product from the stored values and their keep bits, for a matrix
-// whose assembly left the structural values out: entry i of a column is the
-// stored value at its rank among the column's kept entries, +0.0 when it is
-// not stored.  The lanes, the order of their sums and so the result's bits
-// are k_spmv's.  A warp's POPCs and selects (about 40 issue slots per step)
-// fit beside its P FP64 instructions, which take 64 each of an SM quarter.
-// hex27 40^3 (297.7 M entries): 0.87 ms; expanding the structural values
-// first and k_spmv took 2.55 + 0.83 ms.
+// whose assembly left the structural values out.  A warp's POPCs and selects
+// (about 40 issue slots per step) fit beside its P FP64 instructions, which
+// take 64 each of an SM quarter.  hex27 40^3 (297.7 M entries): 0.87 ms;
+// expanding the structural values first and k_spmv took 2.55 + 0.83 ms.
 template <int P>
 __global__ void __launch_bounds__(CG_THREADS)
-k_spmv_kept(const double *__restrict__ vals, const int64_t *__restrict__ colptr_s, const uint2 *__restrict__ keep,
-            const int64_t *__restrict__ nptr, const int32_t *__restrict__ nadj, const double *__restrict__ x,
+k_spmv_kept(KeptCols K, const int64_t *__restrict__ nptr, const int32_t *__restrict__ nadj, const double *__restrict__ x,
             double *__restrict__ y, int64_t non) {
   constexpr int NPW = 32 / SPMV_G;  // nodes per warp
   const int lane = threadIdx.x & 31, g = lane % SPMV_G, wpb = blockDim.x >> 5;
@@ -210,47 +263,7 @@ k_spmv_kept(const double *__restrict__ vals, const int64_t *__restrict__ colptr_
   for (int64_t B0 = ((int64_t)blockIdx.x * wpb + (threadIdx.x >> 5)) * NPW; B0 < non; B0 += stride) {
     const int64_t B = B0 + lane / SPMV_G;
     double acc[P];
-#pragma unroll
-    for (int j = 0; j < P; ++j) acc[j] = 0.0;
-    if (B < non) {
-      const int64_t r0 = nptr[B];
-      const int n = (int)(nptr[B + 1] - r0) * P;
-      const double *v[P];
-      const unsigned *kw[P];   // a word per 32 entries
-      unsigned w[P];
-#pragma unroll
-      for (int j = 0; j < P; ++j) {
-        v[j] = vals + (colptr_s[P * B + j] - 1);
-        kw[j] = reinterpret_cast<const unsigned *>(keep + keep_pos((int64_t)P * P * r0 + (int64_t)j * n, P * B + j));
-        w[j] = n > 0 ? kw[j][0] : 0u;
-      }
-      for (int k0 = 0; k0 < n; k0 += 32) {
-        unsigned nx[P];   // the next words, a block of entries ahead
-#pragma unroll
-        for (int j = 0; j < P; ++j) nx[j] = k0 + 32 < n ? kw[j][(k0 >> 5) + 1] : 0u;
-        const int lim = n - k0 < 32 ? n - k0 : 32;
-#pragma unroll 2
-        for (int i = g; i < lim; i += SPMV_G) {
-          const int k = k0 + i;
-          const double xa = x[(int64_t)P * nadj[r0 + k / P] + k % P];
-          const unsigned below = (1u << i) - 1u;
-          double a[P];
-#pragma unroll
-          for (int j = 0; j < P; ++j) a[j] = (w[j] >> i) & 1u ? v[j][__popc(w[j] & below)] : 0.0;
-#pragma unroll
-          for (int j = 0; j < P; ++j) acc[j] = __fma_rn(a[j], xa, acc[j]);
-        }
-#pragma unroll
-        for (int j = 0; j < P; ++j) {
-          v[j] += __popc(w[j]);
-          w[j] = nx[j];
-        }
-      }
-    }
-#pragma unroll
-    for (int off = SPMV_G / 2; off > 0; off >>= 1)
-#pragma unroll
-      for (int j = 0; j < P; ++j) acc[j] = __dadd_rn(acc[j], __shfl_xor_sync(0xffffffffu, acc[j], off));
+    node_columns_kept<P>(K, nadj, x, B, B < non ? nptr[B] : 0, B < non ? nptr[B + 1] : 0, B < non, g, acc);
     if (B < non && g < P) {
       double t = acc[0];
 #pragma unroll
@@ -267,10 +280,20 @@ __global__ void k_diag_scale(const double *__restrict__ d, const double *__restr
     y[i] = __dmul_rn(d[i], x[i]);
 }
 
+// Entry i of column c (structural start cs) from the stored values.
+__device__ __forceinline__ double kept_entry(const KeptCols &K, int64_t cs, int64_t c, int64_t i) {
+  const unsigned *w = reinterpret_cast<const unsigned *>(K.keep + keep_pos(cs, c));
+  const unsigned last = w[i >> 5], bit = 1u << (i & 31);
+  if (!(last & bit)) return 0.0;
+  int64_t rank = __popc(last & (bit - 1u));
+  for (int64_t k = 0; k < i >> 5; ++k) rank += __popc(w[k]);
+  return K.vals[K.colptr_s[c] - 1 + rank];
+}
+
 // Preconditioner setup: Jacobi 1/diag, or the inverse of each node's P x P
 // diagonal block (fixed DoFs replaced by identity rows/columns).
 template <int P>
-__global__ void k_precond_setup(const double *__restrict__ nz, const int64_t *__restrict__ colptr,
+__global__ void k_precond_setup(const double *__restrict__ nz, KeptCols K, const int64_t *__restrict__ colptr,
                                 const int32_t *__restrict__ diagpos, const uint8_t *__restrict__ fixed,
                                 int64_t non, int mode, double *__restrict__ pinv) {
   for (int64_t B = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; B < non;
@@ -281,7 +304,9 @@ __global__ void k_precond_setup(const double *__restrict__ nz, const int64_t *__
     for (int j = 0; j < P; ++j) {
       const int64_t cs = colptr[P * B + j];
 #pragma unroll
-      for (int i = 0; i < P; ++i) D[i][j] = dp >= 0 ? nz[cs + (int64_t)P * dp + i] : 0.0;
+      for (int i = 0; i < P; ++i)
+        D[i][j] = dp < 0 ? 0.0
+                         : (nz ? nz[cs + (int64_t)P * dp + i] : kept_entry(K, cs, P * B + j, (int64_t)P * dp + i));
     }
     if (mode == LLF_PRECOND_BJACOBI) {
 #pragma unroll
@@ -523,13 +548,14 @@ __global__ void k_seg_dir(Seg S, const double *__restrict__ z, double *__restric
 // node column B (chunks start and end on node boundaries), the chunk's nodes
 // taken in the order S.perm gives (decreasing degree: the eight nodes of a
 // warp have lists of similar length, so few lanes idle in the FP64 products).
-// A column's sums do not depend on the order.  c is kept in shared memory as
+// A column's sums do not depend on the order; KEPT takes them from the stored
+// values (llf_pcg_noalloc, which may not expand the structural ones).  c is kept in shared memory as
 // well, and the partial u.c takes the chunk's DoFs as the update's sums do
 // (thread t: DoFs t, t + 256, t + 512), every lane busy.  The block that brings in a segment's last
 // chunk sums the partials (chunk order) and sets alpha = rho / u.c.
-template <int P>
+template <int P, bool KEPT>
 __global__ void __launch_bounds__(CG_THREADS)
-k_seg_spmv(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ nptr,
+k_seg_spmv(Seg S, const double *__restrict__ nz, KeptCols K, const int64_t *__restrict__ nptr,
            const int32_t *__restrict__ nadj, const double *__restrict__ u,
            const uint8_t *__restrict__ fixed, double *__restrict__ c, double *__restrict__ part) {
   constexpr int NPW = 32 / SPMV_G;  // nodes per warp
@@ -553,7 +579,10 @@ k_seg_spmv(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ npt
       const bool vn = r + step < nb;
       const int64_t q0n = vn ? nptr[Bn] : 0, q1n = vn ? nptr[Bn + 1] : 0;
       double acc[P];
-      node_columns_at<P>(nz, nadj, u, q0, q1, valid, g, acc);
+      if (KEPT)
+        node_columns_kept<P>(K, nadj, u, B, q0, q1, valid, g, acc);
+      else
+        node_columns_at<P>(nz, nadj, u, q0, q1, valid, g, acc);
       if (valid && g == 0) {
 #pragma unroll
         for (int j = 0; j < P; ++j) {
@@ -1374,6 +1403,26 @@ void enqueue_ic0(llf_ctx *ctx, const Seg &S, const llf_matrix *m, const IcApply 
   { KernelScope k(ctx, "k_seg_zr"); k_seg_zr<<<chunk_grid(S), CG_THREADS, 0, ctx->stream>>>(S, ic.zf, r, z, part); }
 }
 
+KeptCols kept_cols(const llf_matrix *m) {
+  return m->d_nz ? KeptCols{nullptr, nullptr, nullptr} : KeptCols{m->d_nzval_s, m->d_colptr_s, m->d_keep};
+}
+
+// y = A x, from whichever values the matrix holds.
+template <int P>
+void launch_spmv(llf_ctx *ctx, const llf_matrix *m, const double *x, double *y) {
+  const llf_pattern *p = m->pat;
+  const int64_t non = p->ndof / P;
+  constexpr int per_block = CG_THREADS / SPMV_G;
+  const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((non + per_block - 1) / per_block, 1 << 30));
+  if (m->d_nz) {
+    KernelScope ks(ctx, "k_spmv");
+    k_spmv<P><<<grid, CG_THREADS, 0, ctx->stream>>>(m->d_nz, p->d_colptr, p->d_nptr, p->d_nadj, x, y, p->ndof);
+  } else {
+    KernelScope ks(ctx, "k_spmv_kept");
+    k_spmv_kept<P><<<grid, CG_THREADS, 0, ctx->stream>>>(kept_cols(m), p->d_nptr, p->d_nadj, x, y, non);
+  }
+}
+
 // z = M^-1 r and rho = z.r of the first iteration.
 template <int P>
 void enqueue_first_prec(llf_ctx *ctx, const Seg &S, const llf_matrix *m, const double *pinv, int precond,
@@ -1401,7 +1450,8 @@ void enqueue_iteration(llf_ctx *ctx, const Seg &S, const llf_matrix *m, const do
   const bool local = precond != LLF_PRECOND_IC0;
   { KernelScope k(ctx, "k_seg_dir"); k_seg_dir<<<chunk_grid(S), CG_THREADS, 0, s>>>(S, z, u); }
   { KernelScope k(ctx, "k_seg_spmv");
-    k_seg_spmv<P><<<chunk_grid(S), CG_THREADS, 0, s>>>(S, m->d_nz, pat->d_nptr, pat->d_nadj, u, fixed, c, part3); }
+    auto fn = m->d_nz ? k_seg_spmv<P, false> : k_seg_spmv<P, true>;
+    fn<<<chunk_grid(S), CG_THREADS, 0, s>>>(S, m->d_nz, kept_cols(m), pat->d_nptr, pat->d_nadj, u, fixed, c, part3); }
   { KernelScope k(ctx, "k_seg_update");
     k_seg_update_fused<P><<<chunk_grid(S), CG_THREADS, 0, s>>>(S, xw, r, u, c, part, part2, pinv, precond, local,
                                                                fixed, z); }
@@ -1684,10 +1734,10 @@ int pcg_core(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double *d_x, 
   if (precond != LLF_PRECOND_IC0) {
     KernelScope k(ctx, "k_precond_setup");
     k_precond_setup<P><<<(unsigned)((pat->mesh->non + 127) / 128), 128, 0, s>>>(
-        m->d_nz, pat->d_colptr, pat->d_diagpos, d_fixed, pat->mesh->non, precond, pinv);
+        m->d_nz, kept_cols(m), pat->d_colptr, pat->d_diagpos, d_fixed, pat->mesh->non, precond, pinv);
   }
   { KernelScope k(ctx, "k_keep_fixed"); k_keep_fixed<<<gv, CG_THREADS, 0, s>>>(d_x, d_fixed, xw, n); }
-  { KernelScope k(ctx, "k_spmv"); k_spmv<P><<<gv, CG_THREADS, 0, s>>>(m->d_nz, pat->d_colptr, pat->d_nptr, pat->d_nadj, xw, c, n); }
+  launch_spmv<P>(ctx, m, xw, c);
   { KernelScope k(ctx, "k_seg_init"); k_seg_init<<<gch, CG_THREADS, 0, s>>>(S, d_b, c, d_fixed, r, xw, u, part); }
   { KernelScope k(ctx, "k_seg_start"); k_seg_start<<<gseg, CG_THREADS, 0, s>>>(S, part, reltol, (long long)maxiter); }
   enqueue_first_prec<P>(ctx, S, m, pinv, precond, r, z, d_fixed, part, gch, gseg, ic);
@@ -2134,7 +2184,7 @@ int pcg_mixed_core(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double 
   if (local) {
     KernelScope k(ctx, "k_precond_setup");
     k_precond_setup<P><<<(unsigned)((pat->mesh->non + 127) / 128), 128, 0, s>>>(
-        m->d_nz, pat->d_colptr, pat->d_diagpos, d_fixed, pat->mesh->non, precond, pinv);
+        m->d_nz, kept_cols(m), pat->d_colptr, pat->d_diagpos, d_fixed, pat->mesh->non, precond, pinv);
   }
   { KernelScope k(ctx, "k_f64_to_f32");
     k_f64_to_f32<<<(unsigned)(ctx->num_sms * 8), CG_THREADS, 0, s>>>(m->d_nz, B.nz32, pat->nnz); }
@@ -2338,7 +2388,7 @@ int pcg_noalloc_typed(llf_ctx *ctx, const llf_matrix *m, const double *d_b, doub
 int pcg_noalloc_impl(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double *d_x,
                      const uint8_t *d_fixed, int precond, double reltol, int64_t maxiter,
                      int64_t *iters, double *relres) {
-  if (!m->d_nz && !m->diagonal_only)
+  if (!m->d_nz && !m->diagonal_only && !(m->d_keep && m->multiplied.load()))
     return llf_fail(ctx, LLF_ERR_STATE,
                     "llf_pcg_noalloc: the matrix's structural values are not expanded yet (its assembly wrote the "
                     "stored CSC only); run llf_pcg or llf_matrix_spmv on it once first");
@@ -2362,21 +2412,6 @@ namespace {
 // One warp per eight column nodes, one round of them per warp, so that the
 // block scheduler balances the nodes' uneven lists (hex27 40^3: 1.00 -> 0.93
 // ms, from the kept values 1.31 -> 0.97 ms, against four blocks per SM).
-template <int P>
-void launch_spmv(llf_ctx *ctx, const llf_matrix *m, const double *x, double *y) {
-  const llf_pattern *p = m->pat;
-  const int64_t non = p->ndof / P;
-  constexpr int per_block = CG_THREADS / SPMV_G;
-  const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((non + per_block - 1) / per_block, 1 << 30));
-  if (m->d_nz) {
-    KernelScope ks(ctx, "k_spmv");
-    k_spmv<P><<<grid, CG_THREADS, 0, ctx->stream>>>(m->d_nz, p->d_colptr, p->d_nptr, p->d_nadj, x, y, p->ndof);
-  } else {
-    KernelScope ks(ctx, "k_spmv_kept");
-    k_spmv_kept<P><<<grid, CG_THREADS, 0, ctx->stream>>>(m->d_nzval_s, m->d_colptr_s, m->d_keep, p->d_nptr, p->d_nadj,
-                                                         x, y, non);
-  }
-}
 }  // namespace
 
 int spmv_impl(llf_ctx *ctx, const llf_matrix *m, const double *d_x, double *d_y) {
@@ -2398,6 +2433,7 @@ int spmv_impl(llf_ctx *ctx, const llf_matrix *m, const double *d_x, double *d_y)
     }
   }
   LLF_CUDA_TRY(ctx, cudaGetLastError());
+  m->multiplied.store(true);
   return LLF_OK;
 }
 
@@ -2863,7 +2899,7 @@ int prepare_t(llf_ctx *ctx, const llf_matrix *K, const double *hb, const double 
     k_chunk_perm<<<chunk_grid(S), CG_THREADS, 0, s>>>(S, pat->d_nptr, P, sy->perm);
   }
   { KernelScope k(ctx, "k_precond_setup");
-    k_precond_setup<P><<<(unsigned)((non + 127) / 128), 128, 0, s>>>(K->d_nz, pat->d_colptr, pat->d_diagpos, sy->fixed,
+    k_precond_setup<P><<<(unsigned)((non + 127) / 128), 128, 0, s>>>(K->d_nz, kept_cols(K), pat->d_colptr, pat->d_diagpos, sy->fixed,
                                                                      non, precond, sy->pinv); }
   { KernelScope k(ctx, "k_keep_fixed"); k_keep_fixed<<<gv, CG_THREADS, 0, s>>>(sy->x, sy->fixed, sy->xw, n); }
   { KernelScope k(ctx, "k_spmv");

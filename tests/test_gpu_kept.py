@@ -59,3 +59,43 @@ def test_kept_product_and_expansion_equal_structural(llf, case, turned, precisio
     x[1], x[-1] = np.nan, np.inf
     again = _assemble(llf, P, op, precision=precision)
     assert np.array_equal(again * x, kept * x, equal_nan=True)
+
+
+@pytest.mark.parametrize("case", [("Solid", (5, 4, 6), 2, 3), ("PlaneStress", (9, 7), 2, 2), ("HeatConduction", (6, 5, 4), 1, 1)],
+                         ids=["hex27", "quad9", "heat"])
+@pytest.mark.parametrize("precond", [0, 1, 2])
+def test_noalloc_from_the_stored_values(llf, case, precond):
+    """A product lets llf_pcg_noalloc take a matrix that holds its stored CSC
+    only; it allocates nothing and gives the bits of the expanded matrix."""
+    typ, cells, order, P = case
+    L = [float(c) for c in cells]
+    m = (llf.structured_box_mesh(lx=L[0], ly=L[1], lz=L[2], dx=1.0, dy=1.0, order=order) if len(cells) == 3 else
+         llf.structured_rect_mesh(lx=L[0], ly=L[1], dx=1.0, dy=1.0, order=order))
+    prob = llf.Problem([llf.Material("body", E=2.1e5, nu=0.3, k=45.0)], type=typ, mesh=m)
+    make = llf.heatConductionMatrix if typ == "HeatConduction" else llf.stiffnessMatrix
+    K1 = make(prob)
+    K2, K3 = make(prob), make(prob)   # assembled into the kept layout
+    fixed = np.repeat(m.xyz[:, 0] < 1e-9, P)
+    b = np.random.default_rng(5).standard_normal(P * m.non)
+    with pytest.raises(llf.LLFError, match="not expanded"):
+        _noalloc(llf, K2, b, fixed, precond)
+    assert np.array_equal(K2.dm.spmv(b), K1.dm.spmv(b))
+    K3.dm.prepare()
+    got, want = _noalloc(llf, K2, b, fixed, precond), _noalloc(llf, K3, b, fixed, precond)
+    assert got[1] == want[1] and np.array_equal(got[0], want[0])
+
+
+def _noalloc(llf, K, b, fixed, precond):
+    import ctypes as C
+
+    torch = pytest.importorskip("torch")
+    db = torch.from_numpy(b).cuda()
+    dx = torch.zeros_like(db)
+    df = torch.from_numpy(fixed.astype(np.uint8)).cuda()
+    torch.cuda.synchronize()
+    it, rr, allocs0 = C.c_int64(0), C.c_double(0.0), K.dm.ctx.allocs()
+    rc = llf._lib.lib().llf_pcg_noalloc(K.dm.ctx.h, K.dm.h, C.c_void_p(db.data_ptr()), C.c_void_p(dx.data_ptr()),
+                                        C.c_void_p(df.data_ptr()), precond, 1e-8, 20 * len(b), C.byref(it), C.byref(rr))
+    K.dm.ctx.check(rc, "llf_pcg_noalloc")
+    assert K.dm.ctx.allocs() == allocs0
+    return dx.cpu().numpy(), it.value
