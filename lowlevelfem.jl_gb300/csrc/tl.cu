@@ -588,25 +588,37 @@ __global__ void __launch_bounds__(TL_THREADS) k_tl_force(TLArgs A, int E) {
 // the tangent is [B_q; G_q]^T diag(w D_q, w S_q (x) I) [B_q; G_q], with B_q
 // the 6 x 3npe matrix B(F) and G_q the 9 x 3npe displacement-gradient
 // operator, so the whole element matrix is one GEMM over K = 15 rows per
-// point.  One CTA computes a 128 x 192 tile of one element matrix:
+// point.  One CTA computes 128 columns x 192 rows of one element matrix:
 //   - the point data (F, w D, w S, physical gradients; FP64 as in the FP64
 //     form, rounded to FP32) come from k_tl_points_tc, two points per
-//     k-block, fetched by cp.async.bulk one k-block ahead;
-//   - per k-block of 2 points (2 x 15 rows, padded to 32) the threads build
-//     the A (= [B; G] rows of the tile) and B (= weighted [D B; S G]) tiles
-//     in shared memory in the K-major core-matrix layout (8 rows x 16 bytes),
-//     each split into TF32 hi and lo parts;
+//     k-block, fetched by cp.async.bulk two k-blocks ahead;
+//   - per k-block of 2 points (2 x 15 K values, padded to 32) eight warps form
+//     the weighted operands [D B; S G] of the tile's columns, a thread per
+//     column and point, and write them to tensor memory (tcgen05.st: the M
+//     operand), while the other eight form [B; G] of the tile's rows in shared
+//     memory (the N operand, K-major core matrices of 8 rows x 16 bytes).
+//     Both are split into TF32 hi and lo parts;
 //   - one thread issues tcgen05.mma kind::tf32 (M 128, N 192, K 8) for the
 //     three split products hi*hi + hi*lo + lo*hi into an FP32 accumulator in
-//     tensor memory and commits to the stage's mbarrier (two stages, the
-//     next k-block is built while the tensor cores run);
+//     tensor memory and commits to an mbarrier;
 //   - the epilogue reads the accumulator with tcgen05.ld and writes the
 //     element matrix (FP32) in the gather's layout.
+// Two CTAs per SM (256 columns of tensor memory each): one builds while the
+// other's products run.
+// Bound by the tensor cores' TF32 rate (1.03 TFLOP of split products for 576
+// hex125: 1.1 ms) and what of the build their two CTAs leave uncovered.
+// Forming both operands in shared memory, one CTA per SM and two stages, was
+// bound by the build: 2.30 ms; with the M operand, the dearer of the two, in
+// tensor memory it is 128 columns a thread each instead of 192, without
+// shared-memory traffic on either side, and the build hides: 1.50 ms.  A
+// separate product for the geometric part (K 6 + 3 instead of 15) took 1.40 ms
+// but sums the same terms in another order.
 // Every mbarrier wait is bounded (2 s): a timeout sets ST_TIMEOUT, the CTA
 // skips its epilogue and releases its tensor memory.
 constexpr int TC_M = 128, TC_N = 192, TC_KB = 32, TC_PTS = 2, TC_THREADS = 512;
-constexpr int TC_TILE_A = TC_M * TC_KB, TC_TILE_B = TC_N * TC_KB;  // floats
-constexpr size_t TC_STAGE = (size_t)2 * (TC_TILE_A + TC_TILE_B);   // floats per stage (hi + lo)
+constexpr int TC_TILE = TC_N * TC_KB;   // floats of the N operand's tile (hi or lo)
+constexpr int TC_COL_HI = TC_N, TC_COL_LO = TC_N + TC_KB, TC_COLS = 256;   // tensor memory: accumulator | M operand
+static_assert(TC_THREADS == 2 * TC_M * TC_PTS, "half the threads: one per column and point");
 
 struct TcArgs {
   const float *pd;     // nel * nip * tc_pstride(npe) packed point data (k_tl_points_tc)
@@ -638,24 +650,48 @@ __device__ __forceinline__ float tc_tf32(float x) {
   return __uint_as_float(r);
 }
 
-// Row `row`, columns k0 .. k0+15 (k0 a multiple of 4) of a tile: TF32 hi and
-// lo parts, one 16-byte store per 4 columns (a core-matrix row).
-__device__ __forceinline__ void tc_put16(float *hi, float *lo, int row, int k0, const float *v) {
+// The 16 K values of a row at a point: b[6], then g in the places of
+// component ci of [G] (gradient index times 3 plus component), hi and lo parts.
+__device__ __forceinline__ void tc_row16(const float (&b)[6], const float (&g)[3], int ci, float (&h)[16],
+                                         float (&l)[16]) {
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    float4 h, l;
-    h.x = tc_tf32(v[4 * c]);
-    h.y = tc_tf32(v[4 * c + 1]);
-    h.z = tc_tf32(v[4 * c + 2]);
-    h.w = tc_tf32(v[4 * c + 3]);
-    l.x = v[4 * c] - h.x;
-    l.y = v[4 * c + 1] - h.y;
-    l.z = v[4 * c + 2] - h.z;
-    l.w = v[4 * c + 3] - h.w;
-    const int o = tc_off(row, k0 + 4 * c);
-    *reinterpret_cast<float4 *>(hi + o) = h;
-    *reinterpret_cast<float4 *>(lo + o) = l;
+  for (int r = 0; r < 6; ++r) {
+    h[r] = tc_tf32(b[r]);
+    l[r] = b[r] - h[r];
   }
+#pragma unroll
+  for (int I = 0; I < 3; ++I) {
+    const float gh = tc_tf32(g[I]), gl = g[I] - gh;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      h[6 + 3 * I + c] = c == ci ? gh : 0.f;
+      l[6 + 3 * I + c] = c == ci ? gl : 0.f;
+    }
+  }
+  h[15] = l[15] = 0.f;
+}
+
+// B(F) of a node with gradient g at component ci (F's row ci).
+__device__ __forceinline__ void tc_brow(const float *F, int ci, const float (&g)[3], float (&b)[6]) {
+  const float v1 = F[3 * ci], v2 = F[3 * ci + 1], v3 = F[3 * ci + 2];
+  b[0] = v1 * g[0];
+  b[1] = v2 * g[1];
+  b[2] = v3 * g[2];
+  b[3] = fmaf(v2, g[2], v3 * g[1]);
+  b[4] = fmaf(v1, g[2], v3 * g[0]);
+  b[5] = fmaf(v1, g[1], v2 * g[0]);
+}
+
+// 16 values of this thread's tensor-memory lane.
+__device__ __forceinline__ void tc_st16(uint32_t addr, const float (&v)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(addr), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
+                 "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
+                 "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])), "r"(__float_as_uint(v[8])),
+                 "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
+                 "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])),
+                 "r"(__float_as_uint(v[15]))
+               : "memory");
 }
 
 __device__ __forceinline__ uint64_t tc_now() {
@@ -679,9 +715,10 @@ __device__ __forceinline__ bool tc_wait(uint64_t *bar, unsigned parity) {
 
 // Packed FP32 point data of the tensor-core form, one CTA per element: for
 // every point q a run of tc_pstride(npe) floats (16-byte multiple)
-//   [0,9) F | [9,45) w D | [45,54) w S | [54,56) 0 | [56, 56+3 npe) grad N_a
+//   [0,9) F | [12,48) w D | [48,57) w S | [60, 60+3 npe) grad N_a, 0 between
 // computed in FP64 (the FP64 form's point record and gradients) and rounded.
-__host__ __device__ __forceinline__ int tc_pstride(int npe) { return (56 + 3 * npe + 3) & ~3; }
+constexpr int TP_D = 12, TP_S = 48, TP_G = 60;   // 16-byte aligned parts
+__host__ __device__ __forceinline__ int tc_pstride(int npe) { return (TP_G + 3 * npe + 3) & ~3; }
 
 __global__ void __launch_bounds__(TL_THREADS) k_tl_points_tc(TLArgs A, float *pd) {
   extern __shared__ double sm[];
@@ -701,10 +738,10 @@ __global__ void __launch_bounds__(TL_THREADS) k_tl_points_tc(TLArgs A, float *pd
       const double *r = rec + (size_t)q * QD;
       double v = 0.0;
       if (f < 9) v = r[10 + f];
-      else if (f < 45) v = __dmul_rn(r[0], r[19 + (f - 9)]);
-      else if (f < 54) v = __dmul_rn(r[0], r[55 + (f - 45)]);
-      else if (f >= 56 && f < 56 + 3 * npe) {
-        const int a = (f - 56) / 3, I = (f - 56) % 3;
+      else if (f >= TP_D && f < TP_D + 36) v = __dmul_rn(r[0], r[19 + (f - TP_D)]);
+      else if (f >= TP_S && f < TP_S + 9) v = __dmul_rn(r[0], r[55 + (f - TP_S)]);
+      else if (f >= TP_G && f < TP_G + 3 * npe) {
+        const int a = (f - TP_G) / 3, I = (f - TP_G) % 3;
         const double *d = A.dN + ((size_t)q * npe + a) * 3;
         double g = 0.0;
         for (int J = 0; J < 3; ++J) g = __fma_rn(r[1 + 3 * J + I], d[J], g);
@@ -723,35 +760,40 @@ __device__ __forceinline__ void tc_bulk(void *dst, const void *src, unsigned byt
                : "memory");
 }
 
-// Shared memory: 2 stages x (A hi, A lo, B hi, B lo) | 2 point-data buffers
-// (TC_PTS points each, fetched by cp.async.bulk one k-block ahead) |
-// (TC_N / (TC_THREADS / 128) must be a multiple of 16)
-// mbarriers: MMA completion x2, point data x2 | tensor-memory address.
-__global__ void __launch_bounds__(TC_THREADS, 1) k_tl_tangent_tc(TcArgs A) {
+// Shared memory: N operand hi, lo | 2 point-data buffers (TC_PTS points each,
+// fetched by cp.async.bulk two k-blocks ahead) | mbarriers: products, point
+// data x2 | tensor-memory address.
+__global__ void __launch_bounds__(TC_THREADS, 2) k_tl_tangent_tc(TcArgs A) {
   extern __shared__ __align__(1024) float tsm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int per_e = A.nstrip * A.nhalf;
   const int64_t e = blockIdx.x / per_e;
   const int rr = (int)(blockIdx.x - e * per_e);
-  const int row0 = (rr / A.nhalf) * TC_M, col0 = (rr % A.nhalf) * TC_N;
+  const int col0 = (rr / A.nhalf) * TC_M, row0 = (rr % A.nhalf) * TC_N;
   if (e >= A.nel || (A.emat && A.emat[e] < 0)) return;  // uniform across the CTA
   const int npe = A.npe, nip = A.nip, n = A.n, ps = tc_pstride(npe);
-  float *pbuf = tsm + 2 * TC_STAGE;                      // 2 x TC_PTS * ps
-  uint64_t *bar = (uint64_t *)(pbuf + 2 * TC_PTS * ps);  // [0,2) MMA, [2,4) point data
-  uint32_t *tslot = (uint32_t *)(bar + 4);
+  float *Nhi = tsm, *Nlo = Nhi + TC_TILE;
+  float *pbuf = tsm + 2 * TC_TILE;                       // 2 x TC_PTS * ps
+  uint64_t *bar = (uint64_t *)(pbuf + 2 * TC_PTS * ps);  // 0 products, 1 and 2 point data
+  uint32_t *tslot = (uint32_t *)(bar + 3);
   const float *pd = A.pd + (size_t)e * nip * ps;
   const int nkb = (nip + TC_PTS - 1) / TC_PTS;
+  auto fetch = [&](int kb) {   // point data of k-block kb into buffer kb & 1
+    const int q0 = kb * TC_PTS, np = nip - q0 < TC_PTS ? nip - q0 : TC_PTS;
+    tc_bulk(pbuf + (kb & 1) * TC_PTS * ps, pd + (size_t)q0 * ps, (unsigned)(np * ps * sizeof(float)), bar + 1 + (kb & 1));
+  };
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_saddr(tslot)), "r"(256u)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_saddr(tslot)),
+                 "r"((uint32_t)TC_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
-    for (int b = 0; b < 4; ++b)
+    for (int b = 0; b < 3; ++b)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_saddr(bar + b)), "r"(1u) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    const int np = nip < TC_PTS ? nip : TC_PTS;
-    tc_bulk(pbuf, pd, (unsigned)(np * ps * sizeof(float)), bar + 2);
+    fetch(0);
+    if (nkb > 1) fetch(1);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -760,149 +802,159 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tl_tangent_tc(TcArgs A) {
   const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(TC_N >> 3) << 17) |
                          ((uint32_t)(TC_M >> 4) << 24);
   bool ok = true;
-  int fetched = 1;  // point-data copies issued (k-blocks 0 .. fetched-1)
+  int fetched = nkb < 2 ? nkb : 2;  // point-data copies issued (k-blocks 0 .. fetched-1)
   for (int kb = 0; kb < nkb; ++kb) {
-    const int st = kb & 1;
-    float *Ahi = tsm + st * TC_STAGE, *Alo = Ahi + TC_TILE_A, *Bhi = Alo + TC_TILE_A, *Blo = Bhi + TC_TILE_B;
-    // tiles of this stage free (MMAs of k-block kb - 2 done) and point data of kb landed
-    bool w = kb < 2 || tc_wait(bar + st, (unsigned)((kb - 2) >> 1) & 1u);
-    w = w && tc_wait(bar + 2 + st, (unsigned)(kb >> 1) & 1u);
+    const int q0 = kb * TC_PTS;
+    const float *pb = pbuf + (kb & 1) * TC_PTS * ps;
+    // the operands' values, formed while the products of k-block kb - 1 run;
+    // they are split and stored once those are done
+    bool w = tc_wait(bar + 1 + (kb & 1), (unsigned)(kb >> 1) & 1u);
+    if (warp < TC_THREADS / 64) {
+      // M operand: column col0 + 32 (warp % 4) + lane (the lanes of tensor
+      // memory this warp may access) at point warp / 4, so w D and w S are
+      // broadcasts
+      const int ql = warp >> 2, gj = col0 + (warp & 3) * 32 + lane;
+      float d[6], sg[3];
+#pragma unroll
+      for (int r = 0; r < 6; ++r) d[r] = 0.f;
+#pragma unroll
+      for (int I = 0; I < 3; ++I) sg[I] = 0.f;
+      const int b = gj / 3, cj = gj - 3 * b;
+      if (gj < n && q0 + ql < nip) {
+        const float *P = pb + ql * ps;
+        const float g[3] = {P[TP_G + 3 * b], P[TP_G + 3 * b + 1], P[TP_G + 3 * b + 2]};
+        float Bv[6];
+        tc_brow(P, cj, g, Bv);
+        const float4 *wD = reinterpret_cast<const float4 *>(P + TP_D);
+#pragma unroll
+        for (int r = 0; r < 6; r += 2) {   // two rows of w D: three 16-byte words
+          float t[12];
+#pragma unroll
+          for (int x = 0; x < 3; ++x) *reinterpret_cast<float4 *>(t + 4 * x) = wD[r * 6 / 4 + x];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            float acc = 0.f;
+#pragma unroll
+            for (int r2 = 0; r2 < 6; ++r2) acc = fmaf(t[6 * u + r2], Bv[r2], acc);
+            d[r + u] = acc;
+          }
+        }
+#pragma unroll
+        for (int I = 0; I < 3; ++I)
+#pragma unroll
+          for (int J = 0; J < 3; ++J) sg[I] = fmaf(P[TP_S + 3 * I + J], g[J], sg[I]);
+      }
+      if (kb > 0) w = w && tc_wait(bar, (unsigned)(kb - 1) & 1u);
+      if (__all_sync(0xffffffffu, w)) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        float h[16], l[16];
+        tc_row16(d, sg, cj, h, l);
+        const uint32_t t0 = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(ql * 16);
+        tc_st16(t0 + TC_COL_HI, h);
+        tc_st16(t0 + TC_COL_LO, l);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      }
+    } else {
+      // N operand: the tile's rows (a warp's rows share the point)
+      constexpr int ROUNDS = (TC_N * TC_PTS + TC_THREADS / 2 - 1) / (TC_THREADS / 2);
+      float g[ROUNDS][3], Bv[ROUNDS][6];
+#pragma unroll
+      for (int k = 0; k < ROUNDS; ++k) {
+        const int t = tid - TC_THREADS / 2 + k * (TC_THREADS / 2), ql = t / TC_N, gi = row0 + t - ql * TC_N;
+#pragma unroll
+        for (int r = 0; r < 6; ++r) Bv[k][r] = 0.f;
+#pragma unroll
+        for (int I = 0; I < 3; ++I) g[k][I] = 0.f;
+        if (t < TC_N * TC_PTS && gi < n && q0 + ql < nip) {
+          const float *P = pb + ql * ps;
+          const int a = gi / 3;
+#pragma unroll
+          for (int I = 0; I < 3; ++I) g[k][I] = P[TP_G + 3 * a + I];
+          tc_brow(P, gi - 3 * a, g[k], Bv[k]);
+        }
+      }
+      if (kb > 0) w = w && tc_wait(bar, (unsigned)(kb - 1) & 1u);
+      if (w) {
+#pragma unroll
+        for (int k = 0; k < ROUNDS; ++k) {
+          const int t = tid - TC_THREADS / 2 + k * (TC_THREADS / 2), ql = t / TC_N, i = t - ql * TC_N;
+          if (t >= TC_N * TC_PTS) break;
+          float h[16], l[16];
+          tc_row16(Bv[k], g[k], i % 3, h, l);   // row0 is a multiple of 3
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int o = tc_off(i, ql * 16 + 4 * c);
+            *reinterpret_cast<float4 *>(Nhi + o) = make_float4(h[4 * c], h[4 * c + 1], h[4 * c + 2], h[4 * c + 3]);
+            *reinterpret_cast<float4 *>(Nlo + o) = make_float4(l[4 * c], l[4 * c + 1], l[4 * c + 2], l[4 * c + 3]);
+          }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      }
+    }
     if (!__syncthreads_and(w)) {
       ok = false;
       break;
     }
-    // prefetch the next k-block's point data into the other buffer (its last
-    // reader, the tile build of kb - 1, finished before the barrier above)
-    if (kb + 1 < nkb) {
-      if (tid == 0) {
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        const int q1 = (kb + 1) * TC_PTS, np = (nip - q1) < TC_PTS ? (nip - q1) : TC_PTS;
-        tc_bulk(pbuf + ((kb + 1) & 1) * TC_PTS * ps, pd + (size_t)q1 * ps, (unsigned)(np * ps * sizeof(float)),
-                bar + 2 + ((kb + 1) & 1));
-      }
-      ++fetched;
-    }
-    const int q0 = kb * TC_PTS;
-    const float *pb = pbuf + st * TC_PTS * ps;
-    // A tile: rows of the strip, K = (point, 16 rows: B(F) 6, grad 9, pad 1)
-    for (int t = tid; t < TC_M * TC_PTS; t += TC_THREADS) {
-      const int ql = t / TC_M, i = t - ql * TC_M, gi = row0 + i, q = q0 + ql;
-      float v[16];
-#pragma unroll
-      for (int r = 0; r < 16; ++r) v[r] = 0.f;
-      if (gi < n && q < nip) {
-        const int a = gi / 3, ci = gi - 3 * (gi / 3);
-        const float *P = pb + ql * ps, *g = P + 56 + 3 * a;
-        const float v1 = P[3 * ci], v2 = P[3 * ci + 1], v3 = P[3 * ci + 2];
-        v[0] = v1 * g[0];
-        v[1] = v2 * g[1];
-        v[2] = v3 * g[2];
-        v[3] = fmaf(v2, g[2], v3 * g[1]);
-        v[4] = fmaf(v1, g[2], v3 * g[0]);
-        v[5] = fmaf(v1, g[1], v2 * g[0]);
-#pragma unroll
-        for (int I = 0; I < 3; ++I)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) v[6 + 3 * I + c] = (c == ci) ? g[I] : 0.f;
-      }
-      tc_put16(Ahi, Alo, i, ql * 16, v);
-    }
-    // B tile: columns of the half, weighted by w D and w S
-    for (int t = tid; t < TC_N * TC_PTS; t += TC_THREADS) {
-      const int ql = t / TC_N, j = t - ql * TC_N, gj = col0 + j, q = q0 + ql;
-      float v[16];
-#pragma unroll
-      for (int r = 0; r < 16; ++r) v[r] = 0.f;
-      if (gj < n && q < nip) {
-        const int b = gj / 3, cj = gj - 3 * (gj / 3);
-        const float *P = pb + ql * ps, *g = P + 56 + 3 * b;
-        const float v1 = P[3 * cj], v2 = P[3 * cj + 1], v3 = P[3 * cj + 2];
-        float Bv[6];
-        Bv[0] = v1 * g[0];
-        Bv[1] = v2 * g[1];
-        Bv[2] = v3 * g[2];
-        Bv[3] = fmaf(v2, g[2], v3 * g[1]);
-        Bv[4] = fmaf(v1, g[2], v3 * g[0]);
-        Bv[5] = fmaf(v1, g[1], v2 * g[0]);
-        const float *wD = P + 9, *wS = P + 45;
-#pragma unroll
-        for (int r = 0; r < 6; ++r) {
-          float sacc = 0.f;
-#pragma unroll
-          for (int r2 = 0; r2 < 6; ++r2) sacc = fmaf(wD[r * 6 + r2], Bv[r2], sacc);
-          v[r] = sacc;
-        }
-#pragma unroll
-        for (int I = 0; I < 3; ++I) {
-          float sacc = 0.f;
-#pragma unroll
-          for (int J = 0; J < 3; ++J) sacc = fmaf(wS[3 * I + J], g[J], sacc);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) v[6 + 3 * I + c] = (c == cj) ? sacc : 0.f;
-        }
-      }
-      tc_put16(Bhi, Blo, j, ql * 16, v);
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
     if (tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
       for (int kk = 0; kk < TC_KB / 8; ++kk)
 #pragma unroll
-        for (int p = 0; p < 3; ++p) {
-          const float *Ax = (p == 2 ? Alo : Ahi) + kk * 64, *Bx = (p == 1 ? Blo : Bhi) + kk * 64;
+        for (int p = 0; p < 3; ++p) {   // hi hi, then the columns' lo, then the rows' lo
+          const uint32_t Mx = tmem + (uint32_t)((p == 1 ? TC_COL_LO : TC_COL_HI) + kk * 8);
+          const float *Nx = (p == 2 ? Nlo : Nhi) + kk * 64;
           const uint32_t acc = (kb | kk | p) != 0;
           asm volatile("{\n\t.reg .pred pa;\n\tsetp.ne.b32 pa, %4, 0;\n\t"
-                       "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, pa;\n\t}"
-                       ::"r"(tmem), "l"(tc_desc(Ax)), "l"(tc_desc(Bx)), "r"(idesc), "r"(acc)
+                       "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, pa;\n\t}"
+                       ::"r"(tmem), "r"(Mx), "l"(tc_desc(Nx)), "r"(idesc), "r"(acc)
                        : "memory");
         }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                       tc_saddr(bar + st))
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_saddr(bar))
                    : "memory");
+      if (kb + 2 < nkb) {   // every thread has read the point data of kb
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        fetch(kb + 2);
+      }
     }
+    if (kb + 2 < nkb) ++fetched;
   }
   // the last commit covers every earlier MMA of this thread
-  const bool fin = ok ? tc_wait(bar + ((nkb - 1) & 1), (unsigned)((nkb - 1) >> 1) & 1u) : false;
+  const bool fin = ok ? tc_wait(bar, (unsigned)(nkb - 1) & 1u) : false;
   ok = __syncthreads_and(fin);
   if (!ok && tid == 0) atomicOr(A.status, ST_TIMEOUT);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (ok) {
-    // warp w reads TMEM lanes 32 (w % 4) .. +31 (the lanes its position in a
-    // warpgroup may access) and one of TC_THREADS / 128 column ranges
-    constexpr int NCR = TC_THREADS / 128, CW = TC_N / NCR;
+    // warp w reads TMEM lanes 32 (w % 4) .. +31 and 48 of the 192 rows (16 nodes)
+    constexpr int CW = TC_N / (TC_THREADS / 128);
+    static_assert(CW % 3 == 0 && CW % 16 == 0, "whole nodes, 16 columns a load");
     const int lanes = (warp & 3) * 32, cbeg = (warp >> 2) * CW;
-    const int gi = row0 + lanes + lane;
-    const int a = gi / 3, ci = gi - 3 * (gi / 3);
-    for (int c0 = cbeg; c0 < cbeg + CW; c0 += 16) {
-      uint32_t r[16];
-      const uint32_t addr = tmem + ((uint32_t)lanes << 16) + (uint32_t)c0;
-      asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                   : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                     "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                     "=r"(r[15])
-                   : "r"(addr));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (gi < n)
+    const int gj = col0 + lanes + lane, b = gj / 3, cj = gj - 3 * b;
+    uint32_t r[CW];
 #pragma unroll
-        for (int u = 0; u < 16; ++u) {
-          const int gj = col0 + c0 + u;
-          if (gj < n) {
-            const int b = gj / 3, cj = gj - 3 * (gj / 3);
-            A.Kf[((size_t)e * npe + b) * A.cs + a * kf_bstride(3, true, 4) + ci * 3 + cj] = __uint_as_float(r[u]);
-          }
-        }
+    for (int c0 = 0; c0 < CW; c0 += 16)
+      asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                   : "=r"(r[c0]), "=r"(r[c0 + 1]), "=r"(r[c0 + 2]), "=r"(r[c0 + 3]), "=r"(r[c0 + 4]), "=r"(r[c0 + 5]),
+                     "=r"(r[c0 + 6]), "=r"(r[c0 + 7]), "=r"(r[c0 + 8]), "=r"(r[c0 + 9]), "=r"(r[c0 + 10]),
+                     "=r"(r[c0 + 11]), "=r"(r[c0 + 12]), "=r"(r[c0 + 13]), "=r"(r[c0 + 14]), "=r"(r[c0 + 15])
+                   : "r"(tmem + ((uint32_t)lanes << 16) + (uint32_t)(cbeg + c0)));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    if (gj < n) {
+      float *K = A.Kf + ((size_t)e * npe + b) * A.cs + cj;
+      const int a0 = (row0 + cbeg) / 3;
+#pragma unroll
+      for (int u = 0; u < CW; ++u)
+        if (a0 + u / 3 < npe) K[(a0 + u / 3) * kf_bstride(3, true, 4) + (u % 3) * 3] = __uint_as_float(r[u]);
     }
   } else {
     // drain this CTA's point-data copies (bounded) before it exits: copy k of
     // buffer k & 1 is that buffer's (k >> 1)-th phase
-    for (int k = 0; k < fetched; ++k) tc_wait(bar + 2 + (k & 1), (unsigned)(k >> 1) & 1u);
+    for (int k = 0; k < fetched; ++k) tc_wait(bar + 1 + (k & 1), (unsigned)(k >> 1) & 1u);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TC_COLS) : "memory");
 }
 
 size_t tl_smem(int npe, int nip) {
@@ -1128,7 +1180,9 @@ int tl_tangent_tc_impl(llf_ctx *ctx, llf_mesh *mesh, llf_pattern *pat, const dou
   t.Kf = Kf;
   t.cs = cs;
   t.status = ctx->d_status;
-  const size_t smem = sizeof(float) * (2 * TC_STAGE + 2 * (size_t)TC_PTS * ps) + 4 * sizeof(uint64_t) + 16;
+  // at least 80 KB, so that at most two CTAs, whose tensor memory fits, share an SM
+  const size_t smem = std::max<size_t>(80 * 1024, sizeof(float) * (2 * TC_TILE + 2 * (size_t)TC_PTS * ps) +
+                                                      3 * sizeof(uint64_t) + 16);
   if (rc == LLF_OK && smem > 220 * 1024) rc = llf_fail(ctx, LLF_ERR_LIMIT, "tensor-core tangent: element too large");
   const int64_t ctas = mesh->nel * t.nstrip * t.nhalf;
   if (rc == LLF_OK && ctas >= ((int64_t)1 << 31)) rc = llf_fail(ctx, LLF_ERR_LIMIT, "tensor-core tangent: too many tiles");
