@@ -707,10 +707,14 @@ __global__ void k_keep_fixed(const double *__restrict__ x, const uint8_t *__rest
 // The whole iteration loop of systems of at most a few hundred chunks in one
 // cooperative kernel: one CTA per chunk, all resident, x, r, z, u and the
 // preconditioner of the chunk in registers, the chunk's node order, row
-// ranges and row nodes in shared memory.  The CTAs of one system meet three
-// times per iteration, each time at one word or word pair per chunk that every
-// CTA of the system polls: the new direction is written (the product reads it
-// from the other chunks), the partials of u.c, the partials of r.r and z.r.
+// ranges and row nodes in shared memory.  The CTAs of one system meet twice
+// per iteration, at word pairs that every CTA of the system pushes and polls:
+// the partials of u.c, the partials of r.r and z.r.  With the second go the z
+// of the chunk: each CTA keeps the u of its halo (the nodes of other chunks
+// that its columns meet) in shared memory and forms their next direction, z +
+// beta u, as their own CTAs do, so the product reads u (and, where they fit,
+// the columns) from shared memory.  Without HALO, for chunks whose halo or row
+// nodes do not fit, the directions themselves are exchanged at a third meeting.
 // Systems do not wait for one another.
 // What bounds the three launches per iteration that this replaces, for these
 // sizes, is latency: eight warps per SM in the product, and three launches
@@ -718,9 +722,12 @@ __global__ void k_keep_fixed(const double *__restrict__ x, const uint8_t *__rest
 // instruction) is what the phases between the meets cost, so no warp issues an
 // FP64 instruction that another one has issued: scalars are formed by one
 // thread, warps without work skip theirs.  Per iteration, with the launches
-// (after their own sums were packed) and here: 200x100 quad4 26.6 -> 14.2 us,
-// hex8 30^3 44 -> 27 us (the product's FP64 instructions alone take 13.8 us
-// of an interior chunk), tet10 heat, 90,945 nodes, 38 -> 20 us.
+// (after their own sums were packed), with the exchange of directions and with
+// the halo: 200x100 quad4 26.6, 13.1 and 11.9 us (5.1 of 26 thousand cycles
+// are the product, 4.0 of them FP64 instructions; most of the rest the meets
+// and the sums beside them); hex8 30^3 44, 26.3 and 25.1 us (the product's FP64
+// instructions alone take 13.8 us of an interior chunk); tet10 heat, 90,945
+// nodes, 38, 19.4 and 18.2 us.
 // Every sum is formed as k_seg_spmv, k_seg_update_fused and seg_total form it
 // (256 virtual threads per chunk, then the chunks by 256 threads), whatever
 // the CTA size, so a solve gives the same bits as the launches and as the
@@ -729,6 +736,7 @@ __global__ void k_keep_fixed(const double *__restrict__ x, const uint8_t *__rest
 // returns, every other one follows, and the host runs the launches instead
 // (x is written at the end only).
 constexpr unsigned long long RES_LIMIT_NS = 20000000000ull;   // 0: gives up at the first poll that fails
+constexpr unsigned RES_NO_ROOM = 2;   // *abort: a halo does not fit (1: a wait ran out)
 
 // Meeting points: every chunk pushes its word pair {bits of the partial,
 // iteration} (or its word, the iteration whose direction is written) to a
@@ -758,6 +766,12 @@ __device__ __forceinline__ ulonglong2 res_get(const ulonglong2 *p) {
                : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ ulonglong2 res_get_acquire(const ulonglong2 *p) {
+  ulonglong2 v;
+  asm volatile("{\n\t.reg .b128 q;\n\tld.acquire.gpu.global.b128 q, [%2];\n\tmov.b128 {%0, %1}, q;\n\t}"
+               : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+  return v;
+}
 __device__ __forceinline__ void res_fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 // Polls until done() (a relaxed load) is true; false: gave up.
 template <class F>
@@ -768,14 +782,15 @@ __device__ __forceinline__ bool res_poll(const ResSync &Y, F done) {
     if (Y.limit == 0) return false;
     if ((n & 1023u) == 1023u) {
       if (t0 == 0) t0 = res_now();
-      else if (res_now() - t0 > Y.limit || *(volatile const unsigned *)Y.abort) return false;
+      else if (res_now() - t0 > Y.limit || *(volatile const unsigned *)Y.abort == 1u) return false;
     }
   }
 }
-// The value of slot p of iteration it.
+// The value of slot p of iteration it; ACQUIRE: and what its writer released.
+template <bool ACQUIRE>
 __device__ __forceinline__ bool res_wait(const ulonglong2 *p, unsigned long long it, double &v, const ResSync &Y) {
   return res_poll(Y, [&]() {
-    const ulonglong2 q = res_get(p);
+    const ulonglong2 q = ACQUIRE ? res_get_acquire(p) : res_get(p);
     v = __longlong_as_double((long long)q.x);
     return q.y == it;
   });
@@ -808,9 +823,13 @@ __device__ __forceinline__ double res_last(const double *sw, int lane) {
 // The P columns of one node by u, the lane group's share (node_columns_at's
 // order).  u was written by other CTAs of this launch, so it is read through
 // plain loads (never the read-only path) after the acquire of the wait.
-template <int P>
+// LOCAL: u is in shared memory and adj holds places in it instead of nodes;
+// VALS: so are the columns.
+template <int P, bool LOCAL, bool VALS>
 __device__ __forceinline__ void res_columns(const double *__restrict__ col, const int32_t *adj, const double *u, int n,
                                             int g, double (&acc)[P]) {
+  auto val = [&](int32_t a, int c) { return LOCAL ? u[a + c] : __ldca(u + (int64_t)P * a + c); };
+  auto at = [&](int i) { return VALS ? col[i] : __ldg(col + i); };
 #pragma unroll
   for (int j = 0; j < P; ++j) acc[j] = 0.0;
   int k = g;
@@ -820,38 +839,41 @@ __device__ __forceinline__ void res_columns(const double *__restrict__ col, cons
     double v[P], v2[P];
 #pragma unroll
     for (int j = 0; j < P; ++j) {
-      v[j] = __ldg(col + (int64_t)j * n + k);
-      v2[j] = __ldg(col + (int64_t)j * n + k2);
+      v[j] = at(j * n + k);
+      v2[j] = at(j * n + k2);
     }
-    const double xa = __ldca(u + (int64_t)P * ra + k % P);
-    const double xb = __ldca(u + (int64_t)P * rb + k2 % P);
+    const double xa = val(ra, k % P);
+    const double xb = val(rb, k2 % P);
     ra = kn < n ? adj[kn / P] : 0;
     rb = kn + SPMV_G < n ? adj[(kn + SPMV_G) / P] : 0;
 #pragma unroll
     for (int j = 0; j < P; ++j) acc[j] = __fma_rn(v2[j], xb, __fma_rn(v[j], xa, acc[j]));
   }
   if (k < n) {
-    const double xa = __ldca(u + (int64_t)P * ra + k % P);
+    const double xa = val(ra, k % P);
 #pragma unroll
-    for (int j = 0; j < P; ++j) acc[j] = __fma_rn(__ldg(col + (int64_t)j * n + k), xa, acc[j]);
+    for (int j = 0; j < P; ++j) acc[j] = __fma_rn(at(j * n + k), xa, acc[j]);
   }
 }
 
 // Shared memory: u, c (then z), r of the chunk [3 CHUNK doubles] | values and
 // partial sums of two sums [2 x (256 + 8)] | scalars [4] | per position of the
 // node order: first row node (relative), row nodes, node and (from bit 16)
-// its fixed DoFs [CHUNK / P each, int] | row nodes of the chunk [adj_cap ints].
+// its fixed DoFs [CHUNK / P each, int] | row nodes of the chunk [adj_cap ints;
+// HALO: as many as there are, then the halo's nodes, its u and, if they fit,
+// the chunk's columns].
 constexpr int RES_SCALARS = 2 * (256 + 8) + 4;
 template <int P>
 constexpr size_t res_smem_fixed() {
   return sizeof(double) * (3 * CHUNK + RES_SCALARS) + sizeof(int) * 3 * (CHUNK / P);
 }
 
-template <int P, int T>
+template <int P, int T, bool HALO>
 __global__ void __launch_bounds__(T, 1024 / T)
 k_cg_resident(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ nptr, const int32_t *__restrict__ nadj,
               const uint8_t *__restrict__ fixed, const double *__restrict__ r0, const double *__restrict__ z0,
-              double *u, double *xw, const double *__restrict__ pinv, int mode, ResSync Y, int adj_cap) {
+              double *u, double *xw, const double *__restrict__ pinv, int mode, ResSync Y, int adj_cap, double *zg,
+              int smem_bytes) {
   extern __shared__ double rsm[];
   constexpr int NPT = (CHUNK + T - 1) / T, NODES = CHUNK / P;
   constexpr bool PV = NPT * P <= 4;   // preconditioner in registers
@@ -880,6 +902,9 @@ k_cg_resident(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ 
   const int64_t a0 = nptr[B0];
   const int na = (int)(nptr[B0 + nb] - a0);
   const bool adj_here = na <= adj_cap;
+  int nh = 0;                 // HALO: nodes of other chunks that this one's columns meet, in node order
+  int *sHid = nullptr;
+  double *sHu = nullptr, *sVal = nullptr;
   for (int p = threadIdx.x; p < nb; p += T) {
     const int k = S.perm ? (int)S.perm[B0 + p] : p;
     int fm = 0;
@@ -917,26 +942,114 @@ k_cg_resident(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ 
   }
   bool fail = false;
   __syncthreads();
+  if (HALO) {
+    // The halo: a bit per node of the system, set for the row nodes outside
+    // the chunk, and its rank among them; the row nodes become places of
+    // their u in shared memory.
+    const int64_t lo = S.cbeg[first] / P;
+    const int64_t hi = S.cend[first + nch - 1] / P;
+    const int words = (int)((hi - lo + 31) / 32);
+    sHid = sAdj + (adj_here ? (na + 1) & ~1 : 0);
+    const int64_t area = smem_bytes - (reinterpret_cast<char *>(sHid) - reinterpret_cast<char *>(rsm));
+    bool fits = adj_here && 8 * (int64_t)words <= area;
+    if (fits) {   // bits and ranks at the end of the area
+      unsigned *bits = reinterpret_cast<unsigned *>(reinterpret_cast<char *>(sHid) + area) - 2 * words;
+      int *rank = reinterpret_cast<int *>(bits + words);
+      for (int k = threadIdx.x; k < words; k += T) bits[k] = 0u;
+      __syncthreads();
+      bool outside = false;   // a row node of another system
+      for (int k = threadIdx.x; k < na; k += T) {
+        const int64_t v = sAdj[k];
+        if (v < lo || v >= hi) outside = true;
+        else if (v < B0 || v >= B0 + nb) atomicOr(bits + ((v - lo) >> 5), 1u << ((v - lo) & 31));
+      }
+      fits = !__syncthreads_or(outside);
+      const int per = (words + T - 1) / T, k0 = min((int)threadIdx.x * per, words), k1 = min(k0 + per, words);
+      int mine = 0;
+      for (int k = k0; k < k1; ++k) mine += __popc(bits[k]);
+      int incl = mine;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += t;
+      }
+      int *tot = reinterpret_cast<int *>(sv0);   // the warps' totals
+      if (lane == 31) tot[w] = incl;
+      __syncthreads();
+      int run = incl - mine;
+      for (int k = 0; k < T / 32; ++k) {
+        run += k < w ? tot[k] : 0;
+        nh += tot[k];
+      }
+      fits = fits && 8 * (int64_t)words + 4 * (int64_t)nh <= area && (4 + 8 * P) * (int64_t)nh + 8 <= area;
+      if (fits) {
+        for (int k = k0; k < k1; ++k) {
+          rank[k] = run;
+          for (unsigned m = bits[k]; m != 0u; m &= m - 1u) sHid[run++] = (int)(lo + 32 * (int64_t)k + __ffs(m) - 1);
+        }
+        sHu = reinterpret_cast<double *>(sHid + ((nh + 1) & ~1));
+        __syncthreads();
+        for (int k = threadIdx.x; k < na; k += T) {
+          const int64_t v = sAdj[k];
+          const int q = (int)((v - lo) >> 5);
+          sAdj[k] = v >= B0 && v < B0 + nb ? P * (int)(v - B0)
+                                           : (int)(sHu - sU) + P * (rank[q] + __popc(bits[q] & ((1u << ((v - lo) & 31)) - 1u)));
+        }
+        __syncthreads();   // the bits are done with
+        for (int k = threadIdx.x; k < P * nh; k += T) sHu[k] = u[(int64_t)P * sHid[k / P] + k % P];
+        const int64_t left = area - (reinterpret_cast<char *>(sHu + P * nh) - reinterpret_cast<char *>(sHid));
+        if (8 * (int64_t)(P * P) * na <= left) {
+          sVal = sHu + P * nh;
+          for (int k = threadIdx.x; k < P * P * na; k += T) sVal[k] = __ldg(nz + (int64_t)P * P * a0 + k);
+        }
+      }
+    }
+    // every chunk of the system must have room: it = 1 yes, 2 no
+    for (int k = threadIdx.x; k < nch; k += T)
+      asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(Y.dir + (first + k) * S.nchunks + ch),
+                   "l"(fits ? 1ull : 2ull) : "memory");
+    bool all = true;
+    for (int k = threadIdx.x; k < nch && !fail; k += T) {
+      unsigned long long v = 0;
+      fail = !res_poll(Y, [&]() {
+        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(Y.dir + ch * S.nchunks + first + k) : "memory");
+        return v != 0ull;
+      });
+      all = all && v == 1ull;
+    }
+    if (__syncthreads_or(fail || !all)) {
+      if (!fail && threadIdx.x == 0) atomicCAS(Y.abort, 0u, RES_NO_ROOM);
+      if (fail) atomicExch(Y.abort, 1u);
+      return;
+    }
+  }
   for (unsigned long long it = 1;; ++it) {
     // u = z + beta u
     const double beta = sq[1];
+    if (HALO) {   // the other chunks' directions as they form them, from their z
+      const double *zs = it == 1 ? z0 : zg;
+      for (int k = threadIdx.x; k < P * nh; k += T)
+        sHu[k] = __fma_rn(beta, sHu[k], __ldca(zs + (int64_t)P * sHid[k / P] + k % P));
+    }
 #pragma unroll
     for (int k = 0; k < NPT; ++k) {
       const int i = threadIdx.x + k * T;
       if (i < len) {
         d[k] = __fma_rn(beta, d[k], z[k]);
         sU[i] = d[k];
-        u[b + i] = d[k];
+        if (!HALO) u[b + i] = d[k];
       }
     }
     __syncthreads();
-    if ((int)threadIdx.x < nch) res_fence();   // release: this chunk's direction
-    for (int k = threadIdx.x; k < nch; k += T)
-      asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(Y.dir + (first + k) * S.nchunks + ch), "l"(it) : "memory");
-    for (int k = threadIdx.x; k < nch && !fail; k += T)
-      fail = !res_wait_dir(Y.dir + ch * S.nchunks + first + k, it, Y);
-    if ((int)threadIdx.x < nch) res_fence();   // acquire: the other chunks' directions
-    if (__syncthreads_or(fail)) break;
+    if (!HALO) {
+      if ((int)threadIdx.x < nch) res_fence();   // release: this chunk's direction
+      for (int k = threadIdx.x; k < nch; k += T)
+        asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(Y.dir + (first + k) * S.nchunks + ch), "l"(it) : "memory");
+      for (int k = threadIdx.x; k < nch && !fail; k += T)
+        fail = !res_wait_dir(Y.dir + ch * S.nchunks + first + k, it, Y);
+      if ((int)threadIdx.x < nch) res_fence();   // acquire: the other chunks' directions
+      if (__syncthreads_or(fail)) break;
+    }
     // c = A u, SPMV_G lanes per node
     for (int p0 = (w << 5) / SPMV_G; p0 < nb; p0 += T / SPMV_G) {   // the warp's first position
       const int p = p0 + lane / SPMV_G;
@@ -944,8 +1057,10 @@ k_cg_resident(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ 
       const int deg = valid ? sDeg[p] : 0, at = valid ? sFirst[p] : 0;
       double acc[P];
       const double *col = nz + (int64_t)P * P * (a0 + at);
-      if (adj_here) res_columns<P>(col, sAdj + at, u, deg * P, g, acc);
-      else res_columns<P>(col, nadj + a0 + at, u, deg * P, g, acc);
+      if (HALO && sVal) res_columns<P, true, true>(sVal + P * P * at, sAdj + at, sU, deg * P, g, acc);
+      else if (HALO) res_columns<P, true, false>(col, sAdj + at, sU, deg * P, g, acc);
+      else if (adj_here) res_columns<P, false, false>(col, sAdj + at, u, deg * P, g, acc);
+      else res_columns<P, false, false>(col, nadj + a0 + at, u, deg * P, g, acc);
 #pragma unroll
       for (int off = SPMV_G / 2; off > 0; off >>= 1)
 #pragma unroll
@@ -981,7 +1096,7 @@ k_cg_resident(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ 
       double s = 0.0;
       for (int k = threadIdx.x; k < nch && !fail; k += 256) {
         double v = 0.0;
-        fail = !res_wait(Y.uc + ch * S.nchunks + first + k, it, v, Y);
+        fail = !res_wait<false>(Y.uc + ch * S.nchunks + first + k, it, v, Y);
         s = __dadd_rn(s, v);
       }
       sv0[threadIdx.x] = s;
@@ -1029,9 +1144,15 @@ k_cg_resident(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ 
         }
         z[k] = fx[k] ? 0.0 : zi;
         sC[i] = z[k];
+        // every chunk has read the z of the iteration before (its u.c has come)
+        if (HALO) zg[b + i] = z[k];
       }
     }
     __syncthreads();
+    // the last two warps push the two sums; they release this chunk's z, which
+    // every thread has stored, while the others form the sums
+    const int pw = w - (T / 32 - 2);
+    if (HALO && pw >= 0) res_fence();
     // the chunk's r.r (threads 0..255) and z.r (256..511, or the same threads)
     if (threadIdx.x < 512) {
       const int t = threadIdx.x & 255;
@@ -1048,9 +1169,9 @@ k_cg_resident(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ 
     __syncthreads();
     if (w < 8) res_fold(w < 4 ? sv0 : sv1, w < 4 ? sw0 : sw1, w, lane);
     __syncthreads();
-    if (w < 2) {
-      const double s = __shfl_sync(0xffffffffu, res_last(w == 0 ? sw0 : sw1, lane), 0);
-      for (int k = lane; k < nch; k += 32) res_put((w == 0 ? Y.rr : Y.zr) + (first + k) * S.nchunks + ch, s, it);
+    if (pw >= 0) {
+      const double s = __shfl_sync(0xffffffffu, res_last(pw == 0 ? sw0 : sw1, lane), 0);
+      for (int k = lane; k < nch; k += 32) res_put((pw == 0 ? Y.rr : Y.zr) + (first + k) * S.nchunks + ch, s, it);
     }
     // the system's r.r and z.r
     if (threadIdx.x < 512) {
@@ -1059,10 +1180,11 @@ k_cg_resident(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ 
       double s = 0.0, s2 = 0.0;
       for (int k = t; k < nch && !fail; k += 256) {
         double v = 0.0;
-        fail = !res_wait((second ? Y.zr : Y.rr) + ch * S.nchunks + first + k, it, v, Y);
+        const ulonglong2 *slot = (second ? Y.zr : Y.rr) + ch * S.nchunks + first + k;
+        fail = HALO && second ? !res_wait<true>(slot, it, v, Y) : !res_wait<false>(slot, it, v, Y);
         s = __dadd_rn(s, v);
         if (T == 256) {
-          fail = fail || !res_wait(Y.zr + ch * S.nchunks + first + k, it, v, Y);
+          fail = fail || !res_wait<HALO>(Y.zr + ch * S.nchunks + first + k, it, v, Y);
           s2 = __dadd_rn(s2, v);
         }
       }
@@ -1491,19 +1613,19 @@ __global__ void k_count_active(Seg S) {
   if (threadIdx.x == 0) *S.active = n;
 }
 
-template <int P, int T>
+template <int P, int T, bool HALO>
 int launch_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const double *r, const double *z, double *u,
-                    double *xw, const double *pinv, const uint8_t *fixed, int precond, unsigned long long *sync,
+                    double *c, double *xw, const double *pinv, const uint8_t *fixed, int precond, unsigned long long *sync,
                     bool *done) {
   const llf_pattern *pat = m->pat;
   const int64_t nch = S.nchunks;
   cudaStream_t s = ctx->stream;
-  auto fn = k_cg_resident<P, T>;
+  auto fn = k_cg_resident<P, T, HALO>;
   // row nodes in shared memory as far as the CTA's share of the SM goes
   const size_t fixed_b = res_smem_fixed<P>(), room = (size_t)(216 * 1024) / (1024 / T);
   const int adj_cap = (int)std::min<int64_t>((int64_t)(CHUNK / P) * std::max(pat->max_deg, 1),
                                              (int64_t)((room - fixed_b) / sizeof(int)));
-  const size_t smem = fixed_b + sizeof(int) * (size_t)adj_cap;
+  const size_t smem = HALO ? room : fixed_b + sizeof(int) * (size_t)adj_cap;
   LLF_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
   LLF_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, T, smem));
@@ -1528,7 +1650,8 @@ int launch_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const doubl
   {
     KernelScope k(ctx, "k_cg_resident");
     if (cudaLaunchKernelEx(&cfg, fn, S, (const double *)m->d_nz, (const int64_t *)pat->d_nptr,
-                           (const int32_t *)pat->d_nadj, fixed, r, z, u, xw, pinv, precond, Y, adj_cap) != cudaSuccess) {
+                           (const int32_t *)pat->d_nadj, fixed, r, z, u, xw, pinv, precond, Y, adj_cap, c, (int)smem) !=
+        cudaSuccess) {
       cudaGetLastError();   // not all CTAs can be resident here (a partitioned GPU)
       return LLF_OK;
     }
@@ -1536,6 +1659,8 @@ int launch_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const doubl
   unsigned aborted = 1;
   LLF_CUDA_TRY(ctx, cudaMemcpyAsync(&aborted, Y.abort, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   LLF_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+  if (HALO && aborted == RES_NO_ROOM)
+    return launch_resident<P, T, false>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, done);
   *done = aborted == 0;
   if (*done) {
     LLF_CUDA_TRY(ctx, cudaMemsetAsync(S.active, 0, sizeof(int), s));
@@ -1553,7 +1678,7 @@ int launch_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const doubl
 // *done = false: the caller runs the launches.
 template <int P>
 int run_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const double *r, const double *z, double *u,
-                 double *xw, const double *pinv, const uint8_t *fixed, int precond, unsigned long long *sync,
+                 double *c, double *xw, const double *pinv, const uint8_t *fixed, int precond, unsigned long long *sync,
                  bool *done) {
   *done = false;
   const int64_t nch = S.nchunks;
@@ -1562,10 +1687,10 @@ int run_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const double *
   std::unique_lock<std::mutex> lock(g_res_mutex[ctx->device], std::try_to_lock);
   if (!lock.owns_lock()) return LLF_OK;
   if (nch <= ctx->num_sms)
-    return launch_resident<P, 1024>(ctx, m, S, r, z, u, xw, pinv, fixed, precond, sync, done);
+    return launch_resident<P, 1024, true>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, done);
   if (nch <= 2 * (int64_t)ctx->num_sms)
-    return launch_resident<P, 512>(ctx, m, S, r, z, u, xw, pinv, fixed, precond, sync, done);
-  return launch_resident<P, 256>(ctx, m, S, r, z, u, xw, pinv, fixed, precond, sync, done);
+    return launch_resident<P, 512, true>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, done);
+  return launch_resident<P, 256, true>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, done);
 }
 
 // Buffers, chunking and preconditioner of the segmented PCG for one matrix
@@ -1745,7 +1870,7 @@ int pcg_core(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double *d_x, 
 
   if (sync && precond != LLF_PRECOND_IC0) {
     bool done = false;
-    const int rc = run_resident<P>(ctx, m, S, r, z, u, xw, pinv, d_fixed, precond, sync, &done);
+    const int rc = run_resident<P>(ctx, m, S, r, z, u, c, xw, pinv, d_fixed, precond, sync, &done);
     if (rc != LLF_OK) return rc;
     if (done) {
       { KernelScope k(ctx, "k_cg_merge"); k_cg_merge<<<gv, CG_THREADS, 0, s>>>(xw, d_fixed, d_x, n); }

@@ -56,6 +56,27 @@ def test_resident_equals_launches(llf, case, precond):
     assert np.array_equal(got[0], want[0]) and got[1:] == want[1:]
 
 
+@pytest.mark.parametrize("n,order", [(12, 1), (22, 2)], ids=["fits", "no-room"])
+def test_resident_with_nodes_in_random_order(llf, n, order):
+    """A chunk whose columns meet nodes all over the system: its halo is most
+    of it, or does not fit beside the chunk."""
+    m = llf.structured_box_mesh(n=n, order=order)
+    new = np.random.default_rng(n).permutation(m.non)
+    xyz = np.empty_like(m.xyz)
+    xyz[new] = m.xyz
+    conn = new[m.conn - 1] + 1
+    body = llf.Group("body", 3, np.arange(1, m.non + 1), m.family, m.order, conn, np.arange(m.nel))
+    sh = llf.Mesh(3, m.family, m.order, xyz, conn, {"body": body})
+    P = llf.Problem([llf.Material("body", k=2.0)], type="Solid" if order == 1 else "HeatConduction", mesh=sh)
+    K = llf.stiffnessMatrix(P) if order == 1 else llf.heatConductionMatrix(P)
+    nd = P.pdim * m.non
+    fixed = np.repeat(xyz[:, 0] < 1e-9, P.pdim).astype(np.uint8)
+    b, x0 = np.random.default_rng(2).standard_normal(nd), np.zeros(nd)
+    got = K.dm.pcg(b, x0, fixed, precond=1, reltol=1e-9, maxiter=50, raise_on_fail=False)
+    want = _noalloc(llf, K, b, x0, fixed, 1, 1e-9, 50)
+    assert np.array_equal(got[0], want[0]) and got[1:] == want[1:]
+
+
 def test_resident_four_per_sm_and_batches(llf):
     """A system with more than two chunks per SM alone (four CTAs per SM), a
     batch of uneven systems in one launch, and a batch with more chunks than
