@@ -76,8 +76,8 @@ __host__ __device__ constexpr int plane_stride(int md, int P) { return (md * P) 
 // T = double (FP64 form) or float (precision form); FP64 sums in element
 // order in both.  BLOCKVAL: P x P blocks, entry (i,j) at i*P+j; otherwise one
 // scalar per node pair, placed on the component diagonal.  NCH: most rounds
-// of G lanes that an element column takes, whose values are then prefetched
-// one element ahead; 0 for longer ones.
+// of G lanes that an element column takes, whose values are prefetched one
+// element ahead (longer ones: k_colgather_wide).
 // first_marked: bit 15 of a map entry marks the first block of its row
 // position; that block is stored and later ones are added, one FP64 addition
 // per contribution after the first.  Otherwise, and with init (values to
@@ -149,7 +149,7 @@ __global__ void k_colgather(const int64_t *__restrict__ nptr, const int64_t *__r
         for (int r = gl; r < P * deg; r += G) accb[j * ps + r] = init ? src[j * P * deg + r] : NEG_ZERO;
       __syncwarp();
     }
-    if constexpr (NCH > 0) {
+    {
       // VPN == 1: a lane's values have row nodes of their own; otherwise lane
       // a of the group holds the position of row node a (npe <= G)
       constexpr int NT = VPN == 1 ? NCH : 1;
@@ -189,30 +189,6 @@ __global__ void k_colgather(const int64_t *__restrict__ nptr, const int64_t *__r
         for (int m = 0; m < NCH; ++m) cur[m] = nxt[m];
 #pragma unroll
         for (int m = 0; m < NT; ++m) tc[m] = tn[m];
-      }
-    } else {
-      for (int k = 0; k < nb; ++k) {
-        const int2 el = n2e[s + k];
-        const W *col = reinterpret_cast<const W *>(Kf) + ((size_t)el.x * npe + el.y) * cs;
-        const uint16_t *pk = pos + (s + k) * npe;
-        constexpr int U = 8;
-        for (int f0 = gl; f0 < NV; f0 += G * U) {
-          W v[U];
-          unsigned raw[U];
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const int f = f0 + u * G;
-            raw[u] = 0xffffu;
-            if (f < NV) {
-              raw[u] = pk[f / VPN];
-              v[u] = col[value_at(f)];
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < U; ++u)
-            if (raw[u] != 0xffffu) put(f0 + u * G, raw[u], v[u]);
-        }
-        __syncwarp();
       }
     }
     // write-out, the warp over each of its column nodes: 64 entries at a time
@@ -279,6 +255,142 @@ __global__ void k_colgather(const int64_t *__restrict__ nptr, const int64_t *__r
       }
     }
     __syncwarp();
+  }
+}
+
+// The same gather with a CTA of NT threads per column node, for element
+// columns longer than a warp takes in the rounds above: the accumulator of
+// such a node (hex125: 18 to 53 KB) leaves room for few nodes on an SM, and a
+// warp each left it with four warps.  The values of an element column (at most
+// NT R) go over the CTA's threads, R each, loaded an element ahead, with a
+// barrier between elements; a plane is written out by the
+// warps w, w + P, ..., a part each.
+// Bound by latency and the barriers.  Both degree classes, against a warp
+// each: hex125 576 elements from FP32 matrices 0.98 -> 0.37 ms, 216 from FP64
+// ones 0.53 -> 0.29; tet35, 3,072 turned 0.46 -> 0.30; hex64, 1,000 turned 0.305
+// -> 0.301 and, from FP32, 0.34 -> 0.28 ms.  hex27 (243 values) stays with a
+// warp each: 1.88 against 2.56 ms for 64,000 elements.
+template <int P, bool BLOCKVAL, class T, int NT, int R>
+__global__ void __launch_bounds__(NT, NT == 192 ? 5 : 0)
+k_colgather_wide(const int64_t *__restrict__ nptr, const int64_t *__restrict__ n2e_ptr,
+                 const int2 *__restrict__ n2e, const uint16_t *__restrict__ pos, const T *__restrict__ Kf, int64_t cs,
+                 int npe, int64_t non, int max_deg, const double *__restrict__ init, double *__restrict__ nz,
+                 int64_t *__restrict__ cnt, const int32_t *__restrict__ list, const int32_t *__restrict__ nadj,
+                 StoredSpec spec, int first_marked) {
+  extern __shared__ double cg_smem[];
+  constexpr int VPN = BLOCKVAL ? P * P : P;
+  constexpr int BSTR = kf_bstride(P, BLOCKVAL, (int)sizeof(T));
+  constexpr int PARTS = NT / 32 / P;   // warps per plane of the write-out
+  static_assert(PARTS >= 1, "a warp per plane");
+  using W = typename GatherWord<T>::type;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ps = plane_stride(max_deg, P), NV = npe * VPN;
+  double *acc = cg_smem;
+  unsigned long long *accb = reinterpret_cast<unsigned long long *>(acc);
+  const bool store_first = first_marked && init == nullptr;
+  const unsigned tmask = first_marked ? 0x7fffu : 0xffffu;
+  auto put = [&](int f, unsigned raw, W v) {   // k_colgather's
+    const int t = (int)(raw & tmask), r = f % VPN;
+    const int at = BLOCKVAL ? (r % P) * ps + t * P + r / P : r * ps + t * P + r;
+    if (store_first && (raw & 0x8000u)) {
+      accb[at] = value_bits(v);
+      if (!BLOCKVAL)
+#pragma unroll
+        for (int j = 1; j < P; ++j) accb[((r + j) % P) * ps + t * P + r] = 0ull;
+    } else {
+      acc[at] = __dadd_rn(acc[at], widen(v));
+      if (!BLOCKVAL && P > 1 && !store_first)
+#pragma unroll
+        for (int j = 1; j < P; ++j) {
+          double *o = acc + ((r + j) % P) * ps + t * P + r;
+          *o = __dadd_rn(*o, 0.0);
+        }
+    }
+  };
+  for (int w = blockIdx.x; w < (int)non; w += (int)gridDim.x) {
+    const int B = list ? __ldg(list + w) : w;
+    const int64_t c0 = nptr[B], s = n2e_ptr[B];
+    const int deg = (int)(nptr[B + 1] - c0), nb = (int)(n2e_ptr[B + 1] - s), len = P * deg;
+    if (!store_first) {
+      const unsigned long long *src = reinterpret_cast<const unsigned long long *>(init) + (size_t)P * P * c0;
+      for (int j = 0; j < P; ++j)
+        for (int r = tid; r < len; r += NT) accb[j * ps + r] = init ? src[j * len + r] : NEG_ZERO;
+      __syncthreads();
+    }
+    auto load = [&](int2 el, int k, W *v, unsigned *raw) {
+      const W *col = reinterpret_cast<const W *>(Kf) + ((size_t)el.x * npe + el.y) * cs;
+      const uint16_t *pk = pos + (s + k) * npe;
+#pragma unroll
+      for (int m = 0; m < R; ++m) {
+        const int f = tid + m * NT;
+        raw[m] = 0xffffu;
+        if (f < NV) {
+          raw[m] = pk[f / VPN];
+          v[m] = col[BLOCKVAL ? (f / VPN) * BSTR + f % VPN : f / VPN];
+        }
+      }
+    };
+    W cur[R], nxt[R];
+    unsigned rc[R], rn[R];
+    int2 en = nb > 1 ? n2e[s + 1] : make_int2(0, 0);   // the next element of the list
+    if (nb > 0) load(n2e[s], 0, cur, rc);
+    for (int k = 0; k < nb; ++k) {   // elements of B, ascending
+      const int2 e2 = k + 2 < nb ? n2e[s + k + 2] : make_int2(0, 0);
+      if (k + 1 < nb) load(en, k + 1, nxt, rn);
+#pragma unroll
+      for (int m = 0; m < R; ++m)
+        if (rc[m] != 0xffffu) put(tid + m * NT, rc[m], cur[m]);
+#pragma unroll
+      for (int m = 0; m < R; ++m) {
+        cur[m] = nxt[m];
+        rc[m] = rn[m];
+      }
+      en = e2;
+      __syncthreads();   // an entry's sum goes by elements
+    }
+    const int j = warp % P, part = warp / P;
+    if (part < PARTS) {
+      const unsigned long long *ab = accb + (size_t)j * ps;
+      const unsigned below = (1u << lane) - 1u;
+      const int blocks = (len + 63) / 64, i0 = blocks * part / PARTS * 64, i1 = min(blocks * (part + 1) / PARTS * 64, len);
+      int run = 0;   // non-zeros of the plane before the current 64 entries
+      for (int i = lane; i < i0; i += 32) run += (ab[i] << 1) != 0ull;   // every value but +-0
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) run += __shfl_xor_sync(0xffffffffu, run, off);
+      const int64_t c = (int64_t)P * B + j;
+      const int64_t o = spec.ptr0 ? spec.ptr0[c] : 0, oend = spec.ptr0 ? spec.ptr0[c + 1] : 0;
+      unsigned long long *out = reinterpret_cast<unsigned long long *>(nz) + (size_t)P * P * c0 + (size_t)j * len;
+      for (int i = i0; i < i1; i += 64) {
+        const int ia = i + lane, ib = ia + 32;
+        const unsigned long long va = ia < len ? ab[ia] : 0ull, vb = ib < len ? ab[ib] : 0ull;
+        const bool ka = (va << 1) != 0ull, kb = (vb << 1) != 0ull;
+        const unsigned ba = __ballot_sync(0xffffffffu, ka), bb = __ballot_sync(0xffffffffu, kb);
+        if (spec.ptr0) {
+          const int64_t ta = o + run + __popc(ba & below), tb = o + run + __popc(ba) + __popc(bb & below);
+          if (ka && ta < oend) {
+            spec.rowval_s[ta] = (int64_t)P * nadj[c0 + ia / P] + ia % P + 1;
+            reinterpret_cast<unsigned long long *>(spec.nzval_s)[ta] = va;
+          }
+          if (kb && tb < oend) {
+            spec.rowval_s[tb] = (int64_t)P * nadj[c0 + ib / P] + ib % P + 1;
+            reinterpret_cast<unsigned long long *>(spec.nzval_s)[tb] = vb;
+          }
+          if (lane == 0) spec.keep[keep_pos((int64_t)P * P * c0 + (int64_t)j * len, c) + (i >> 6)] = make_uint2(ba, bb);
+        } else {
+          if (ia < len) out[ia] = va;
+          if (ib < len) out[ib] = vb;
+        }
+        run += __popc(ba) + __popc(bb);
+      }
+      if (part == PARTS - 1 && lane == 0) {   // run: the plane's count
+        if (spec.ptr0) {
+          if ((int64_t)run != oend - o) atomicOr(spec.mismatch, 1u);
+        } else if (cnt) {
+          cnt[c] = run;
+        }
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -353,15 +465,32 @@ __global__ void k_mark_first(const int64_t *__restrict__ nptr, const int64_t *__
   }
 }
 
+// launch(md, list, b0, count): the column nodes of the list, or [b0, b0 +
+// count), with accumulators of md row positions; the pattern's two degree
+// classes one after the other when all its nodes are asked for.
+template <class F>
+int gather_classes(llf_ctx *ctx, llf_pattern *pat, int64_t B0, int64_t nB, F launch) {
+  const int md = pat->max_deg > 0 ? pat->max_deg : 1;
+  if (B0 == 0 && nB == pat->mesh->non) {
+    int rc = gather_split(ctx, pat);
+    if (rc != LLF_OK) return rc;
+    if (pat->d_gather_nodes) {
+      rc = launch(pat->gather_md_low, pat->d_gather_nodes, (int64_t)0, pat->gather_n_low);
+      if (rc == LLF_OK)
+        rc = launch(md, pat->d_gather_nodes + pat->gather_n_low, (int64_t)0, pat->mesh->non - pat->gather_n_low);
+      return rc;
+    }
+  }
+  return launch(md, (const int32_t *)nullptr, B0, nB);
+}
+
 template <int P, bool BV, class T, int G, int NCH>
 int launch_colgather(llf_ctx *ctx, llf_pattern *pat, const int64_t *n2e_ptr, const int2 *n2e, const uint16_t *pos,
                      int npe, const T *Kf, int64_t cs, const double *init, double *nz, int64_t *cnt, int64_t B0,
                      int64_t nB, const StoredSpec &sp, bool first_marked) {
   auto fn = k_colgather<P, BV, T, G, NCH>;
   constexpr int NPW = 32 / G;
-  // one launch over `count` column nodes (the list's, or [B0, B0 + count))
-  // with accumulators of md row positions
-  auto launch = [&](int md, const int32_t *list, int64_t b0, int64_t count) -> int {
+  return gather_classes(ctx, pat, B0, nB, [&](int md, const int32_t *list, int64_t b0, int64_t count) -> int {
     if (count <= 0) return LLF_OK;
     const size_t per_warp = (size_t)NPW * P * plane_stride(md, P) * sizeof(double);
     int wpb = (int)std::min<size_t>(pat->tune.gather_wpb > 0 ? pat->tune.gather_wpb : 4, (200 * 1024) / per_warp);
@@ -381,19 +510,31 @@ int launch_colgather(llf_ctx *ctx, llf_pattern *pat, const int64_t *n2e_ptr, con
                                                         pat->d_nadj, sp, first_marked ? 1 : 0);
     LLF_CUDA_TRY(ctx, cudaGetLastError());
     return LLF_OK;
-  };
-  const int md = pat->max_deg > 0 ? pat->max_deg : 1;
-  if (B0 == 0 && nB == pat->mesh->non) {
-    int rc = gather_split(ctx, pat);
-    if (rc != LLF_OK) return rc;
-    if (pat->d_gather_nodes) {
-      rc = launch(pat->gather_md_low, pat->d_gather_nodes, 0, pat->gather_n_low);
-      if (rc == LLF_OK)
-        rc = launch(md, pat->d_gather_nodes + pat->gather_n_low, 0, pat->mesh->non - pat->gather_n_low);
-      return rc;
-    }
-  }
-  return launch(md, nullptr, B0, nB);
+  });
+}
+
+template <int P, bool BV, class T, int NT, int R>
+int launch_wide(llf_ctx *ctx, llf_pattern *pat, const int64_t *n2e_ptr, const int2 *n2e, const uint16_t *pos, int npe,
+                const T *Kf, int64_t cs, const double *init, double *nz, int64_t *cnt, int64_t B0, int64_t nB,
+                const StoredSpec &sp, bool first_marked) {
+  auto fn = k_colgather_wide<P, BV, T, NT, R>;
+  return gather_classes(ctx, pat, B0, nB, [&](int md, const int32_t *list, int64_t b0, int64_t count) -> int {
+    if (count <= 0) return LLF_OK;
+    const size_t smem = (size_t)P * plane_stride(md, P) * sizeof(double);
+    if (smem > 200 * 1024)
+      return llf_fail(ctx, LLF_ERR_LIMIT, "a column node has too many neighbours for the gather buffer");
+    if (smem > 48 * 1024)
+      LLF_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 1;
+    LLF_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, NT, smem));
+    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->num_sms * std::max(per_sm, 1), count));
+    KernelScope ks(ctx, "k_colgather_wide");
+    fn<<<(unsigned)grid, NT, smem, ctx->stream>>>(pat->d_nptr + b0, n2e_ptr + b0, n2e, pos, Kf, cs, npe, count, md, init,
+                                                  nz, cnt ? cnt + b0 * P : nullptr, list, pat->d_nadj, sp,
+                                                  first_marked ? 1 : 0);
+    LLF_CUDA_TRY(ctx, cudaGetLastError());
+    return LLF_OK;
+  });
 }
 
 // Gather over explicit node -> element lists and element-to-column map (the
@@ -437,8 +578,16 @@ int run_colgather(llf_ctx *ctx, llf_pattern *pat, const int64_t *n2e_ptr, const 
   if (rounds == 1) LLF_GATHER(32, 1);
   if (rounds <= 3 && lanes) LLF_GATHER(32, 3);
   if (rounds <= 8 && lanes) LLF_GATHER(32, 8);
-  LLF_GATHER(32, 0);
 #undef LLF_GATHER
+#define LLF_WIDE(NT, R) \
+  return launch_wide<P, BV, T, NT, R>(ctx, pat, n2e_ptr, n2e, pos, npe, Kf, cs, init, nz, cnt, B0, nB, sp, first_marked)
+  // longer: a CTA per column node, the rounds that use its threads and its
+  // registers best (measured with 64 to 576 threads)
+  if (nv <= 160 * 2) LLF_WIDE(160, 2);
+  if (nv <= 192 * 3) LLF_WIDE(192, 3);
+  if (nv <= 288 * 4) LLF_WIDE(288, 4);
+  return llf_fail(ctx, LLF_ERR_LIMIT, "an element has too many nodes for the gather");
+#undef LLF_WIDE
 }
 
 template <class T>

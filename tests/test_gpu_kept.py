@@ -14,7 +14,8 @@ CASES = {
     "hex64": ("box", (2, 2, 1), 3, False, "K"), "tet4": ("box", (1, 1, 1), 1, True, "K"),
     "tet10": ("box", (3, 2, 3), 2, True, "K"), "quad4": ("rect", (7, 5), 1, False, "K"),
     "tri6": ("rect", (3, 4), 2, True, "K"), "hex8-heat": ("box", (5, 4, 3), 1, False, "heat"),
-    "hex125-heat": ("box", (2, 1, 2), 4, False, "heat"), "hex27-mass": ("box", (3, 2, 2), 2, False, "mass"),
+    "hex125": ("box", (2, 1, 1), 4, False, "K"), "tet35": ("box", (2, 1, 1), 4, True, "K"),
+    "hex125-mass": ("box", (1, 2, 1), 4, False, "mass"), "hex125-heat": ("box", (2, 1, 2), 4, False, "heat"), "hex27-mass": ("box", (3, 2, 2), 2, False, "mass"),
 }
 
 

@@ -58,7 +58,9 @@ def _cauchy_green(A, m):
 ASM_CASES = {"hex8": ((11, 10, 11), 1, False), "tet4": ((8, 7, 7), 1, True), "tet10": ((5, 4, 5), 2, True),
              "quad4": ((49, 47), 1, False), "tri3": ((61, 59), 1, True), "tri6": ((29, 29), 2, True),
              "quad9": ((28, 28), 2, False), "hex27": ((7, 7, 7), 2, False), "tet20": ((4, 4, 5), 3, True),
-             "quad25": ((18, 18), 4, False)}
+             "quad25": ((18, 18), 4, False),
+             # beyond the packed kernel, with a CTA per column node in the gather
+             "hex64": ((3, 2, 2), 3, False), "hex125": ((2, 1, 2), 4, False), "tet35": ((2, 2, 1), 4, True)}
 
 
 def _shaped(llf, cells, order, simplex, shape):
