@@ -820,6 +820,7 @@ __device__ __forceinline__ double res_last(const double *sw, int lane) {
   return t;
 }
 
+constexpr int RES_STEPS = 4;
 // The P columns of one node by u, the lane group's share (node_columns_at's
 // order).  u was written by other CTAs of this launch, so it is read through
 // plain loads (never the read-only path) after the acquire of the wait.
@@ -828,11 +829,34 @@ __device__ __forceinline__ double res_last(const double *sw, int lane) {
 template <int P, bool LOCAL, bool VALS>
 __device__ __forceinline__ void res_columns(const double *__restrict__ col, const int32_t *adj, const double *u, int n,
                                             int g, double (&acc)[P]) {
+  constexpr int U = LOCAL && !VALS ? RES_STEPS : 2;   // positions whose values a lane loads at once
   auto val = [&](int32_t a, int c) { return LOCAL ? u[a + c] : __ldca(u + (int64_t)P * a + c); };
   auto at = [&](int i) { return VALS ? col[i] : __ldg(col + i); };
 #pragma unroll
   for (int j = 0; j < P; ++j) acc[j] = 0.0;
   int k = g;
+  if (LOCAL) {
+    for (; k + (U - 1) * SPMV_G < n; k += U * SPMV_G) {
+      double v[U][P];
+#pragma unroll
+      for (int q = 0; q < U; ++q)
+#pragma unroll
+        for (int j = 0; j < P; ++j) v[q][j] = at(j * n + k + q * SPMV_G);
+#pragma unroll
+      for (int q = 0; q < U; ++q) {
+        const int kq = k + q * SPMV_G;
+        const double xa = val(adj[kq / P], kq % P);
+#pragma unroll
+        for (int j = 0; j < P; ++j) acc[j] = __fma_rn(v[q][j], xa, acc[j]);
+      }
+    }
+    for (; k < n; k += SPMV_G) {
+      const double xa = val(adj[k / P], k % P);
+#pragma unroll
+      for (int j = 0; j < P; ++j) acc[j] = __fma_rn(at(j * n + k), xa, acc[j]);
+    }
+    return;
+  }
   int32_t ra = k < n ? adj[k / P] : 0, rb = k + SPMV_G < n ? adj[(k + SPMV_G) / P] : 0;
   for (; k + SPMV_G < n; k += 2 * SPMV_G) {
     const int k2 = k + SPMV_G, kn = k + 2 * SPMV_G;
@@ -875,6 +899,7 @@ k_cg_resident(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ 
               double *u, double *xw, const double *__restrict__ pinv, int mode, ResSync Y, int adj_cap, double *zg,
               int smem_bytes) {
   extern __shared__ double rsm[];
+  static_assert(T >= 512, "two sums side by side");
   constexpr int NPT = (CHUNK + T - 1) / T, NODES = CHUNK / P;
   constexpr bool PV = NPT * P <= 4;   // preconditioner in registers
   double *sU = rsm, *sC = sU + CHUNK, *sR = sC + CHUNK;
@@ -1153,18 +1178,13 @@ k_cg_resident(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ 
     // every thread has stored, while the others form the sums
     const int pw = w - (T / 32 - 2);
     if (HALO && pw >= 0) res_fence();
-    // the chunk's r.r (threads 0..255) and z.r (256..511, or the same threads)
+    // the chunk's r.r (threads 0..255) and z.r (256..511)
+    const bool second = threadIdx.x >= 256;
     if (threadIdx.x < 512) {
-      const int t = threadIdx.x & 255;
+      const double *a = second ? sC : sR;
       double s = 0.0;
-      const double *a = T > 256 && threadIdx.x >= 256 ? sC : sR;
-      for (int i = t; i < len; i += 256) s = __fma_rn(a[i], sR[i], s);
-      (T > 256 && threadIdx.x >= 256 ? sv1 : sv0)[t] = s;
-      if (T == 256) {
-        s = 0.0;
-        for (int i = t; i < len; i += 256) s = __fma_rn(sC[i], sR[i], s);
-        sv1[t] = s;
-      }
+      for (int i = threadIdx.x & 255; i < len; i += 256) s = __fma_rn(a[i], sR[i], s);
+      (second ? sv1 : sv0)[threadIdx.x & 255] = s;
     }
     __syncthreads();
     if (w < 8) res_fold(w < 4 ? sv0 : sv1, w < 4 ? sw0 : sw1, w, lane);
@@ -1175,21 +1195,14 @@ k_cg_resident(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ 
     }
     // the system's r.r and z.r
     if (threadIdx.x < 512) {
-      const int t = threadIdx.x & 255;
-      const bool second = T > 256 && threadIdx.x >= 256;
-      double s = 0.0, s2 = 0.0;
-      for (int k = t; k < nch && !fail; k += 256) {
+      double s = 0.0;
+      for (int k = threadIdx.x & 255; k < nch && !fail; k += 256) {
         double v = 0.0;
         const ulonglong2 *slot = (second ? Y.zr : Y.rr) + ch * S.nchunks + first + k;
         fail = HALO && second ? !res_wait<true>(slot, it, v, Y) : !res_wait<false>(slot, it, v, Y);
         s = __dadd_rn(s, v);
-        if (T == 256) {
-          fail = fail || !res_wait<HALO>(Y.zr + ch * S.nchunks + first + k, it, v, Y);
-          s2 = __dadd_rn(s2, v);
-        }
       }
-      (second ? sv1 : sv0)[t] = s;
-      if (T == 256) sv1[t] = s2;
+      (second ? sv1 : sv0)[threadIdx.x & 255] = s;
     }
     if (__syncthreads_or(fail)) break;
     if (w < 8) res_fold(w < 4 ? sv0 : sv1, w < 4 ? sw0 : sw1, w, lane);
@@ -1592,7 +1605,7 @@ int pcg_mixed_core(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double 
                    double *part2, double *part3, int precond, double reltol, int64_t maxiter, bool use_graph,
                    SegState *hst, const IcApply &ic);
 
-constexpr int64_t RES_MAX_CHUNKS = 1024;
+constexpr int64_t RES_MAX_CHUNKS = 512;
 // Words of the resident CG's meeting points for nch chunks (zeroed before
 // every launch): three word pairs and one word per pair of chunks, and the
 // abort flag; none for a solve that has too many chunks.
@@ -1672,9 +1685,17 @@ int launch_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const doubl
   return LLF_OK;
 }
 
-// The resident CG when every chunk gets a CTA at once: the largest CTA whose
-// chunks still fit, one per SM (the product's loads then have all the warps
-// an SM holds, whatever the number of chunks), else two or four per SM.
+// The resident CG when every chunk gets a CTA at once: one CTA of 1024 threads
+// per SM (the product's loads then have all the warps an SM holds, whatever
+// the number of chunks), or two of 512 while the values take no more than five
+// eighths of the L2, of which each die holds half and the vectors and row nodes
+// their part.  Per solve, launches and here: one per SM 1.3 to 2.1 times faster
+// (hex27 11^3 20.2 and 14.0 ms, tet10 heat with 103,823 nodes 19.1 and 10.0
+// ms); two per SM, values of 20 to 80 MB 0.95 to 1.9 times (tri3 heat with
+// 160,801 nodes 54 and 38 ms, quad16 100x100 349 and 187), of 86 to 111 MB 0.8
+// to 1.3 times and not twice the same, of 137 to 320 MB 0.6 to 0.8 times (hex8
+// 41^3 49 and 66 ms): those stream from HBM, and the launches keep more loads
+// under way.  Four CTAs of 256 threads were 0.8 to 1.1 times as fast.
 // *done = false: the caller runs the launches.
 template <int P>
 int run_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const double *r, const double *z, double *u,
@@ -1682,15 +1703,18 @@ int run_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const double *
                  bool *done) {
   *done = false;
   const int64_t nch = S.nchunks;
-  if (nch < 1 || nch > std::min<int64_t>(4 * ctx->num_sms, RES_MAX_CHUNKS) || ctx->shares_gpu || ctx->device < 0 || ctx->device >= 128)
+  if (nch < 1 || nch > std::min<int64_t>(2 * ctx->num_sms, RES_MAX_CHUNKS) || ctx->shares_gpu || ctx->device < 0 || ctx->device >= 128)
     return LLF_OK;
+  if (nch > ctx->num_sms) {
+    int l2 = 0;
+    LLF_CUDA_TRY(ctx, cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device));
+    if ((int64_t)sizeof(double) * m->pat->nnz > (int64_t)l2 / 8 * 5) return LLF_OK;
+  }
   std::unique_lock<std::mutex> lock(g_res_mutex[ctx->device], std::try_to_lock);
   if (!lock.owns_lock()) return LLF_OK;
   if (nch <= ctx->num_sms)
     return launch_resident<P, 1024, true>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, done);
-  if (nch <= 2 * (int64_t)ctx->num_sms)
-    return launch_resident<P, 512, true>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, done);
-  return launch_resident<P, 256, true>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, done);
+  return launch_resident<P, 512, true>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, done);
 }
 
 // Buffers, chunking and preconditioner of the segmented PCG for one matrix

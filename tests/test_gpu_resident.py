@@ -77,8 +77,8 @@ def test_resident_with_nodes_in_random_order(llf, n, order):
     assert np.array_equal(got[0], want[0]) and got[1:] == want[1:]
 
 
-def test_resident_four_per_sm_and_batches(llf):
-    """A system with more than two chunks per SM alone (four CTAs per SM), a
+def test_resident_batches(llf):
+    """A system with more than two chunks per SM alone (the launches), a
     batch of uneven systems in one launch, and a batch with more chunks than
     CTAs (the launches): every system as it is alone."""
     ms = [llf.structured_box_mesh(n=n, order=1) for n in (62, 62, 62)]
