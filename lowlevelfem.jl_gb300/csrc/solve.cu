@@ -157,40 +157,6 @@ __device__ __forceinline__ void node_columns_at(const double *__restrict__ nz, c
     for (int j = 0; j < P; ++j) acc[j] = __dadd_rn(acc[j], __shfl_xor_sync(0xffffffffu, acc[j], off));
 }
 
-// The same for node B, whose row nodes are nadj[nptr[B] .. nptr[B+1]).
-template <int P>
-__device__ __forceinline__ void node_columns(const double *__restrict__ nz, const int64_t *__restrict__ nptr,
-                                             const int32_t *__restrict__ nadj, const double *__restrict__ x,
-                                             int64_t B, bool valid, int g, double (&acc)[P]) {
-  const int64_t r0 = valid ? nptr[B] : 0, r1 = valid ? nptr[B + 1] : 0;
-  node_columns_at<P>(nz, nadj, x, r0, r1, valid, g, acc);
-}
-
-// y = A x for all columns (plain product, llf_matrix_spmv), SPMV_G lanes per
-// column node.
-template <int P>
-__global__ void __launch_bounds__(CG_THREADS)
-k_spmv(const double *__restrict__ nz, const int64_t *__restrict__ colptr,
-       const int64_t *__restrict__ nptr, const int32_t *__restrict__ nadj,
-       const double *__restrict__ x, double *__restrict__ y, int64_t ndof) {
-  (void)colptr;
-  constexpr int NPW = 32 / SPMV_G;  // nodes per warp
-  const int lane = threadIdx.x & 31, g = lane % SPMV_G, wpb = blockDim.x >> 5;
-  const int64_t non = ndof / P;
-  const int64_t stride = (int64_t)gridDim.x * wpb * NPW;
-  for (int64_t B0 = ((int64_t)blockIdx.x * wpb + (threadIdx.x >> 5)) * NPW; B0 < non; B0 += stride) {
-    const int64_t B = B0 + lane / SPMV_G;
-    double acc[P];
-    node_columns<P>(nz, nptr, nadj, x, B, B < non, g, acc);
-    if (B < non && g < P) {
-      double v = acc[0];
-#pragma unroll
-      for (int j = 1; j < P; ++j) v = g == j ? acc[j] : v;
-      y[P * B + g] = v;
-    }
-  }
-}
-
 // Stored values, stored column starts (1-based) and keep bits of a matrix
 // whose assembly left the structural values out; vals null otherwise.
 struct KeptCols {
@@ -202,7 +168,7 @@ struct KeptCols {
 // node_columns_at from the stored values: entry i of a column is the stored
 // value at its rank among the column's kept entries, +0.0 when it is not
 // stored.  The lanes, the order of their sums and so the bits are the same.
-template <int P>
+template <int P, int U = 2>
 __device__ __forceinline__ void node_columns_kept(const KeptCols &K, const int32_t *__restrict__ nadj,
                                                   const double *__restrict__ x, int64_t B, int64_t r0, int64_t r1,
                                                   bool valid, int g, double (&acc)[P]) {
@@ -248,27 +214,71 @@ __device__ __forceinline__ void node_columns_kept(const KeptCols &K, const int32
     for (int j = 0; j < P; ++j) acc[j] = __dadd_rn(acc[j], __shfl_xor_sync(0xffffffffu, acc[j], off));
 }
 
-// The same product from the stored values and their keep bits, for a matrix
-// whose assembly left the structural values out.  A warp's POPCs and selects
-// (about 40 issue slots per step) fit beside its P FP64 instructions, which
-// take 64 each of an SM quarter.  hex27 40^3 (297.7 M entries): 0.87 ms;
-// expanding the structural values first and k_spmv took 2.55 + 0.83 ms.
-template <int P>
+constexpr int SPMV_TILE = 128;
+// The nodes of a tile by decreasing degree, then index: sOrd[r] is the r-th
+// one's place in the tile (nodes past the end last).
+__device__ __forceinline__ void tile_order(const int64_t *__restrict__ nptr, int64_t base, int64_t non, int4 *sKey,
+                                           int *sOrd) {
+  static_assert(CG_THREADS == 2 * SPMV_TILE, "two threads per node");
+  const int t = threadIdx.x, i = t >> 1;
+  int *key = reinterpret_cast<int *>(sKey);
+  if (t < SPMV_TILE)
+    key[t] = (base + t < non ? (int)(nptr[base + t + 1] - nptr[base + t]) + 1 : 0) * SPMV_TILE + (SPMV_TILE - 1 - t);
+  __syncthreads();
+  const int mine = key[i];
+  int rank = 0;
+#pragma unroll 4
+  for (int k = t & 1; k < SPMV_TILE / 4; k += 2) {
+    const int4 q = sKey[k];
+    rank += (q.x > mine) + (q.y > mine) + (q.z > mine) + (q.w > mine);
+  }
+  rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+  if ((t & 1) == 0) sOrd[rank] = i;
+  __syncthreads();
+}
+
+// y = A x for all columns (plain product, llf_matrix_spmv), SPMV_G lanes per
+// column node, from the structural values or (KEPT, for a matrix whose
+// assembly left them out) the stored values and their keep bits.
+// SORT, for large meshes of unlike nodes: the FP64 pipe bounds it
+// and is spent per warp instruction, so the eight nodes of a warp should have
+// rows of similar length, which in node order they have not (hex27: 27 to 125
+// row nodes).  A block takes 128 nodes by decreasing degree, a warp the groups
+// w and 15 - w, which also evens out the warps.  With fewer nodes a warp of
+// eight long rows is the last to end, so they stay in node order.  A column's
+// sums do not depend on the order.  KEPT's POPCs and selects (about 40 issue
+// slots per step) fit beside its P FP64 instructions, which take 64 each of an
+// SM quarter.
+// hex27 40^3 (297.7 M entries), KEPT: 0.845 -> 0.70 ms (the operations take
+// 0.49; four positions at a time instead of two 0.72 -> 0.70); tet10, 253,000
+// nodes 0.213 -> 0.186 ms.  Expanding the structural values of the first and
+// multiplying by those took 2.55 + 0.83 ms.
+template <int P, bool KEPT, bool SORT>
 __global__ void __launch_bounds__(CG_THREADS)
-k_spmv_kept(KeptCols K, const int64_t *__restrict__ nptr, const int32_t *__restrict__ nadj, const double *__restrict__ x,
-            double *__restrict__ y, int64_t non) {
-  constexpr int NPW = 32 / SPMV_G;  // nodes per warp
-  const int lane = threadIdx.x & 31, g = lane % SPMV_G, wpb = blockDim.x >> 5;
-  const int64_t stride = (int64_t)gridDim.x * wpb * NPW;
-  for (int64_t B0 = ((int64_t)blockIdx.x * wpb + (threadIdx.x >> 5)) * NPW; B0 < non; B0 += stride) {
-    const int64_t B = B0 + lane / SPMV_G;
-    double acc[P];
-    node_columns_kept<P>(K, nadj, x, B, B < non ? nptr[B] : 0, B < non ? nptr[B + 1] : 0, B < non, g, acc);
-    if (B < non && g < P) {
-      double t = acc[0];
+k_spmv(const double *__restrict__ nz, KeptCols K, const int64_t *__restrict__ nptr, const int32_t *__restrict__ nadj,
+       const double *__restrict__ x, double *__restrict__ y, int64_t non) {
+  constexpr int NPW = 32 / SPMV_G, NPB = NPW * (CG_THREADS / 32);  // nodes per warp, per round of a block
+  constexpr int TILE = SORT ? SPMV_TILE : NPB;
+  __shared__ int4 sKey[SORT ? SPMV_TILE / 4 : 1];
+  __shared__ int sOrd[SORT ? SPMV_TILE : 1];
+  const int g = threadIdx.x % SPMV_G, p = threadIdx.x / SPMV_G;
+  for (int64_t base = (int64_t)blockIdx.x * TILE; base < non; base += (int64_t)gridDim.x * TILE) {
+    if (SORT) tile_order(nptr, base, non, sKey, sOrd);
+#pragma unroll 1
+    for (int r = 0; r < TILE / NPB; ++r) {
+      const int at = r * NPB + (r & 1 ? (NPB / NPW - 1 - p / NPW) * NPW + p % NPW : p);
+      const int64_t B = base + (SORT ? sOrd[at] : at);
+      const bool valid = B < non;
+      const int64_t r0 = valid ? nptr[B] : 0, r1 = valid ? nptr[B + 1] : 0;
+      double acc[P];
+      if (KEPT) node_columns_kept<P, SORT && P == 3 ? 4 : 2>(K, nadj, x, B, r0, r1, valid, g, acc);
+      else node_columns_at<P>(nz, nadj, x, r0, r1, valid, g, acc);
+      if (valid && g < P) {
+        double t = acc[0];
 #pragma unroll
-      for (int j = 1; j < P; ++j) t = g == j ? acc[j] : t;
-      y[P * B + g] = t;
+        for (int j = 1; j < P; ++j) t = g == j ? acc[j] : t;
+        y[P * B + g] = t;
+      }
     }
   }
 }
@@ -1543,18 +1553,29 @@ KeptCols kept_cols(const llf_matrix *m) {
 }
 
 // y = A x, from whichever values the matrix holds.
+template <int P, bool KEPT, bool SORT>
+void launch_spmv_as(llf_ctx *ctx, const llf_matrix *m, const double *x, double *y) {
+  const llf_pattern *p = m->pat;
+  const int64_t non = p->ndof / P, tile = SORT ? SPMV_TILE : CG_THREADS / SPMV_G;
+  const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((non + tile - 1) / tile, 1 << 30));
+  KernelScope ks(ctx, KEPT ? "k_spmv_kept" : "k_spmv");
+  k_spmv<P, KEPT, SORT><<<grid, CG_THREADS, 0, ctx->stream>>>(m->d_nz, kept_cols(m), p->d_nptr, p->d_nadj, x, y, non);
+}
+
+// By degree where that leaves four blocks per SM and the longest row is well
+// above the mean one (quad4 300x300, all alike: 19 us in node order, 21 by
+// degree; tet20 with 20,000 nodes, two blocks per SM: 150 against 164 us).
 template <int P>
 void launch_spmv(llf_ctx *ctx, const llf_matrix *m, const double *x, double *y) {
-  const llf_pattern *p = m->pat;
-  const int64_t non = p->ndof / P;
-  constexpr int per_block = CG_THREADS / SPMV_G;
-  const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((non + per_block - 1) / per_block, 1 << 30));
+  const int64_t non = m->pat->ndof / P;
+  const bool sort = non >= (int64_t)SPMV_TILE * 4 * ctx->num_sms &&
+                    4 * (int64_t)m->pat->max_deg * P * P * non > 5 * m->pat->nnz;
   if (m->d_nz) {
-    KernelScope ks(ctx, "k_spmv");
-    k_spmv<P><<<grid, CG_THREADS, 0, ctx->stream>>>(m->d_nz, p->d_colptr, p->d_nptr, p->d_nadj, x, y, p->ndof);
+    if (sort) launch_spmv_as<P, false, true>(ctx, m, x, y);
+    else launch_spmv_as<P, false, false>(ctx, m, x, y);
   } else {
-    KernelScope ks(ctx, "k_spmv_kept");
-    k_spmv_kept<P><<<grid, CG_THREADS, 0, ctx->stream>>>(kept_cols(m), p->d_nptr, p->d_nadj, x, y, non);
+    if (sort) launch_spmv_as<P, true, true>(ctx, m, x, y);
+    else launch_spmv_as<P, true, false>(ctx, m, x, y);
   }
 }
 
@@ -2210,7 +2231,7 @@ k_mx_true(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ nptr
       const bool valid = rr_idx < nb;
       const int64_t B = b0 + (valid ? rr_idx : 0);
       double acc[P];
-      node_columns<P>(nz, nptr, nadj, xw, B, valid, g, acc);
+      node_columns_at<P>(nz, nadj, xw, valid ? nptr[B] : 0, valid ? nptr[B + 1] : 0, valid, g, acc);
       if (valid && g == 0) {
         float rn[P];
 #pragma unroll
@@ -2338,7 +2359,7 @@ int pcg_mixed_core(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double 
   { KernelScope k(ctx, "k_f64_to_f32");
     k_f64_to_f32<<<(unsigned)(ctx->num_sms * 8), CG_THREADS, 0, s>>>(m->d_nz, B.nz32, pat->nnz); }
   { KernelScope k(ctx, "k_keep_fixed"); k_keep_fixed<<<gv, CG_THREADS, 0, s>>>(d_x, d_fixed, xw, n); }
-  { KernelScope k(ctx, "k_spmv"); k_spmv<P><<<gv, CG_THREADS, 0, s>>>(m->d_nz, pat->d_colptr, pat->d_nptr, pat->d_nadj, xw, tmp, n); }
+  launch_spmv<P>(ctx, m, xw, tmp);
   { KernelScope k(ctx, "k_mx_init"); k_mx_init<<<gch, CG_THREADS, 0, s>>>(S, d_b, tmp, d_fixed, B.rb, B.r, xw, B.u, part); }
   { KernelScope k(ctx, "k_seg_start"); k_seg_start<<<gseg, CG_THREADS, 0, s>>>(S, part, reltol, (long long)maxiter); }
   if (local) {
@@ -3051,8 +3072,7 @@ int prepare_t(llf_ctx *ctx, const llf_matrix *K, const double *hb, const double 
     k_precond_setup<P><<<(unsigned)((non + 127) / 128), 128, 0, s>>>(K->d_nz, kept_cols(K), pat->d_colptr, pat->d_diagpos, sy->fixed,
                                                                      non, precond, sy->pinv); }
   { KernelScope k(ctx, "k_keep_fixed"); k_keep_fixed<<<gv, CG_THREADS, 0, s>>>(sy->x, sy->fixed, sy->xw, n); }
-  { KernelScope k(ctx, "k_spmv");
-    k_spmv<P><<<gv, CG_THREADS, 0, s>>>(K->d_nz, pat->d_colptr, pat->d_nptr, pat->d_nadj, sy->xw, sy->c, n); }
+  launch_spmv<P>(ctx, K, sy->xw, sy->c);
   { KernelScope k(ctx, "k_seg_init"); k_seg_init<<<gch, CG_THREADS, 0, s>>>(S, sy->b, sy->c, sy->fixed, sy->r, sy->xw, sy->u, part); }
   { KernelScope k(ctx, "k_seg_start"); k_seg_start<<<1, CG_THREADS, 0, s>>>(S, part, reltol, (long long)maxiter); }
   { KernelScope k(ctx, "k_seg_prec"); k_seg_prec<P><<<gch, CG_THREADS, 0, s>>>(S, sy->pinv, precond, sy->r, sy->fixed, sy->z, part); }
