@@ -388,9 +388,9 @@ class DeviceMatrix:
 
     def copy_csc(self):
         nnz = self.nnz()
-        colptr = np.zeros(self.n + 1, dtype=np.int64)
-        rowval = np.zeros(nnz, dtype=np.int64)
-        nzval = np.zeros(nnz)
+        colptr = np.empty(self.n + 1, dtype=np.int64)
+        rowval = np.empty(nnz, dtype=np.int64)
+        nzval = np.empty(nnz)
         self.ctx.check(lib().llf_matrix_copy_csc(self.ctx.h, self.h, ptr(colptr, C.c_int64),
                                                  ptr(rowval, C.c_int64), ptr(nzval, C.c_double)))
         return colptr, rowval, nzval
@@ -411,7 +411,7 @@ class DeviceMatrix:
 
     def spmv(self, x: np.ndarray) -> np.ndarray:
         x = f64(x)
-        y = np.zeros(self.n)
+        y = np.empty(self.n)
         self.ctx.check(lib().llf_matrix_spmv(self.ctx.h, self.h, ptr(x, C.c_double), ptr(y, C.c_double)))
         return y
 

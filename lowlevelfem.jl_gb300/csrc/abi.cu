@@ -40,10 +40,12 @@ void prof_resolve(llf_ctx *ctx) {
   ctx->pending.clear();
 }
 
-int llf_check_status(llf_ctx *ctx, const char *what) {
-  LLF_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(unsigned),
-                                    cudaMemcpyDeviceToHost, ctx->stream));
-  LLF_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+int llf_check_status(llf_ctx *ctx, const char *what, bool fetched) {
+  if (!fetched) {
+    LLF_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(unsigned),
+                                      cudaMemcpyDeviceToHost, ctx->stream));
+    LLF_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+  }
   unsigned st = *ctx->h_status;
   if (st == 0) return LLF_OK;
   LLF_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(unsigned), ctx->stream));
@@ -211,9 +213,9 @@ int llf_ctx_create(int device, llf_ctx **out) {
   if (!c) return LLF_ERR_LIMIT;
   c->device = device;
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc((void **)&c->d_status, sizeof(unsigned)) != cudaSuccess ||
-      cudaMallocHost((void **)&c->h_status, sizeof(unsigned)) != cudaSuccess ||
-      cudaMemset(c->d_status, 0, sizeof(unsigned)) != cudaSuccess ||
+      cudaMalloc((void **)&c->d_status, 2 * sizeof(unsigned)) != cudaSuccess ||
+      cudaMallocHost((void **)&c->h_status, 2 * sizeof(unsigned)) != cudaSuccess ||
+      cudaMemset(c->d_status, 0, 2 * sizeof(unsigned)) != cudaSuccess ||
       cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
     delete c;
     return LLF_ERR_CUDA;

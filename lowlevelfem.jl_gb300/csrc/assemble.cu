@@ -1331,31 +1331,28 @@ int assemble_impl(llf_ctx *ctx, llf_mesh *mesh, llf_pattern *pat, int kind, int 
   const int BS = (kind == KIND_ELASTIC) ? P * P : 1;
   cudaStream_t s = ctx->stream;
 
-  double *d_c1 = nullptr, *d_c2 = nullptr;
+  double *d_c1 = nullptr;   // c1, then c2
   int64_t *cnt = nullptr;
-  LLF_CUDA_TRY(ctx, dalloc(ctx, &d_c1, nmat));
-  LLF_CUDA_TRY(ctx, dalloc(ctx, &d_c2, nmat));
+  LLF_CUDA_TRY(ctx, dalloc(ctx, &d_c1, 2 * (size_t)nmat));
   LLF_CUDA_TRY(ctx, dalloc(ctx, &cnt, pat->ndof + 1));
-  LLF_CUDA_TRY(ctx, cudaMemsetAsync(cnt, 0, sizeof(int64_t) * (pat->ndof + 1), s));
-  LLF_CUDA_TRY(ctx, cudaMemcpyAsync(d_c1, c1, sizeof(double) * nmat, cudaMemcpyHostToDevice, s));
-  LLF_CUDA_TRY(ctx, cudaMemcpyAsync(d_c2, c2 ? c2 : c1, sizeof(double) * nmat,
-                                    cudaMemcpyHostToDevice, s));
+  std::vector<double> hc(c1, c1 + nmat);
+  hc.insert(hc.end(), c2 ? c2 : c1, (c2 ? c2 : c1) + nmat);
+  LLF_CUDA_TRY(ctx, cudaMemcpyAsync(d_c1, hc.data(), sizeof(double) * hc.size(), cudaMemcpyHostToDevice, s));
+  const double *d_c2 = d_c1 + nmat;
   // the stored layout of the last assembly of this operator and form on
   // the pattern: the gather then writes the stored CSC itself, and the
   // structural values are left to matrix_ensure_nz
   const bool reuse = !sink && !init && !(kind == KIND_MASS && lumped) && !m->keep_pattern && layout_reuse_enabled();
   llf_pattern::StoredLayout *lay = reuse ? layout_find(pat, kind, form) : nullptr;
   StoredSpec spec;
-  unsigned *d_mis = nullptr;
+  if (!lay) LLF_CUDA_TRY(ctx, cudaMemsetAsync(cnt, 0, sizeof(int64_t) * (pat->ndof + 1), s));
   if (lay) {
     LLF_CUDA_TRY(ctx, dalloc(ctx, &m->d_rowval_s, lay->total > 0 ? lay->total : 1));
     LLF_CUDA_TRY(ctx, dalloc(ctx, &m->d_nzval_s, lay->total > 0 ? lay->total : 1));
-    LLF_CUDA_TRY(ctx, dalloc(ctx, &d_mis, 1));
-    LLF_CUDA_TRY(ctx, cudaMemsetAsync(d_mis, 0, sizeof(unsigned), s));
     spec.ptr0 = lay->d_ptr0;
     spec.rowval_s = m->d_rowval_s;
     spec.nzval_s = m->d_nzval_s;
-    spec.mismatch = d_mis;
+    spec.mismatch = ctx->d_status + 1;
     LLF_CUDA_TRY(ctx, dalloc(ctx, &m->d_keep, keep_words(pat->nnz, pat->ndof)));
     spec.keep = m->d_keep;
     spec.nz_slot = &m->d_nz;
@@ -1472,8 +1469,7 @@ int assemble_impl(llf_ctx *ctx, llf_mesh *mesh, llf_pattern *pat, int kind, int 
     dfree(ctx, Kf);
   }
   dfree(ctx, d_c1);
-  dfree(ctx, d_c2);
-  if (rc == LLF_OK) rc = llf_check_status(ctx, "assembly");
+  if (rc == LLF_OK) rc = llf_check_status(ctx, "assembly", spec.status_read && !spec.fell_back);
   if (sink) {
     dfree(ctx, cnt);
     return rc;
@@ -1489,7 +1485,6 @@ int assemble_impl(llf_ctx *ctx, llf_mesh *mesh, llf_pattern *pat, int kind, int 
     }
   }
   if (lay && rc == LLF_OK) {
-    dfree(ctx, d_mis);
     if (!spec.fell_back) {  // every column's count matched: the stored CSC is complete
       m->nnz_s = lay->total;
       lay->used = ++pat->layout_clock;
@@ -1502,7 +1497,6 @@ int assemble_impl(llf_ctx *ctx, llf_mesh *mesh, llf_pattern *pat, int kind, int 
     dfree(ctx, m->d_nzval_s);
     rc = matrix_finalize(ctx, m, cnt, reuse ? &ptr0 : nullptr);
   } else {
-    dfree(ctx, d_mis);
     if (rc == LLF_OK)
       rc = matrix_finalize(ctx, m, (kind == KIND_MASS && lumped) ? nullptr : cnt, reuse ? &ptr0 : nullptr);
   }

@@ -44,8 +44,10 @@ struct llf_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   std::string err;
-  unsigned *d_status = nullptr;   // device status word
-  unsigned *h_status = nullptr;   // pinned host mirror
+  // device status word, then a word that a gather into a kept stored layout sets
+  // when a column's count differs (zero between assemblies)
+  unsigned *d_status = nullptr;
+  unsigned *h_status = nullptr;   // pinned host mirror of both
   int num_sms = 0;
   bool profiling = false;
   bool shares_gpu = false;        // other contexts' kernels run beside this one's (a server's contexts)
@@ -190,6 +192,7 @@ struct StoredSpec {
   double **nz_slot = nullptr;
   int64_t *cnt_fallback = nullptr;
   bool fell_back = false;
+  bool status_read = false;        // ctx->h_status holds the status after the gather
 };
 
 struct llf_matrix {
@@ -235,7 +238,8 @@ int llf_fail(llf_ctx *ctx, int code, const std::string &msg);
 int llf_ok(llf_ctx *ctx);
 
 // Read and clear the device status word (synchronises the stream).
-int llf_check_status(llf_ctx *ctx, const char *what);
+// Reads the status word (fetched: it is in ctx->h_status already) and fails on it.
+int llf_check_status(llf_ctx *ctx, const char *what, bool fetched = false);
 
 template <class T>
 cudaError_t dalloc(llf_ctx *ctx, T **p, size_t count) {

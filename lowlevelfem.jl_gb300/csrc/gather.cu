@@ -612,11 +612,16 @@ int gather_spec_t(llf_ctx *ctx, llf_pattern *pat, const T *Kf, int64_t cs, bool 
   int rc = gather_full_t<T>(ctx, pat, pat->d_n2e_ptr, pat->d_n2e, pat->d_pos, pat->mesh->npe, Kf, cs, blockval,
                             nullptr, nullptr, nullptr, spec);
   if (rc != LLF_OK) return rc;
-  unsigned mis = 1;
-  LLF_CUDA_TRY(ctx, cudaMemcpyAsync(&mis, spec->mismatch, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+  // the status of the whole assembly comes with the mismatch word: one copy
+  // into pinned memory and one wait
+  LLF_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_status, ctx->d_status, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost,
+                                    ctx->stream));
   LLF_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-  if (mis == 0) return LLF_OK;
+  spec->status_read = true;
+  if (ctx->h_status[1] == 0) return LLF_OK;
   spec->fell_back = true;
+  LLF_CUDA_TRY(ctx, cudaMemsetAsync(spec->mismatch, 0, sizeof(unsigned), ctx->stream));
+  LLF_CUDA_TRY(ctx, cudaMemsetAsync(spec->cnt_fallback, 0, sizeof(int64_t) * (pat->ndof + 1), ctx->stream));
   LLF_CUDA_TRY(ctx, dalloc(ctx, spec->nz_slot, pat->nnz));
   return gather_full_t<T>(ctx, pat, pat->d_n2e_ptr, pat->d_n2e, pat->d_pos, pat->mesh->npe, Kf, cs, blockval,
                           nullptr, *spec->nz_slot, spec->cnt_fallback);
