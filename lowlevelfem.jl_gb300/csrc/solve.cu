@@ -1657,6 +1657,9 @@ int launch_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const doubl
   auto fn = k_cg_resident<P, T, HALO>;
   // row nodes in shared memory as far as the CTA's share of the SM goes
   const size_t fixed_b = res_smem_fixed<P>(), room = (size_t)(216 * 1024) / (1024 / T);
+  // row nodes that do not fit on average leave no room for a halo
+  if (HALO && fixed_b + sizeof(int) * (size_t)(pat->nnzb / nch) > room)
+    return launch_resident<P, T, false>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, done);
   const int adj_cap = (int)std::min<int64_t>((int64_t)(CHUNK / P) * std::max(pat->max_deg, 1),
                                              (int64_t)((room - fixed_b) / sizeof(int)));
   const size_t smem = HALO ? room : fixed_b + sizeof(int) * (size_t)adj_cap;
