@@ -157,6 +157,42 @@ __device__ __forceinline__ void node_columns_at(const double *__restrict__ nz, c
     for (int j = 0; j < P; ++j) acc[j] = __dadd_rn(acc[j], __shfl_xor_sync(0xffffffffu, acc[j], off));
 }
 
+// node_columns_at for long rows, U positions of a lane at once.
+template <int P, int U>
+__device__ __forceinline__ void node_columns_long(const double *__restrict__ nz, const int32_t *__restrict__ nadj,
+                                                  const double *__restrict__ x, int64_t r0, int64_t r1, bool valid,
+                                                  int g, double (&acc)[P]) {
+#pragma unroll
+  for (int j = 0; j < P; ++j) acc[j] = 0.0;
+  if (valid) {
+    const int n = (int)(r1 - r0) * P;  // entries per column
+    const double *col = nz + (int64_t)P * r0 * P;
+    int k = g;
+    for (; k + (U - 1) * SPMV_G < n; k += U * SPMV_G) {
+      double v[U][P], xv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int j = 0; j < P; ++j) v[u][j] = col[(int64_t)j * n + k + u * SPMV_G];
+#pragma unroll
+      for (int u = 0; u < U; ++u) xv[u] = x[(int64_t)P * nadj[r0 + (k + u * SPMV_G) / P] + (k + u * SPMV_G) % P];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int j = 0; j < P; ++j) acc[j] = __fma_rn(v[u][j], xv[u], acc[j]);
+    }
+    for (; k < n; k += SPMV_G) {
+      const double xa = x[(int64_t)P * nadj[r0 + k / P] + k % P];
+#pragma unroll
+      for (int j = 0; j < P; ++j) acc[j] = __fma_rn(col[(int64_t)j * n + k], xa, acc[j]);
+    }
+  }
+#pragma unroll
+  for (int off = SPMV_G / 2; off > 0; off >>= 1)
+#pragma unroll
+    for (int j = 0; j < P; ++j) acc[j] = __dadd_rn(acc[j], __shfl_xor_sync(0xffffffffu, acc[j], off));
+}
+
 // Stored values, stored column starts (1-based) and keep bits of a matrix
 // whose assembly left the structural values out; vals null otherwise.
 struct KeptCols {
@@ -168,7 +204,7 @@ struct KeptCols {
 // node_columns_at from the stored values: entry i of a column is the stored
 // value at its rank among the column's kept entries, +0.0 when it is not
 // stored.  The lanes, the order of their sums and so the bits are the same.
-template <int P, int U = 2>
+template <int P>
 __device__ __forceinline__ void node_columns_kept(const KeptCols &K, const int32_t *__restrict__ nadj,
                                                   const double *__restrict__ x, int64_t B, int64_t r0, int64_t r1,
                                                   bool valid, int g, double (&acc)[P]) {
@@ -249,15 +285,22 @@ __device__ __forceinline__ void tile_order(const int64_t *__restrict__ nptr, int
 // sums do not depend on the order.  KEPT's POPCs and selects (about 40 issue
 // slots per step) fit beside its P FP64 instructions, which take 64 each of an
 // SM quarter.
-// hex27 40^3 (297.7 M entries), KEPT: 0.845 -> 0.70 ms (the operations take
-// 0.49; four positions at a time instead of two 0.72 -> 0.70); tet10, 253,000
-// nodes 0.213 -> 0.186 ms.  Expanding the structural values of the first and
-// multiplying by those took 2.55 + 0.83 ms.
-template <int P, bool KEPT, bool SORT>
-__global__ void __launch_bounds__(CG_THREADS)
+// The second launch bound is a register allowance: with three components the
+// compiler otherwise keeps to 32 registers (56 with KEPT) by placing loads
+// beside their uses, and every load is waited for.  LONG (rows of 512 entries
+// or more, no SORT): eight positions of a lane at once.
+// hex27 40^3 (297.7 M entries), KEPT: 0.845 -> 0.72 by degree -> 0.68 ms with
+// the allowance (the operations take 0.49); tet10, 253,000 nodes 0.213 -> 0.19 ->
+// 0.178; expanding the structural values of the first and multiplying by those
+// took 2.55 + 0.83 ms.  In node
+// order, 128 threads a block so that more rows are under way beside a long
+// one: hex64 0.225 -> 0.189, tet20 0.154 -> 0.133 ms and, structural values and
+// LONG, hex125 with 40,293 nodes 0.425 -> 0.302 ms.
+template <int P, bool KEPT, bool SORT, bool LONG>
+__global__ void __launch_bounds__(SORT ? CG_THREADS : 128, P != 3 ? 0 : (SORT ? 3 : (LONG ? 4 : 6)))
 k_spmv(const double *__restrict__ nz, KeptCols K, const int64_t *__restrict__ nptr, const int32_t *__restrict__ nadj,
        const double *__restrict__ x, double *__restrict__ y, int64_t non) {
-  constexpr int NPW = 32 / SPMV_G, NPB = NPW * (CG_THREADS / 32);  // nodes per warp, per round of a block
+  constexpr int NPW = 32 / SPMV_G, NPB = (SORT ? CG_THREADS : 128) / SPMV_G;  // nodes per warp, per round of a block
   constexpr int TILE = SORT ? SPMV_TILE : NPB;
   __shared__ int4 sKey[SORT ? SPMV_TILE / 4 : 1];
   __shared__ int sOrd[SORT ? SPMV_TILE : 1];
@@ -271,7 +314,8 @@ k_spmv(const double *__restrict__ nz, KeptCols K, const int64_t *__restrict__ np
       const bool valid = B < non;
       const int64_t r0 = valid ? nptr[B] : 0, r1 = valid ? nptr[B + 1] : 0;
       double acc[P];
-      if (KEPT) node_columns_kept<P, SORT && P == 3 ? 4 : 2>(K, nadj, x, B, r0, r1, valid, g, acc);
+      if (KEPT) node_columns_kept<P>(K, nadj, x, B, r0, r1, valid, g, acc);
+      else if (LONG) node_columns_long<P, 8>(nz, nadj, x, r0, r1, valid, g, acc);
       else node_columns_at<P>(nz, nadj, x, r0, r1, valid, g, acc);
       if (valid && g < P) {
         double t = acc[0];
@@ -563,8 +607,9 @@ __global__ void k_seg_dir(Seg S, const double *__restrict__ z, double *__restric
 // well, and the partial u.c takes the chunk's DoFs as the update's sums do
 // (thread t: DoFs t, t + 256, t + 512), every lane busy.  The block that brings in a segment's last
 // chunk sums the partials (chunk order) and sets alpha = rho / u.c.
+// Registers as in k_spmv: eight tet10 systems together, 94 -> 87 us a product.
 template <int P, bool KEPT>
-__global__ void __launch_bounds__(CG_THREADS)
+__global__ void __launch_bounds__(CG_THREADS, P == 3 ? 4 : 0)
 k_seg_spmv(Seg S, const double *__restrict__ nz, KeptCols K, const int64_t *__restrict__ nptr,
            const int32_t *__restrict__ nadj, const double *__restrict__ u,
            const uint8_t *__restrict__ fixed, double *__restrict__ c, double *__restrict__ part) {
@@ -1553,13 +1598,14 @@ KeptCols kept_cols(const llf_matrix *m) {
 }
 
 // y = A x, from whichever values the matrix holds.
-template <int P, bool KEPT, bool SORT>
+template <int P, bool KEPT, bool SORT, bool LONG>
 void launch_spmv_as(llf_ctx *ctx, const llf_matrix *m, const double *x, double *y) {
   const llf_pattern *p = m->pat;
-  const int64_t non = p->ndof / P, tile = SORT ? SPMV_TILE : CG_THREADS / SPMV_G;
+  constexpr int threads = SORT ? CG_THREADS : 128;
+  const int64_t non = p->ndof / P, tile = SORT ? SPMV_TILE : threads / SPMV_G;
   const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((non + tile - 1) / tile, 1 << 30));
   KernelScope ks(ctx, KEPT ? "k_spmv_kept" : "k_spmv");
-  k_spmv<P, KEPT, SORT><<<grid, CG_THREADS, 0, ctx->stream>>>(m->d_nz, kept_cols(m), p->d_nptr, p->d_nadj, x, y, non);
+  k_spmv<P, KEPT, SORT, LONG><<<grid, threads, 0, ctx->stream>>>(m->d_nz, kept_cols(m), p->d_nptr, p->d_nadj, x, y, non);
 }
 
 // By degree where that leaves four blocks per SM and the longest row is well
@@ -1571,11 +1617,12 @@ void launch_spmv(llf_ctx *ctx, const llf_matrix *m, const double *x, double *y) 
   const bool sort = non >= (int64_t)SPMV_TILE * 4 * ctx->num_sms &&
                     4 * (int64_t)m->pat->max_deg * P * P * non > 5 * m->pat->nnz;
   if (m->d_nz) {
-    if (sort) launch_spmv_as<P, false, true>(ctx, m, x, y);
-    else launch_spmv_as<P, false, false>(ctx, m, x, y);
+    if (sort) launch_spmv_as<P, false, true, false>(ctx, m, x, y);
+    else if (m->pat->max_deg * P >= 512) launch_spmv_as<P, false, false, true>(ctx, m, x, y);
+    else launch_spmv_as<P, false, false, false>(ctx, m, x, y);
   } else {
-    if (sort) launch_spmv_as<P, true, true>(ctx, m, x, y);
-    else launch_spmv_as<P, true, false>(ctx, m, x, y);
+    if (sort) launch_spmv_as<P, true, true, false>(ctx, m, x, y);
+    else launch_spmv_as<P, true, false, false>(ctx, m, x, y);
   }
 }
 

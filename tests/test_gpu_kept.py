@@ -100,3 +100,18 @@ def _noalloc(llf, K, b, fixed, precond):
     K.dm.ctx.check(rc, "llf_pcg_noalloc")
     assert K.dm.ctx.allocs() == allocs0
     return dx.cpu().numpy(), it.value
+
+
+@pytest.mark.parametrize("case", [("box", (3, 3, 2), 4, False, "K"), ("box", (44, 43, 42), 1, True, "K"),
+                                  ("rect", (190, 210), 2, False, "K")], ids=["long-rows", "by-degree", "by-degree-2d"])
+def test_product_against_the_stored_matrix(llf, case):
+    """Long rows in node order and the product by degree (77,824 nodes and
+    more), from structural and stored values, against scipy on the CSC."""
+    P = _problem(llf, *case, turned=True)
+    first = _assemble(llf, P, case[-1])
+    x = np.random.default_rng(9).standard_normal(P.pdim * P.non)
+    y = first * x
+    A = first.A
+    bound = abs(A) @ abs(x)   # of a row's sum: 2,187 terms at most, each rounded twice
+    assert np.all(np.abs(y - A @ x) <= 2 * 2187 * 2.0**-53 * bound)
+    assert np.array_equal(_assemble(llf, P, case[-1]) * x, y)
