@@ -47,14 +47,14 @@ def workload_name(n):
     """The workload label for n cells per edge (the headline case is 40)."""
     return f"hooke3d-unit-cube-hex27-{n}x{n}x{n}"
 # ncu DRAM bytes (read + write) of one FP64 assembly of hex27 16^3 (19,320,201
-# structural nnz): k_affine_geometry 1.3 MB, k_elem_affine 153.8 MB (the
-# general-geometry k_elem_fp64 165.0 MB), k_colgather 338.2 MB, k_compact 417.5 MB
+# structural nnz): k_affine_geometry 1.3 MB, k_affine_coeff 0.4 MB, k_elem_packed
+# 152.9 MB, k_colgather 338.2 MB (into the kept layout 420.2 MB), k_compact 417.5 MB
 NNZ_16CUBE = 19320201
-KERNEL_DRAM_BYTES_16CUBE = {"k_affine_geometry": 1.324032e6, "k_elem_fp64": (6.096128 + 158.8992) * 1e6,
-                            "k_elem_affine": (0.392704 + 153.449984) * 1e6,
+KERNEL_DRAM_BYTES_16CUBE = {"k_affine_geometry": 1.324032e6, "k_affine_coeff": 0.353536e6,
+                            "k_elem_packed": (1.539712 + 151.400576) * 1e6,
                             "k_colgather": (224.209664 + 114.00704) * 1e6, "k_compact": (165.33248 + 252.210688) * 1e6,
                             # the gather compacting into the pattern's kept stored layout (both launches)
-                            "k_colgather_layout": (179.443968 + 174.397696 + 58.287104 + 7.202048) * 1e6}
+                            "k_colgather_layout": (179.8208 + 177.19424 + 58.180224 + 5.301632) * 1e6}
 
 
 def parse():
@@ -859,17 +859,16 @@ def main():
         del x
     except Exception:
         pass
-    ek = prof.get("k_elem_affine") or prof.get("k_elem_fp64") or {}
-    elem_ms = ek.get("ms", 0.0) / max(ek.get("launches", 1), 1)
+    # the element kernel with the kernel that forms its coefficients
+    elem_ms = sum(prof[k]["ms"] / max(prof[k]["launches"], 1) for k in ("k_affine_coeff", "k_elem_packed") if k in prof)
     fp64_achieved = flops / (elem_ms * 1e-3) / 1e12 if elem_ms > 0 else None
 
     # DRAM traffic of one FP64 assembly from ncu captures of its kernels on
     # hex27 16^3 (profiles/k_*_hex27_16cube.md), scaled by structural nnz
     traffic = traffic_k = None
     if form == L.FP64 and ORDER == 2:
-        elem_k = "k_elem_affine" if "k_elem_affine" in prof else "k_elem_fp64"
         layout = "k_compact" not in prof   # every timed assembly wrote into the kept stored layout
-        parts = [elem_k, "k_colgather_layout"] if layout else [elem_k, "k_colgather", "k_compact"]
+        parts = ["k_affine_coeff", "k_elem_packed"] + (["k_colgather_layout"] if layout else ["k_colgather", "k_compact"])
         if "k_affine_geometry" in prof:    # (kept on the mesh after the first assembly)
             parts.insert(0, "k_affine_geometry")
         if all(k in KERNEL_DRAM_BYTES_16CUBE for k in parts):
