@@ -223,9 +223,10 @@ int llf_pattern_destroy(llf_ctx *ctx, llf_pattern *pat);
  * usual way and keeps the new layout.  The arrays returned are the same
  * either way.  A matrix assembled into a kept layout holds the stored CSC
  * only; its structural values (the solvers' format) are expanded from it on
- * the first call that needs them (llf_pcg*, llf_matrix_spmv,
- * llf_matrix_copy_structural, llf_matrix_axpby, llf_heat_fdm, or
- * llf_matrix_prepare), except llf_pcg_noalloc, which refuses such a matrix.
+ * the first call that needs them (llf_pcg*, llf_matrix_copy_structural,
+ * llf_matrix_axpby, llf_heat_fdm, or llf_matrix_prepare).  llf_matrix_spmv
+ * multiplies by the stored values, and llf_pcg_noalloc refuses such a matrix
+ * until llf_matrix_spmv or llf_matrix_prepare has run on it.
  * LLF_STORED_LAYOUT=0 in the environment turns the reuse off.  Not used for
  * lumped mass matrices, nor for assemblies that accumulate into a matrix. */
 
@@ -557,8 +558,9 @@ int llf_heat_fdm(llf_ctx *ctx, const llf_matrix *K, const llf_matrix *C,
  * and writes every other work vector before reading it.  Calls whose work
  * overlaps on the GPU (two contexts or threads at once) race on the array:
  * serialise them.  The matrix's structural values must be resident (see
- * llf_matrix_prepare); a matrix that holds its stored CSC only is refused
- * with LLF_ERR_STATE. */
+ * llf_matrix_prepare), or a product (llf_matrix_spmv) must have run on it;
+ * another matrix that holds its stored CSC only is refused with
+ * LLF_ERR_STATE. */
 int llf_pcg_noalloc(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double *d_x,
                     const uint8_t *d_fixed, int precond, double reltol, int64_t maxiter,
                     int64_t *iters, double *relres);

@@ -22,9 +22,11 @@
 // test — inside the same launches.  DoFs are cut into fixed chunks that never
 // straddle a segment; every reduction is per chunk (block tree), then per
 // segment over its chunks in order, so results do not depend on the launch
-// shape or on what else is in the batch.  One CG iteration is seven
-// launches; the host captures a run of iterations into a CUDA graph once and
-// replays it, polling the count of still-active segments between replays.
+// shape or on what else is in the batch.  Systems small enough run their whole
+// loop in one resident kernel (k_cg_resident).  Otherwise one CG iteration is
+// three launches (with IC(0), its sweeps besides); the host captures a run of
+// iterations into a CUDA graph once and replays it, polling the count of
+// still-active segments between replays.
 // Iterations after a segment converged are no-ops for that segment, so every
 // segment stops exactly where IterativeSolvers would.
 #include "common.cuh"
