@@ -6,7 +6,7 @@
 //                 reference element (and which of those are axis-aligned
 //                 bricks), with their J^-1 and det;
 //   k_elem_packed elements of up to 384 node pairs: as many per CTA as fill
-//                 its threads (one hex27, ten hex8), after k_affine_coeff
+//                 its threads (one hex27, eight hex8), after k_affine_coeff
 //                 has formed the affine ones' coefficients;
 //   k_elem_affine larger elements of meshes whose elements are all affine:
 //                 one CTA per element at a time (persistent), the node-pair
