@@ -34,6 +34,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdio>
 #include <cstdlib>
 #include <mutex>
 
@@ -790,8 +791,8 @@ __global__ void k_keep_fixed(const double *__restrict__ x, const uint8_t *__rest
 // the CTA size, so a solve gives the same bits as the launches and as the
 // serving engine.
 // Waits are bounded (RES_LIMIT_NS): a CTA that gives up sets *abort and
-// returns, every other one follows, and the host runs the launches instead
-// (x is written at the end only).
+// returns, every other one follows, and the host sets the solve up again and
+// runs the launches instead.
 constexpr unsigned long long RES_LIMIT_NS = 20000000000ull;   // 0: gives up at the first poll that fails
 constexpr unsigned RES_NO_ROOM = 2;   // *abort: a halo does not fit (1: a wait ran out)
 
@@ -805,6 +806,8 @@ struct ResSync {
   unsigned long long *dir;
   unsigned *abort;
   unsigned long long limit;   // ns
+  long long quit_chunk;       // tests: this chunk's CTA gives up at the second meeting of iteration quit_it (-1: none)
+  unsigned long long quit_it;
 };
 
 __device__ __forceinline__ unsigned long long res_now() {
@@ -1261,6 +1264,7 @@ k_cg_resident(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ 
       }
       (second ? sv1 : sv0)[threadIdx.x & 255] = s;
     }
+    if (ch == Y.quit_chunk && it == Y.quit_it && threadIdx.x == 0) fail = true;
     if (__syncthreads_or(fail)) break;
     if (w < 8) res_fold(w < 4 ? sv0 : sv1, w < 4 ? sw0 : sw1, w, lane);
     __syncthreads();
@@ -1685,21 +1689,17 @@ inline int64_t res_sync_words(int64_t nch) { return nch > RES_MAX_CHUNKS ? 0 : 7
 // the other waits for.  Another solve takes the launches meanwhile.
 std::mutex g_res_mutex[128];
 
-// Systems not done (one block).
-__global__ void k_count_active(Seg S) {
-  __shared__ int n;
-  if (threadIdx.x == 0) n = 0;
-  __syncthreads();
-  for (int g = threadIdx.x; g < S.nseg; g += blockDim.x)
-    if (!S.st[g].done) atomicAdd(&n, 1);
-  __syncthreads();
-  if (threadIdx.x == 0) *S.active = n;
-}
+// What became of a resident CG: nothing was launched, every system is
+// finished, or a wait ran out.  In the last case neither x nor the states hold
+// anything (a CTA leaves its last meeting alone, so one of a system's CTAs may
+// have written its part of x, and the first one the state, where another gave
+// up): the solve starts over from its first iteration.
+enum class Resident { SKIPPED, DONE, ABANDONED };
 
 template <int P, int T, bool HALO>
 int launch_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const double *r, const double *z, double *u,
                     double *c, double *xw, const double *pinv, const uint8_t *fixed, int precond, unsigned long long *sync,
-                    bool *done) {
+                    Resident *out) {
   const llf_pattern *pat = m->pat;
   const int64_t nch = S.nchunks;
   cudaStream_t s = ctx->stream;
@@ -1708,7 +1708,7 @@ int launch_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const doubl
   const size_t fixed_b = res_smem_fixed<P>(), room = (size_t)(216 * 1024) / (1024 / T);
   // row nodes that do not fit on average leave no room for a halo
   if (HALO && fixed_b + sizeof(int) * (size_t)(pat->nnzb / nch) > room)
-    return launch_resident<P, T, false>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, done);
+    return launch_resident<P, T, false>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, out);
   const int adj_cap = (int)std::min<int64_t>((int64_t)(CHUNK / P) * std::max(pat->max_deg, 1),
                                              (int64_t)((room - fixed_b) / sizeof(int)));
   const size_t smem = HALO ? room : fixed_b + sizeof(int) * (size_t)adj_cap;
@@ -1722,7 +1722,11 @@ int launch_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const doubl
   const int64_t sq = nch * nch;
   const char *lim = getenv("LLF_RESIDENT_WAIT_NS");   // tests: 0 makes the waits run out
   const unsigned long long limit = lim ? strtoull(lim, nullptr, 10) : RES_LIMIT_NS;
-  ResSync Y{pairs, pairs + sq, pairs + 2 * sq, sync + 6 * sq, reinterpret_cast<unsigned *>(sync + 7 * sq), limit};
+  long long quit_chunk = -1, quit_it = 0;
+  if (const char *quit = getenv("LLF_RESIDENT_GIVE_UP"))   // tests: "chunk,iteration" whose CTA gives up
+    if (sscanf(quit, "%lld,%lld", &quit_chunk, &quit_it) != 2) quit_chunk = -1;
+  ResSync Y{pairs, pairs + sq, pairs + 2 * sq, sync + 6 * sq, reinterpret_cast<unsigned *>(sync + 7 * sq), limit,
+            quit_chunk, (unsigned long long)quit_it};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;
   at[0].val.cooperative = 1;
@@ -1742,18 +1746,16 @@ int launch_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const doubl
       return LLF_OK;
     }
   }
+  *out = Resident::ABANDONED;
   unsigned aborted = 1;
   LLF_CUDA_TRY(ctx, cudaMemcpyAsync(&aborted, Y.abort, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   LLF_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+  // no wait ran out: the systems that had room are finished, the others untouched
   if (HALO && aborted == RES_NO_ROOM)
-    return launch_resident<P, T, false>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, done);
-  *done = aborted == 0;
-  if (*done) {
+    return launch_resident<P, T, false>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, out);
+  if (aborted == 0) {
+    *out = Resident::DONE;
     LLF_CUDA_TRY(ctx, cudaMemsetAsync(S.active, 0, sizeof(int), s));
-  } else {   // the launches start from the first direction; systems that finished stay done
-    LLF_CUDA_TRY(ctx, cudaMemsetAsync(u, 0, sizeof(double) * pat->ndof, s));
-    k_count_active<<<1, CG_THREADS, 0, s>>>(S);
-    LLF_CUDA_TRY(ctx, cudaGetLastError());
   }
   return LLF_OK;
 }
@@ -1769,12 +1771,12 @@ int launch_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const doubl
 // to 1.3 times and not twice the same, of 137 to 320 MB 0.6 to 0.8 times (hex8
 // 41^3 49 and 66 ms): those stream from HBM, and the launches keep more loads
 // under way.  Four CTAs of 256 threads were 0.8 to 1.1 times as fast.
-// *done = false: the caller runs the launches.
+// Unless *out is DONE the caller runs the launches.
 template <int P>
 int run_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const double *r, const double *z, double *u,
                  double *c, double *xw, const double *pinv, const uint8_t *fixed, int precond, unsigned long long *sync,
-                 bool *done) {
-  *done = false;
+                 Resident *out) {
+  *out = Resident::SKIPPED;
   const int64_t nch = S.nchunks;
   if (nch < 1 || nch > std::min<int64_t>(2 * ctx->num_sms, RES_MAX_CHUNKS) || ctx->shares_gpu || ctx->device < 0 || ctx->device >= 128)
     return LLF_OK;
@@ -1786,8 +1788,8 @@ int run_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const double *
   std::unique_lock<std::mutex> lock(g_res_mutex[ctx->device], std::try_to_lock);
   if (!lock.owns_lock()) return LLF_OK;
   if (nch <= ctx->num_sms)
-    return launch_resident<P, 1024, true>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, done);
-  return launch_resident<P, 512, true>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, done);
+    return launch_resident<P, 1024, true>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, out);
+  return launch_resident<P, 512, true>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, out);
 }
 
 // Buffers, chunking and preconditioner of the segmented PCG for one matrix
@@ -1958,18 +1960,28 @@ int pcg_core(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double *d_x, 
     k_precond_setup<P><<<(unsigned)((pat->mesh->non + 127) / 128), 128, 0, s>>>(
         m->d_nz, kept_cols(m), pat->d_colptr, pat->d_diagpos, d_fixed, pat->mesh->non, precond, pinv);
   }
-  { KernelScope k(ctx, "k_keep_fixed"); k_keep_fixed<<<gv, CG_THREADS, 0, s>>>(d_x, d_fixed, xw, n); }
-  launch_spmv<P>(ctx, m, xw, c);
-  { KernelScope k(ctx, "k_seg_init"); k_seg_init<<<gch, CG_THREADS, 0, s>>>(S, d_b, c, d_fixed, r, xw, u, part); }
-  { KernelScope k(ctx, "k_seg_start"); k_seg_start<<<gseg, CG_THREADS, 0, s>>>(S, part, reltol, (long long)maxiter); }
-  enqueue_first_prec<P>(ctx, S, m, pinv, precond, r, z, d_fixed, part, gch, gseg, ic);
-  LLF_CUDA_TRY(ctx, cudaGetLastError());
+  auto start = [&]() -> int {   // r, z, u, x and the states before the first iteration
+    { KernelScope k(ctx, "k_keep_fixed"); k_keep_fixed<<<gv, CG_THREADS, 0, s>>>(d_x, d_fixed, xw, n); }
+    launch_spmv<P>(ctx, m, xw, c);
+    { KernelScope k(ctx, "k_seg_init"); k_seg_init<<<gch, CG_THREADS, 0, s>>>(S, d_b, c, d_fixed, r, xw, u, part); }
+    { KernelScope k(ctx, "k_seg_start"); k_seg_start<<<gseg, CG_THREADS, 0, s>>>(S, part, reltol, (long long)maxiter); }
+    enqueue_first_prec<P>(ctx, S, m, pinv, precond, r, z, d_fixed, part, gch, gseg, ic);
+    LLF_CUDA_TRY(ctx, cudaGetLastError());
+    return LLF_OK;
+  };
+  int rc = start();
+  if (rc != LLF_OK) return rc;
 
   if (sync && precond != LLF_PRECOND_IC0) {
-    bool done = false;
-    const int rc = run_resident<P>(ctx, m, S, r, z, u, c, xw, pinv, d_fixed, precond, sync, &done);
+    Resident out = Resident::SKIPPED;
+    rc = run_resident<P>(ctx, m, S, r, z, u, c, xw, pinv, d_fixed, precond, sync, &out);
     if (rc != LLF_OK) return rc;
-    if (done) {
+    if (out == Resident::ABANDONED) {
+      LLF_CUDA_TRY(ctx, cudaMemsetAsync(d_active, 0, sizeof(int), s));
+      rc = start();
+      if (rc != LLF_OK) return rc;
+    }
+    if (out == Resident::DONE) {
       { KernelScope k(ctx, "k_cg_merge"); k_cg_merge<<<gv, CG_THREADS, 0, s>>>(xw, d_fixed, d_x, n); }
       LLF_CUDA_TRY(ctx, cudaGetLastError());
       LLF_CUDA_TRY(ctx, cudaMemcpyAsync(hst, S.st, sizeof(SegState) * nseg, cudaMemcpyDeviceToHost, s));
