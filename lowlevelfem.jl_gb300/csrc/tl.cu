@@ -26,6 +26,11 @@ constexpr int TLP_THREADS = 384;  // most threads of k_tl_packed: hex27's 378 no
 // per-point record: wq, invJ[9], F or S [9], D[36], S[9] (tangent); an odd
 // stride, so that the threads of the point phase write to different banks
 constexpr int QD = 65;
+// k_tl_matrix's stride: with 65 doubles a hex125 element takes 116 KB instead of
+// 115, and one CTA fits on an SM instead of two (216 elements 75 instead of 60
+// ms); its point phase is a small part.  The limits on an element's size are
+// those of this stride.
+constexpr int QM = 64;
 constexpr int QF = 19;  // the internal force's record: wq, invJ[9], P[9]
 // TL_FORCE: F in, first Piola-Kirchhoff stress out (internal force)
 enum { TL_KMAT = 0, TL_KGEO_S = 1, TL_KGEO_C = 2, TL_KTAN = 3, TL_FORCE = 4 };
@@ -256,8 +261,8 @@ __global__ void __launch_bounds__(TL_THREADS) k_tl_matrix(TLArgs A) {
   const int npe = A.npe, nip = A.nip;
   double *sX = sm;                         // npe*3
   double *sT = sX + npe * 3;               // npe*9
-  double *qd = sT + npe * 9;               // nip*QD
-  double *sG = qd + (size_t)nip * QD;      // npe*3
+  double *qd = sT + npe * 9;               // nip*QM
+  double *sG = qd + (size_t)nip * QM;      // npe*3
   double *sB = sG + npe * 3;               // npe*18
   double *sTb = sB + npe * 18;             // npe*18 (KMAT)
   constexpr bool MAT = (MODE == TL_KMAT || MODE == TL_KTAN);
@@ -268,7 +273,7 @@ __global__ void __launch_bounds__(TL_THREADS) k_tl_matrix(TLArgs A) {
       sX[t] = A.xyz[(size_t)A.conn[e * npe + t / 3] * 3 + t % 3];
     for (int t = threadIdx.x; t < npe * 9; t += blockDim.x) sT[t] = A.T[(size_t)e * npe * 9 + t];
     __syncthreads();
-    for (int q = threadIdx.x; q < nip; q += blockDim.x) tl_point<MODE>(A, q, sX, sT, qd + (size_t)q * QD);
+    for (int q = threadIdx.x; q < nip; q += blockDim.x) tl_point<MODE>(A, q, sX, sT, qd + (size_t)q * QM);
     __syncthreads();
     double *Ke = A.out + (size_t)e * npe * npe * BS;  // [column node][row node][block]
     const int tile = blockDim.x * PPT;
@@ -279,7 +284,7 @@ __global__ void __launch_bounds__(TL_THREADS) k_tl_matrix(TLArgs A) {
 #pragma unroll
         for (int m = 0; m < BS; ++m) acc[k][m] = 0.0;
       for (int q = 0; q < nip; ++q) {
-        const double *rec = qd + (size_t)q * QD;
+        const double *rec = qd + (size_t)q * QM;
         // physical gradients of all nodes at q
         for (int t = threadIdx.x; t < npe * 3; t += blockDim.x) {
           int a = t / 3, i = t % 3;
@@ -958,7 +963,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) k_tl_tangent_tc(TcArgs A) {
 }
 
 size_t tl_smem(int npe, int nip) {
-  return sizeof(double) * ((size_t)npe * 12 + (size_t)nip * QD + (size_t)npe * 39);
+  return sizeof(double) * ((size_t)npe * 12 + (size_t)nip * QM + (size_t)npe * 39);
 }
 
 int fill_args(llf_ctx *ctx, llf_mesh *mesh, const double *T, int law, const double *params,
@@ -1154,8 +1159,9 @@ int tl_tangent_tc_impl(llf_ctx *ctx, llf_mesh *mesh, llf_pattern *pat, const dou
   LLF_CUDA_TRY(ctx, dalloc(ctx, &cnt, pat->ndof + 1));
   LLF_CUDA_TRY(ctx, cudaMemsetAsync(cnt, 0, sizeof(int64_t) * (pat->ndof + 1), s));
   {
-    const size_t smem = sizeof(double) * ((size_t)npe * 12 + (size_t)nip * QD);
-    if (smem > 200 * 1024) rc = llf_fail(ctx, LLF_ERR_LIMIT, "tensor-core tangent: element too large");
+    const size_t smem = sizeof(double) * ((size_t)npe * 12 + (size_t)nip * QD);   // 203 KB at most
+    if (sizeof(double) * ((size_t)npe * 12 + (size_t)nip * QM) > 200 * 1024)
+      rc = llf_fail(ctx, LLF_ERR_LIMIT, "tensor-core tangent: element too large");
     if (rc == LLF_OK && smem > 48 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(k_tl_points_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) rc = llf_fail(ctx, LLF_ERR_CUDA, cudaGetErrorString(e));
