@@ -541,10 +541,11 @@ __global__ void __launch_bounds__(TLP_THREADS, 2) k_tl_packed(TLArgs A, int E) {
 // Internal force: element vectors fe[e][a][i], E elements per CTA (the
 // points of small elements fill whole warps: hex8 took 8 lanes of 128 one
 // element at a time).  A point's record holds only w, J^-1 and P, and a
-// thread makes the three components of a node, so that the node's physical
-// gradient is formed once per point.  hex8, 29,760 elements: 1.49 -> 0.25 ms;
-// hex125, 576 elements: 1.46 -> 0.68 ms.
-template <int MODE>  // TL_FORCE: T = F with law, TL_KGEO_S: T = P
+// thread makes NC components of a node: all three, so that the node's physical
+// gradient is formed once per point (hex8, 29,760 elements: 1.49 -> 0.25 ms;
+// hex125, 576 elements: 1.46 -> 0.68 ms), or one on meshes of few CTAs, where
+// its longest chain is what counts.
+template <int MODE, int NC>  // TL_FORCE: T = F with law, TL_KGEO_S: T = P
 __global__ void __launch_bounds__(TL_THREADS) k_tl_force(TLArgs A, int E) {
   extern __shared__ double sm[];
   const int npe = A.npe, nip = A.nip;
@@ -562,9 +563,10 @@ __global__ void __launch_bounds__(TL_THREADS) k_tl_force(TLArgs A, int E) {
       tl_point<MODE>(A, t - k * nip, sX + (size_t)k * npe * 3, sT + (size_t)k * npe * 9, qd + (size_t)t * QF);
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < ne * npe; t += blockDim.x) {
-      const int k = t / npe, a = t - k * npe;
-      double fe[3] = {0.0, 0.0, 0.0};
+    constexpr int NT = 3 / NC;   // threads per node
+    for (int t = threadIdx.x; t < ne * npe * NT; t += blockDim.x) {
+      const int n = t / NT, k = n / npe, a = n - k * npe, i0 = t - n * NT;
+      double fe[NC] = {};
       for (int q = 0; q < nip; ++q) {
         const double *rec = qd + ((size_t)k * nip + q) * QF;
         const double *d = A.dN + ((size_t)q * npe + a) * 3;
@@ -574,14 +576,14 @@ __global__ void __launch_bounds__(TL_THREADS) k_tl_force(TLArgs A, int E) {
         for (int c = 0; c < 3; ++c)
           g[c] = __fma_rn(rec[7 + c], d2, __fma_rn(rec[4 + c], d1, __fma_rn(rec[1 + c], d0, 0.0)));
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          const double *P = rec + 10 + 3 * i;
+        for (int i = 0; i < NC; ++i) {
+          const double *P = rec + 10 + 3 * (i0 + i);
           const double v = __fma_rn(P[2], g[2], __fma_rn(P[1], g[1], __fma_rn(P[0], g[0], 0.0)));
           fe[i] = __fma_rn(v, rec[0], fe[i]);
         }
       }
 #pragma unroll
-      for (int i = 0; i < 3; ++i) A.out[((size_t)e0 * npe + t) * 3 + i] = fe[i];
+      for (int i = 0; i < NC; ++i) A.out[((size_t)e0 * npe + n) * 3 + i0 + i] = fe[i];
     }
     __syncthreads();
   }
@@ -995,8 +997,10 @@ int fill_args(llf_ctx *ctx, llf_mesh *mesh, const double *T, int law, const doub
 
 // Elements per CTA of k_tl_packed: the count whose node pairs fill their
 // warps best within TLP_THREADS threads and 110 KB of shared memory (two
-// CTAs per SM), the larger one of equals; 0 when one element does not fit.
-int packed_elements(const TLArgs &a, size_t per_elem) {
+// CTAs per SM), the larger one of equals; 0 when one element does not fit.  A
+// mesh that would leave SMs idle puts fewer in a CTA (216 hex8: 94 us with ten
+// in each of 22 CTAs).
+int packed_elements(const TLArgs &a, size_t per_elem, int sms) {
   int best = 0;
   double fill = 0.0;
   for (int E = 1; E * a.npairs <= TLP_THREADS && E * per_elem <= 110 * 1024; ++E) {
@@ -1006,7 +1010,7 @@ int packed_elements(const TLArgs &a, size_t per_elem) {
       best = E;
     }
   }
-  return best;
+  return (int)std::min<int64_t>(best, std::max<int64_t>(1, (a.nel + sms - 1) / sms));
 }
 
 template <int MODE>
@@ -1014,7 +1018,7 @@ int launch_matrix(llf_ctx *ctx, TLArgs a, size_t smem) {
   const char *name = MODE == TL_KMAT ? "k_tl_material" : (MODE == TL_KTAN ? "k_tl_tangent" : "k_tl_geometric");
   const size_t per_elem = sizeof(double) * ((size_t)a.npe * 3 + (size_t)a.nip * QD + (size_t)a.nip * a.npe * 3 +
                                             (size_t)a.npe * 39);
-  if (const int E = packed_elements(a, per_elem)) {
+  if (const int E = packed_elements(a, per_elem, ctx->num_sms)) {
     auto fn = k_tl_packed<MODE>;
     const size_t sp = E * per_elem;
     const int threads = (E * a.npairs + 31) / 32 * 32;
@@ -1247,10 +1251,16 @@ int tl_internal_force_impl(llf_ctx *ctx, llf_mesh *mesh, const double *d_P, cons
     rc = fill_args(ctx, mesh, d_F, law, params, nparams, a);
   }
   if (rc) return rc;
-  // elements per CTA: as many as fill the CTA's threads with points and nodes
+  // elements per CTA: as many as fill the CTA's threads with points and nodes,
+  // or, where that leaves at most two CTAs per SM, with points and node
+  // components in one round (48 tet35: 152 and 115 us, 64 hex27 65 and 53, 216
+  // hex8 35 and 28; with more CTAs the repeated gradients cost more than the
+  // shorter chain saves: 512 hex27 65 and 82)
   const size_t per_elem = sizeof(double) * ((size_t)mesh->npe * 12 + (size_t)mesh->nip * QF);
-  const int E = std::max(1, std::min<int>(TL_THREADS / std::max(mesh->npe, mesh->nip),
-                                          (int)((100 * 1024) / per_elem)));
+  const int fit = (int)((100 * 1024) / per_elem);
+  const int E1 = std::max(1, std::min(TL_THREADS / std::max(3 * mesh->npe, mesh->nip), fit));
+  const bool few = 3 * mesh->npe <= TL_THREADS && (mesh->nel + E1 - 1) / E1 <= 2 * (int64_t)ctx->num_sms;
+  const int E = few ? E1 : std::max(1, std::min(TL_THREADS / std::max(mesh->npe, mesh->nip), fit));
   const size_t smem = E * per_elem;
   if (smem > 200 * 1024) return llf_fail(ctx, LLF_ERR_LIMIT, "element too large for the TL kernels");
   double *fe = nullptr;
@@ -1268,7 +1278,10 @@ int tl_internal_force_impl(llf_ctx *ctx, llf_mesh *mesh, const double *d_P, cons
     LLF_CUDA_TRY(ctx, cudaGetLastError());
     return LLF_OK;
   };
-  rc = d_P ? go(k_tl_force<TL_KGEO_S>) : go(k_tl_force<TL_FORCE>);
+  if (few)
+    rc = d_P ? go(k_tl_force<TL_KGEO_S, 1>) : go(k_tl_force<TL_FORCE, 1>);
+  else
+    rc = d_P ? go(k_tl_force<TL_KGEO_S, 3>) : go(k_tl_force<TL_FORCE, 3>);
   if (rc == LLF_OK) {
     LLF_CUDA_TRY(ctx, cudaMemsetAsync(d_f, 0, sizeof(double) * 3 * mesh->non, ctx->stream));
     rc = node_gather(ctx, mesh->d_conn, mesh->nel, mesh->npe, mesh->non, 3, fe, d_f);

@@ -49,3 +49,24 @@ def test_largest_rules(llf, orc):
     want = llf.tangentMatrix(p, F, params=PRM, precision="tf32x3")
     for a, b in zip(Kt.csc(), want.csc()):
         assert np.array_equal(a, b)
+
+
+# meshes of one element per CTA, of fewer than a full CTA holds and of full
+# CTAs; internal force with a thread per component (at most two CTAs per SM)
+# and per node
+@pytest.mark.parametrize("cells,order,simplex", [((1, 1, 1), 1, False), ((8, 7, 6), 1, False), ((13, 12, 11), 1, False),
+                                                 ((14, 13, 13), 1, False), ((1, 1, 1), 1, True), ((8, 7, 7), 1, True),
+                                                 ((4, 3, 2), 2, True), ((5, 6, 7), 2, True), ((3, 3, 2), 2, False),
+                                                 ((7, 7, 7), 2, False), ((2, 1, 1), 4, True), ((5, 4, 3), 3, True)],
+                         ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else str(v))
+def test_elements_per_cta(llf, orc, cells, order, simplex):
+    m, p, F = _problem(llf, cells, order, simplex, 2)
+    rule = llf._lib.builtin_rule(m.family, m.order)
+    f = llf.internalForceVector(p, F=F, energy="NeoHookeCompressible", params=PRM)
+    assert np.array_equal(f.a[:, 0], orc.tl_internal_force(0, m.xyz, m.conn, rule, F.A, orc.LAW_NEOHOOKE, [1.0, 10.0]))
+    P = llf.TensorField(np.random.default_rng(5).standard_normal((m.nel, 9 * m.npe)), p)
+    f = llf.internalForceVector(p, P=P)
+    assert np.array_equal(f.a[:, 0], orc.tl_internal_force(1, m.xyz, m.conn, rule, P.A))
+    K = llf.tangentMatrix(p, F, params=PRM)
+    ref = orc.tl_matrix(3, m.xyz, m.conn, rule, F.A, orc.LAW_NEOHOOKE, [1.0, 10.0])
+    assert_csc_identical(K.csc(), ref.julia(), f"tangent {cells} p{order}")
