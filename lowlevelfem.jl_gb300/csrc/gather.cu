@@ -577,7 +577,12 @@ int run_colgather(llf_ctx *ctx, llf_pattern *pat, const int64_t *n2e_ptr, const 
   if (nv <= 16) LLF_GATHER(16, 1);
   if (rounds == 1) LLF_GATHER(32, 1);
   if (rounds <= 3 && lanes) LLF_GATHER(32, 3);
-  if (rounds <= 8 && lanes) LLF_GATHER(32, 8);
+  // the longest columns are quad25's (100 values) with two components and
+  // hex125's (125) with one, hex27's (243) with three: rounds that no column
+  // needs still cost registers and predicates (quad25, 40,000 elements: 737 us
+  // with eight rounds, 503 with four)
+  constexpr int LONGEST = P <= 2 ? 4 : 8;
+  if (rounds <= LONGEST && lanes) LLF_GATHER(32, LONGEST);
 #undef LLF_GATHER
 #define LLF_WIDE(NT, R) \
   return launch_wide<P, BV, T, NT, R>(ctx, pat, n2e_ptr, n2e, pos, npe, Kf, cs, init, nz, cnt, B0, nB, sp, first_marked)
