@@ -610,9 +610,12 @@ __global__ void k_seg_dir(Seg S, const double *__restrict__ z, double *__restric
 // well, and the partial u.c takes the chunk's DoFs as the update's sums do
 // (thread t: DoFs t, t + 256, t + 512), every lane busy.  The block that brings in a segment's last
 // chunk sums the partials (chunk order) and sets alpha = rho / u.c.
-// Registers as in k_spmv: eight tet10 systems together, 94 -> 87 us a product.
+// Registers as in k_spmv, for every component count (without the bound the
+// compiler keeps two components to 32): eight tet10 systems together 94 -> 87
+// us a product; 60 iterations with IC(0), quad25 with 116,162 DoFs 20.7 -> 17.1
+// ms, hex27 conduction with 226,981 37.0 -> 34.9.
 template <int P, bool KEPT>
-__global__ void __launch_bounds__(CG_THREADS, P == 3 ? 4 : 0)
+__global__ void __launch_bounds__(CG_THREADS, 4)
 k_seg_spmv(Seg S, const double *__restrict__ nz, KeptCols K, const int64_t *__restrict__ nptr,
            const int32_t *__restrict__ nadj, const double *__restrict__ u,
            const uint8_t *__restrict__ fixed, double *__restrict__ c, double *__restrict__ part) {
@@ -2161,9 +2164,11 @@ __global__ void __launch_bounds__(CG_THREADS) k_mx_dir(Seg S, const float *__res
   }
 }
 
-// c = A32 u (masked) and alpha = rho / u.c (u.c in FP64) — k_seg_spmv in FP32.
+// c = A32 u (masked) and alpha = rho / u.c (u.c in FP64) — k_seg_spmv in FP32,
+// with its register allowance: 60 iterations with Jacobi, quad25 with
+// 116,162 DoFs 4.5 -> 2.9 ms, tet10 with 206,763 5.3 -> 3.5.
 template <int P>
-__global__ void __launch_bounds__(CG_THREADS)
+__global__ void __launch_bounds__(CG_THREADS, 4)
 k_mx_spmv(Seg S, const float *__restrict__ nz, const int64_t *__restrict__ nptr, const int32_t *__restrict__ nadj,
           const float *__restrict__ u, const uint8_t *__restrict__ fixed, float *__restrict__ c,
           double *__restrict__ part) {
