@@ -288,19 +288,22 @@ __device__ __forceinline__ void tile_order(const int64_t *__restrict__ nptr, int
 // sums do not depend on the order.  KEPT's POPCs and selects (about 40 issue
 // slots per step) fit beside its P FP64 instructions, which take 64 each of an
 // SM quarter.
-// The second launch bound is a register allowance: with three components the
-// compiler otherwise keeps to 32 registers (56 with KEPT) by placing loads
-// beside their uses, and every load is waited for.  LONG (rows of 512 entries
-// or more, no SORT): eight positions of a lane at once.
-// hex27 40^3 (297.7 M entries), KEPT: 0.845 -> 0.72 by degree -> 0.68 ms with
-// the allowance (the operations take 0.49); tet10, 253,000 nodes 0.213 -> 0.19 ->
-// 0.178; expanding the structural values of the first and multiplying by those
-// took 2.55 + 0.83 ms.  In node
-// order, 128 threads a block so that more rows are under way beside a long
-// one: hex64 0.225 -> 0.189, tet20 0.154 -> 0.133 ms and, structural values and
-// LONG, hex125 with 40,293 nodes 0.425 -> 0.302 ms.
+// The second launch bound is a register allowance: without one the compiler
+// places loads beside their uses (32 registers with one component, by degree;
+// 56 with three and KEPT), and every load is waited for.  LONG (three
+// components, rows of 512 entries or more, no SORT): eight positions of a lane
+// at once.  With one component the two positions of node_columns_at are the
+// better ones for long rows too (hex125 conduction, structural values: LONG
+// 37 us with 9,261 nodes and 60 with 35,937, two positions and the allowance
+// 21 and 39), and by degree the allowance takes 91,125 nodes from 110 to 80 us.
+// KEPT of one or two components is left without: hex8 conduction, 357,911
+// nodes, 38 us and 41 with it.
+// Structural values, us: hex27 40^3 583, hex64 14^3 229, hex125 8^3 273, tet10
+// 24^3 86; KEPT 667, 328, 353, 99.  In node order 128 threads a block, so that
+// more rows are under way beside a long one: 256 threads took 1.04 to 1.09
+// times as long for rows of three components.
 template <int P, bool KEPT, bool SORT, bool LONG>
-__global__ void __launch_bounds__(SORT ? CG_THREADS : 128, P != 3 ? 0 : (SORT ? 3 : (LONG ? 4 : 6)))
+__global__ void __launch_bounds__(SORT ? CG_THREADS : 128, P == 3 ? (SORT ? 3 : (LONG ? 4 : 6)) : (KEPT ? 0 : (SORT ? 5 : 10)))
 k_spmv(const double *__restrict__ nz, KeptCols K, const int64_t *__restrict__ nptr, const int32_t *__restrict__ nadj,
        const double *__restrict__ x, double *__restrict__ y, int64_t non) {
   constexpr int NPW = 32 / SPMV_G, NPB = (SORT ? CG_THREADS : 128) / SPMV_G;  // nodes per warp, per round of a block
@@ -1627,7 +1630,7 @@ void launch_spmv(llf_ctx *ctx, const llf_matrix *m, const double *x, double *y) 
                     4 * (int64_t)m->pat->max_deg * P * P * non > 5 * m->pat->nnz;
   if (m->d_nz) {
     if (sort) launch_spmv_as<P, false, true, false>(ctx, m, x, y);
-    else if (m->pat->max_deg * P >= 512) launch_spmv_as<P, false, false, true>(ctx, m, x, y);
+    else if (P == 3 && m->pat->max_deg * P >= 512) launch_spmv_as<P, false, false, P == 3>(ctx, m, x, y);
     else launch_spmv_as<P, false, false, false>(ctx, m, x, y);
   } else {
     if (sort) launch_spmv_as<P, true, true, false>(ctx, m, x, y);
