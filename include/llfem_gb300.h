@@ -225,8 +225,10 @@ int llf_pattern_destroy(llf_ctx *ctx, llf_pattern *pat);
  * only; its structural values (the solvers' format) are expanded from it on
  * the first call that needs them (llf_pcg*, llf_matrix_copy_structural,
  * llf_matrix_axpby, llf_heat_fdm, or llf_matrix_prepare).  llf_matrix_spmv
- * multiplies by the stored values, and llf_pcg_noalloc refuses such a matrix
- * until llf_matrix_spmv or llf_matrix_prepare has run on it.
+ * multiplies by the stored values three times and expands the structural ones
+ * at the fourth (without memory for them it goes on with the stored values);
+ * llf_pcg_noalloc refuses such a matrix until llf_matrix_spmv or
+ * llf_matrix_prepare has run on it.
  * LLF_STORED_LAYOUT=0 in the environment turns the reuse off.  Not used for
  * lumped mass matrices, nor for assemblies that accumulate into a matrix. */
 
@@ -560,7 +562,9 @@ int llf_heat_fdm(llf_ctx *ctx, const llf_matrix *K, const llf_matrix *C,
  * serialise them.  The matrix's structural values must be resident (see
  * llf_matrix_prepare), or a product (llf_matrix_spmv) must have run on it;
  * another matrix that holds its stored CSC only is refused with
- * LLF_ERR_STATE. */
+ * LLF_ERR_STATE.  After a product alone the iterations take the stored
+ * values, whose products last up to twice as long (long scalar rows):
+ * llf_matrix_prepare is the better preparation. */
 int llf_pcg_noalloc(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double *d_x,
                     const uint8_t *d_fixed, int precond, double reltol, int64_t maxiter,
                     int64_t *iters, double *relres);

@@ -1205,12 +1205,16 @@ int matrix_ensure_nz(llf_ctx *ctx, const llf_matrix *cm) {
   if (m->d_nz || m->diagonal_only) return LLF_OK;
   if (!m->d_colptr_s || !m->d_keep)
     return llf_fail(ctx, LLF_ERR_STATE, "matrix has neither structural nor stored values");
-  llf_pattern *pat = m->pat;
+  return matrix_expand_nz(ctx, m, &m->d_nz);
+}
+
+int matrix_expand_nz(llf_ctx *ctx, const llf_matrix *m, double **nz) {
+  const llf_pattern *pat = m->pat;
   const int64_t n = pat->ndof;
-  LLF_CUDA_TRY(ctx, dalloc(ctx, &m->d_nz, pat->nnz > 0 ? pat->nnz : 1));
+  LLF_CUDA_TRY(ctx, dalloc(ctx, nz, pat->nnz > 0 ? pat->nnz : 1));
   KernelScope ks(ctx, "k_expand_nz");
   k_expand_nz<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 7) / 8, (int64_t)1 << 30)), 256, 0, ctx->stream>>>(
-      pat->d_colptr, n, m->d_colptr_s, m->d_nzval_s, m->d_keep, m->d_nz);
+      pat->d_colptr, n, m->d_colptr_s, m->d_nzval_s, m->d_keep, *nz);
   LLF_CUDA_TRY(ctx, cudaGetLastError());
   return LLF_OK;
 }

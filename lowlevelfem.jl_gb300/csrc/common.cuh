@@ -214,9 +214,10 @@ struct llf_matrix {
   // pair of words per 64 entries at keep_pos(s, c): entries 0..31 in word x,
   // 32..63 in word y.
   uint2 *d_keep = nullptr;
-  // a product has run: llf_pcg_noalloc takes the matrix, from the stored
-  // values where the structural ones are not expanded
-  mutable std::atomic<bool> multiplied{false};
+  // products that have run.  From the first on llf_pcg_noalloc takes the
+  // matrix, from the stored values where the structural ones are not expanded
+  mutable std::atomic<long long> products{0};
+  mutable std::atomic<bool> expanding{false};   // a product has set out to expand the structural values
 };
 
 // First keep word pair of column c, whose structural entries start at s, and
@@ -316,6 +317,8 @@ void pattern_free_layouts(llf_ctx *ctx, llf_pattern *pat);
 // structural positions, +0.0 at the others.  Allocates; a no-op when they
 // exist.
 int matrix_ensure_nz(llf_ctx *ctx, const llf_matrix *m);
+// The same into an array of its own, allocated here (m holds keep bits).
+int matrix_expand_nz(llf_ctx *ctx, const llf_matrix *m, double **nz);
 // assemble_fp32.cu: precision form (FP32 quadrature, FP64 accumulation) into nz
 // aflag/ageo: per-element affine flag and invJ/det (null: quadrature form
 // only); all_affine: every element in use is affine, so the quadrature

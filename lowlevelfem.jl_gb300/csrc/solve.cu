@@ -1605,36 +1605,43 @@ void enqueue_ic0(llf_ctx *ctx, const Seg &S, const llf_matrix *m, const IcApply 
   { KernelScope k(ctx, "k_seg_zr"); k_seg_zr<<<chunk_grid(S), CG_THREADS, 0, ctx->stream>>>(S, ic.zf, r, z, part); }
 }
 
-KeptCols kept_cols(const llf_matrix *m) {
-  return m->d_nz ? KeptCols{nullptr, nullptr, nullptr} : KeptCols{m->d_nzval_s, m->d_colptr_s, m->d_keep};
+// The values a call multiplies by, read once: a product of another context
+// may publish the structural ones meanwhile.
+struct MatVals {
+  const double *nz;   // null: the stored values
+  KeptCols kept;
+};
+MatVals mat_vals(const llf_matrix *m) {
+  const double *nz = __atomic_load_n(&m->d_nz, __ATOMIC_ACQUIRE);
+  return {nz, nz ? KeptCols{nullptr, nullptr, nullptr} : KeptCols{m->d_nzval_s, m->d_colptr_s, m->d_keep}};
 }
 
 // y = A x, from whichever values the matrix holds.
 template <int P, bool KEPT, bool SORT, bool LONG>
-void launch_spmv_as(llf_ctx *ctx, const llf_matrix *m, const double *x, double *y) {
+void launch_spmv_as(llf_ctx *ctx, const llf_matrix *m, const MatVals &A, const double *x, double *y) {
   const llf_pattern *p = m->pat;
   constexpr int threads = SORT ? CG_THREADS : 128;
   const int64_t non = p->ndof / P, tile = SORT ? SPMV_TILE : threads / SPMV_G;
   const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((non + tile - 1) / tile, 1 << 30));
   KernelScope ks(ctx, KEPT ? "k_spmv_kept" : "k_spmv");
-  k_spmv<P, KEPT, SORT, LONG><<<grid, threads, 0, ctx->stream>>>(m->d_nz, kept_cols(m), p->d_nptr, p->d_nadj, x, y, non);
+  k_spmv<P, KEPT, SORT, LONG><<<grid, threads, 0, ctx->stream>>>(A.nz, A.kept, p->d_nptr, p->d_nadj, x, y, non);
 }
 
 // By degree where that leaves four blocks per SM and the longest row is well
 // above the mean one (quad4 300x300, all alike: 19 us in node order, 21 by
 // degree; tet20 with 20,000 nodes, two blocks per SM: 150 against 164 us).
 template <int P>
-void launch_spmv(llf_ctx *ctx, const llf_matrix *m, const double *x, double *y) {
+void launch_spmv(llf_ctx *ctx, const llf_matrix *m, const MatVals &A, const double *x, double *y) {
   const int64_t non = m->pat->ndof / P;
   const bool sort = non >= (int64_t)SPMV_TILE * 4 * ctx->num_sms &&
                     4 * (int64_t)m->pat->max_deg * P * P * non > 5 * m->pat->nnz;
-  if (m->d_nz) {
-    if (sort) launch_spmv_as<P, false, true, false>(ctx, m, x, y);
-    else if (P == 3 && m->pat->max_deg * P >= 512) launch_spmv_as<P, false, false, P == 3>(ctx, m, x, y);
-    else launch_spmv_as<P, false, false, false>(ctx, m, x, y);
+  if (A.nz) {
+    if (sort) launch_spmv_as<P, false, true, false>(ctx, m, A, x, y);
+    else if (P == 3 && m->pat->max_deg * P >= 512) launch_spmv_as<P, false, false, P == 3>(ctx, m, A, x, y);
+    else launch_spmv_as<P, false, false, false>(ctx, m, A, x, y);
   } else {
-    if (sort) launch_spmv_as<P, true, true, false>(ctx, m, x, y);
-    else launch_spmv_as<P, true, false, false>(ctx, m, x, y);
+    if (sort) launch_spmv_as<P, true, true, false>(ctx, m, A, x, y);
+    else launch_spmv_as<P, true, false, false>(ctx, m, A, x, y);
   }
 }
 
@@ -1657,16 +1664,16 @@ void enqueue_first_prec(llf_ctx *ctx, const Seg &S, const llf_matrix *m, const d
 // updated with the residual check, then the next z and rho (fused for the
 // local preconditioners, the IC(0) sweeps after the update otherwise).
 template <int P>
-void enqueue_iteration(llf_ctx *ctx, const Seg &S, const llf_matrix *m, const double *pinv, int precond,
-                       double *r, double *z, double *u, double *c, double *xw, const uint8_t *fixed,
+void enqueue_iteration(llf_ctx *ctx, const Seg &S, const llf_matrix *m, const MatVals &A, const double *pinv,
+                       int precond, double *r, double *z, double *u, double *c, double *xw, const uint8_t *fixed,
                        double *part, double *part2, double *part3, const IcApply &ic) {
   const llf_pattern *pat = m->pat;
   cudaStream_t s = ctx->stream;
   const bool local = precond != LLF_PRECOND_IC0;
   { KernelScope k(ctx, "k_seg_dir"); k_seg_dir<<<chunk_grid(S), CG_THREADS, 0, s>>>(S, z, u); }
   { KernelScope k(ctx, "k_seg_spmv");
-    auto fn = m->d_nz ? k_seg_spmv<P, false> : k_seg_spmv<P, true>;
-    fn<<<chunk_grid(S), CG_THREADS, 0, s>>>(S, m->d_nz, kept_cols(m), pat->d_nptr, pat->d_nadj, u, fixed, c, part3); }
+    auto fn = A.nz ? k_seg_spmv<P, false> : k_seg_spmv<P, true>;
+    fn<<<chunk_grid(S), CG_THREADS, 0, s>>>(S, A.nz, A.kept, pat->d_nptr, pat->d_nadj, u, fixed, c, part3); }
   { KernelScope k(ctx, "k_seg_update");
     k_seg_update_fused<P><<<chunk_grid(S), CG_THREADS, 0, s>>>(S, xw, r, u, c, part, part2, pinv, precond, local,
                                                                fixed, z); }
@@ -1960,15 +1967,16 @@ int pcg_core(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double *d_x, 
   const unsigned gch = (unsigned)std::max<int64_t>(1, std::min<int64_t>(nch, (int64_t)ctx->num_sms * 8));
   const unsigned gseg = (unsigned)std::max(1, std::min(nseg, ctx->num_sms * 8));
   const unsigned gv = (unsigned)(ctx->num_sms * 4);
+  const MatVals A = mat_vals(m);
 
   if (precond != LLF_PRECOND_IC0) {
     KernelScope k(ctx, "k_precond_setup");
     k_precond_setup<P><<<(unsigned)((pat->mesh->non + 127) / 128), 128, 0, s>>>(
-        m->d_nz, kept_cols(m), pat->d_colptr, pat->d_diagpos, d_fixed, pat->mesh->non, precond, pinv);
+        A.nz, A.kept, pat->d_colptr, pat->d_diagpos, d_fixed, pat->mesh->non, precond, pinv);
   }
   auto start = [&]() -> int {   // r, z, u, x and the states before the first iteration
     { KernelScope k(ctx, "k_keep_fixed"); k_keep_fixed<<<gv, CG_THREADS, 0, s>>>(d_x, d_fixed, xw, n); }
-    launch_spmv<P>(ctx, m, xw, c);
+    launch_spmv<P>(ctx, m, A, xw, c);
     { KernelScope k(ctx, "k_seg_init"); k_seg_init<<<gch, CG_THREADS, 0, s>>>(S, d_b, c, d_fixed, r, xw, u, part); }
     { KernelScope k(ctx, "k_seg_start"); k_seg_start<<<gseg, CG_THREADS, 0, s>>>(S, part, reltol, (long long)maxiter); }
     enqueue_first_prec<P>(ctx, S, m, pinv, precond, r, z, d_fixed, part, gch, gseg, ic);
@@ -2005,7 +2013,8 @@ int pcg_core(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double *d_x, 
     cudaGraph_t graph = nullptr;
     if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
       const long long saved = ctx->launches;
-      for (int k = 0; k < per_graph; ++k) enqueue_iteration<P>(ctx, S, m, pinv, precond, r, z, u, c, xw, d_fixed, part, part2, part3, ic);
+      for (int k = 0; k < per_graph; ++k)
+        enqueue_iteration<P>(ctx, S, m, A, pinv, precond, r, z, u, c, xw, d_fixed, part, part2, part3, ic);
       launches_per_graph = ctx->launches - saved;
       ctx->launches = saved;
       if (cudaStreamEndCapture(s, &graph) != cudaSuccess ||
@@ -2024,7 +2033,8 @@ int pcg_core(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double *d_x, 
       LLF_CUDA_TRY(ctx, cudaGraphLaunch(exec, s));
       ctx->launches += launches_per_graph;
     } else {
-      for (int k = 0; k < per_graph; ++k) enqueue_iteration<P>(ctx, S, m, pinv, precond, r, z, u, c, xw, d_fixed, part, part2, part3, ic);
+      for (int k = 0; k < per_graph; ++k)
+        enqueue_iteration<P>(ctx, S, m, A, pinv, precond, r, z, u, c, xw, d_fixed, part, part2, part3, ic);
     }
     LLF_CUDA_TRY(ctx, cudaGetLastError());
     LLF_CUDA_TRY(ctx, cudaMemcpyAsync(h_active, d_active, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -2426,12 +2436,12 @@ int pcg_mixed_core(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double 
   if (local) {
     KernelScope k(ctx, "k_precond_setup");
     k_precond_setup<P><<<(unsigned)((pat->mesh->non + 127) / 128), 128, 0, s>>>(
-        m->d_nz, kept_cols(m), pat->d_colptr, pat->d_diagpos, d_fixed, pat->mesh->non, precond, pinv);
+        m->d_nz, KeptCols{}, pat->d_colptr, pat->d_diagpos, d_fixed, pat->mesh->non, precond, pinv);
   }
   { KernelScope k(ctx, "k_f64_to_f32");
     k_f64_to_f32<<<(unsigned)(ctx->num_sms * 8), CG_THREADS, 0, s>>>(m->d_nz, B.nz32, pat->nnz); }
   { KernelScope k(ctx, "k_keep_fixed"); k_keep_fixed<<<gv, CG_THREADS, 0, s>>>(d_x, d_fixed, xw, n); }
-  launch_spmv<P>(ctx, m, xw, tmp);
+  launch_spmv<P>(ctx, m, mat_vals(m), xw, tmp);
   { KernelScope k(ctx, "k_mx_init"); k_mx_init<<<gch, CG_THREADS, 0, s>>>(S, d_b, tmp, d_fixed, B.rb, B.r, xw, B.u, part); }
   { KernelScope k(ctx, "k_seg_start"); k_seg_start<<<gseg, CG_THREADS, 0, s>>>(S, part, reltol, (long long)maxiter); }
   if (local) {
@@ -2630,7 +2640,7 @@ int pcg_noalloc_typed(llf_ctx *ctx, const llf_matrix *m, const double *d_b, doub
 int pcg_noalloc_impl(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double *d_x,
                      const uint8_t *d_fixed, int precond, double reltol, int64_t maxiter,
                      int64_t *iters, double *relres) {
-  if (!m->d_nz && !m->diagonal_only && !(m->d_keep && m->multiplied.load()))
+  if (!m->d_nz && !m->diagonal_only && !(m->d_keep && m->products.load() > 0))
     return llf_fail(ctx, LLF_ERR_STATE,
                     "llf_pcg_noalloc: the matrix's structural values are not expanded yet (its assembly wrote the "
                     "stored CSC only); run llf_pcg or llf_matrix_spmv on it once first");
@@ -2650,11 +2660,15 @@ int pcg_noalloc_impl(llf_ctx *ctx, const llf_matrix *m, const double *d_b, doubl
   return llf_fail(ctx, LLF_ERR_UNSUPPORTED, "pdim must be 1, 2 or 3");
 }
 
-namespace {
-// One warp per eight column nodes, one round of them per warp, so that the
-// block scheduler balances the nodes' uneven lists (hex27 40^3: 1.00 -> 0.93
-// ms, from the kept values 1.31 -> 0.97 ms, against four blocks per SM).
-}  // namespace
+// A matrix that holds its stored CSC only is multiplied by its stored values
+// KEPT_PRODUCTS times; the next product expands its structural values, which
+// the products from then on take.  The stored values save the expansion (hex27
+// 40^3: 0.91 ms beside a product of 0.67) where a matrix is multiplied once or a
+// few times, as an operator assembled anew every step is, but most products
+// are slower by them (hex125 conduction, 35,937 nodes, 84 and 39 us; hex8
+// stiffness, 206,763 DoFs, 48 and 42), and an expansion costs about as much as
+// one to three products.
+constexpr int KEPT_PRODUCTS = 3;
 
 int spmv_impl(llf_ctx *ctx, const llf_matrix *m, const double *d_x, double *d_y) {
   const int64_t n = m->pat->ndof;
@@ -2667,15 +2681,28 @@ int spmv_impl(llf_ctx *ctx, const llf_matrix *m, const double *d_x, double *d_y)
       const int rc = matrix_ensure_nz(ctx, m);   // reports the missing values
       if (rc != LLF_OK) return rc;
     }
+    if (!mat_vals(m).nz && m->products.load() >= KEPT_PRODUCTS && !m->expanding.exchange(true)) {
+      // complete before they are published: another context may multiply by m
+      double *nz = nullptr, *none = nullptr;
+      if (matrix_expand_nz(ctx, m, &nz) != LLF_OK || cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+        dfree(ctx, nz);   // no room for them: the stored values still serve
+        cudaGetLastError();
+        llf_ok(ctx);
+      } else if (!__atomic_compare_exchange_n(&const_cast<llf_matrix *>(m)->d_nz, &none, nz, false, __ATOMIC_ACQ_REL,
+                                              __ATOMIC_ACQUIRE)) {
+        dfree(ctx, nz);   // a solve expanded them meanwhile
+      }
+    }
+    const MatVals A = mat_vals(m);
     switch (m->pat->pdim) {
-      case 1: launch_spmv<1>(ctx, m, d_x, d_y); break;
-      case 2: launch_spmv<2>(ctx, m, d_x, d_y); break;
-      case 3: launch_spmv<3>(ctx, m, d_x, d_y); break;
+      case 1: launch_spmv<1>(ctx, m, A, d_x, d_y); break;
+      case 2: launch_spmv<2>(ctx, m, A, d_x, d_y); break;
+      case 3: launch_spmv<3>(ctx, m, A, d_x, d_y); break;
       default: return llf_fail(ctx, LLF_ERR_UNSUPPORTED, "pdim must be 1, 2 or 3");
     }
   }
   LLF_CUDA_TRY(ctx, cudaGetLastError());
-  m->multiplied.store(true);
+  m->products.fetch_add(1);
   return LLF_OK;
 }
 
@@ -3141,10 +3168,10 @@ int prepare_t(llf_ctx *ctx, const llf_matrix *K, const double *hb, const double 
     k_chunk_perm<<<chunk_grid(S), CG_THREADS, 0, s>>>(S, pat->d_nptr, P, sy->perm);
   }
   { KernelScope k(ctx, "k_precond_setup");
-    k_precond_setup<P><<<(unsigned)((non + 127) / 128), 128, 0, s>>>(K->d_nz, kept_cols(K), pat->d_colptr, pat->d_diagpos, sy->fixed,
+    k_precond_setup<P><<<(unsigned)((non + 127) / 128), 128, 0, s>>>(K->d_nz, KeptCols{}, pat->d_colptr, pat->d_diagpos, sy->fixed,
                                                                      non, precond, sy->pinv); }
   { KernelScope k(ctx, "k_keep_fixed"); k_keep_fixed<<<gv, CG_THREADS, 0, s>>>(sy->x, sy->fixed, sy->xw, n); }
-  launch_spmv<P>(ctx, K, sy->xw, sy->c);
+  launch_spmv<P>(ctx, K, mat_vals(K), sy->xw, sy->c);
   { KernelScope k(ctx, "k_seg_init"); k_seg_init<<<gch, CG_THREADS, 0, s>>>(S, sy->b, sy->c, sy->fixed, sy->r, sy->xw, sy->u, part); }
   { KernelScope k(ctx, "k_seg_start"); k_seg_start<<<1, CG_THREADS, 0, s>>>(S, part, reltol, (long long)maxiter); }
   { KernelScope k(ctx, "k_seg_prec"); k_seg_prec<P><<<gch, CG_THREADS, 0, s>>>(S, sy->pinv, precond, sy->r, sy->fixed, sy->z, part); }
