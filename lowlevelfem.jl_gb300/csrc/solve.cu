@@ -1751,7 +1751,7 @@ int launch_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const doubl
   cfg.attrs = at;
   cfg.numAttrs = 1;
   {
-    KernelScope k(ctx, "k_cg_resident");
+    KernelScope k(ctx, HALO ? "k_cg_resident" : "k_cg_resident_directions");
     if (cudaLaunchKernelEx(&cfg, fn, S, (const double *)m->d_nz, (const int64_t *)pat->d_nptr,
                            (const int32_t *)pat->d_nadj, fixed, r, z, u, xw, pinv, precond, Y, adj_cap, c, (int)smem) !=
         cudaSuccess) {
