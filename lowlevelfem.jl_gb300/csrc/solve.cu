@@ -1692,11 +1692,10 @@ int pcg_mixed_core(llf_ctx *ctx, const llf_matrix *m, const double *d_b, double 
                    double *part2, double *part3, int precond, double reltol, int64_t maxiter, bool use_graph,
                    SegState *hst, const IcApply &ic);
 
-constexpr int64_t RES_MAX_CHUNKS = 512;
 // Words of the resident CG's meeting points for nch chunks (zeroed before
 // every launch): three word pairs and one word per pair of chunks, and the
-// abort flag; none for a solve that has too many chunks.
-inline int64_t res_sync_words(int64_t nch) { return nch > RES_MAX_CHUNKS ? 0 : 7 * nch * nch + 2; }
+// abort flag.
+inline int64_t res_sync_words(int64_t nch) { return 7 * nch * nch + 2; }
 
 // One resident CG per device at a time: two of them could each hold SMs that
 // the other waits for.  Another solve takes the launches meanwhile.
@@ -1773,7 +1772,8 @@ int launch_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const doubl
   return LLF_OK;
 }
 
-// The resident CG when every chunk gets a CTA at once: one CTA of 1024 threads
+// Whether the resident CG takes a solve of nch chunks with m (its plan then
+// holds the meeting points): every chunk gets a CTA at once, one of 1024 threads
 // per SM (the product's loads then have all the warps an SM holds, whatever
 // the number of chunks), or two of 512 while the values take no more than five
 // eighths of the L2, of which each die holds half and the vectors and row nodes
@@ -1784,23 +1784,24 @@ int launch_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const doubl
 // to 1.3 times and not twice the same, of 137 to 320 MB 0.6 to 0.8 times (hex8
 // 41^3 49 and 66 ms): those stream from HBM, and the launches keep more loads
 // under way.  Four CTAs of 256 threads were 0.8 to 1.1 times as fast.
-// Unless *out is DONE the caller runs the launches.
+bool resident_eligible(const llf_ctx *ctx, const llf_matrix *m, int64_t nch) {
+  if (nch < 1 || nch > 2 * ctx->num_sms || ctx->shares_gpu || ctx->device < 0 || ctx->device >= 128) return false;
+  if (nch <= ctx->num_sms) return true;
+  int l2 = 0;
+  return cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device) == cudaSuccess &&
+         (int64_t)sizeof(double) * m->pat->nnz <= (int64_t)l2 / 8 * 5;
+}
+
+// The resident CG of an eligible solve.  Unless *out is DONE the caller runs
+// the launches.
 template <int P>
 int run_resident(llf_ctx *ctx, const llf_matrix *m, const Seg &S, const double *r, const double *z, double *u,
                  double *c, double *xw, const double *pinv, const uint8_t *fixed, int precond, unsigned long long *sync,
                  Resident *out) {
   *out = Resident::SKIPPED;
-  const int64_t nch = S.nchunks;
-  if (nch < 1 || nch > std::min<int64_t>(2 * ctx->num_sms, RES_MAX_CHUNKS) || ctx->shares_gpu || ctx->device < 0 || ctx->device >= 128)
-    return LLF_OK;
-  if (nch > ctx->num_sms) {
-    int l2 = 0;
-    LLF_CUDA_TRY(ctx, cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device));
-    if ((int64_t)sizeof(double) * m->pat->nnz > (int64_t)l2 / 8 * 5) return LLF_OK;
-  }
   std::unique_lock<std::mutex> lock(g_res_mutex[ctx->device], std::try_to_lock);
   if (!lock.owns_lock()) return LLF_OK;
-  if (nch <= ctx->num_sms)
+  if (S.nchunks <= ctx->num_sms)
     return launch_resident<P, 1024, true>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, out);
   return launch_resident<P, 512, true>(ctx, m, S, r, z, u, c, xw, pinv, fixed, precond, sync, out);
 }
@@ -1820,7 +1821,7 @@ struct PcgPlan {
   double *part2 = nullptr, *part3 = nullptr;
   int *d_arrive = nullptr;
   int16_t *d_perm = nullptr;
-  unsigned long long *d_sync = nullptr;   // resident CG: res_sync_words(nch) words
+  unsigned long long *d_sync = nullptr;   // resident CG, if it may run: res_sync_words(nch) words
   Ic0Factor icf;
   IcApply ic;
   int32_t *d_node_seg = nullptr;
@@ -1875,7 +1876,8 @@ struct PcgPlan {
     LLF_CUDA_TRY(ctx, dalloc(ctx, &part, nch));
     LLF_CUDA_TRY(ctx, dalloc(ctx, &part2, nch));
     LLF_CUDA_TRY(ctx, dalloc(ctx, &part3, nch));
-    if (!mixed && precond != LLF_PRECOND_IC0) LLF_CUDA_TRY(ctx, dalloc(ctx, &d_sync, res_sync_words(nch)));
+    if (!mixed && precond != LLF_PRECOND_IC0 && resident_eligible(ctx, m, nch))
+      LLF_CUDA_TRY(ctx, dalloc(ctx, &d_sync, res_sync_words(nch)));
     LLF_CUDA_TRY(ctx, dalloc(ctx, &d_arrive, 3 * (int64_t)nseg));
     LLF_CUDA_TRY(ctx, cudaMemsetAsync(d_arrive, 0, sizeof(int) * 3 * nseg, s));
     if (nch) {

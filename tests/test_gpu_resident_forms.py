@@ -66,3 +66,15 @@ def test_fallback_runs_the_launches(llf, monkeypatch):
     assert _forms(ctx, solve) == {HALO, LAUNCHES}
     monkeypatch.delenv("LLF_RESIDENT_GIVE_UP")
     assert _forms(ctx, solve) == {HALO}
+
+
+def test_meeting_points_only_where_the_loop_may_run(llf):
+    """A solve with more chunks than the resident CG takes allocates nothing
+    for it: one allocation fewer than a solve that it takes."""
+    count = []
+    for n in (20, 62):
+        ctx, solve = _solve(llf, llf.structured_box_mesh(n=n, order=1), "HeatConduction")
+        a = ctx.allocs()
+        solve()
+        count.append(ctx.allocs() - a)
+    assert count[0] == count[1] + 1
