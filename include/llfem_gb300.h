@@ -115,6 +115,15 @@ int llf_ctx_sync(llf_ctx *ctx);
 /* The stream the context launches on, as a cudaStream_t cast to void*. */
 int llf_ctx_stream(llf_ctx *ctx, void **stream);
 
+/* on != 0: this context's kernels run beside those of other contexts or
+ * programs, and its CG solves keep to launches that leave the GPU to others
+ * between them.  Off (the default), a llf_pcg, llf_pcg_batched or llf_heat_fdm
+ * solve of up to two chunks per SM holds nearly all SMs from its first
+ * iteration to its last, and work of other contexts waits for it to end; it is
+ * up to two and a half times as fast that way, and its results have the same
+ * bits either way.  A server's own contexts share. */
+int llf_ctx_share_gpu(llf_ctx *ctx, int on);
+
 /* Tracing (no counterpart in the reference, which times with @time).
  * Every kernel launch of the context is counted; with profiling enabled,
  * CUDA events bracket each launch on the context stream and the report

@@ -60,6 +60,7 @@ SIGNATURES = {
     "llf_profile_report": (i32, [vp, C.c_char_p, i64, P_i64]),
     "llf_launch_count": (i32, [vp, P_i64]),
     "llf_alloc_count": (i32, [vp, P_i64]),
+    "llf_ctx_share_gpu": (i32, [vp, i32]),
     "llf_mesh_upload": (i32, [vp, i32, i64, P_dbl, i64, i32, P_i64, i32, i32, PP]),
     "llf_mesh_update": (i32, [vp, vp, P_dbl, P_i64]),
     "llf_mesh_set_materials": (i32, [vp, vp, P_i32]),
@@ -191,6 +192,11 @@ class Context:
         s = C.c_void_p()
         self.check(lib().llf_ctx_stream(self.h, C.byref(s)))
         return s.value or 0
+
+    def share_gpu(self, on: bool = True):
+        """Solves of this context leave the GPU to other contexts' work between
+        their launches (llf_ctx_share_gpu)."""
+        self.check(lib().llf_ctx_share_gpu(self.h, int(on)))
 
     def profile(self, on: bool = True):
         self.check(lib().llf_profile_enable(self.h, int(on)))

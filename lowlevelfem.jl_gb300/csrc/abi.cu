@@ -255,6 +255,12 @@ int llf_ctx_stream(llf_ctx *ctx, void **stream) {
   return LLF_OK;
 }
 
+int llf_ctx_share_gpu(llf_ctx *ctx, int on) {
+  if (!ctx) return LLF_ERR_ARG;
+  ctx->shares_gpu = on != 0;
+  return llf_ok(ctx);
+}
+
 int llf_profile_enable(llf_ctx *ctx, int on) {
   if (!ctx) return LLF_ERR_ARG;
   prof_resolve(ctx);

@@ -50,7 +50,7 @@ struct llf_ctx {
   unsigned *h_status = nullptr;   // pinned host mirror of both
   int num_sms = 0;
   bool profiling = false;
-  bool shares_gpu = false;        // other contexts' kernels run beside this one's (a server's contexts)
+  bool shares_gpu = false;        // other contexts' kernels run beside this one's (llf_ctx_share_gpu)
   long long launches = 0;
   long long allocs = 0;           // device allocations made through the context
   std::vector<ProfPending> pending;

@@ -33,10 +33,6 @@ struct Done {
   std::vector<double> x;   // the solution, fixed entries kept
 };
 
-// Marks a context whose kernels run beside those of other contexts (a
-// server's): its solves keep to launches that leave the SMs to others.
-void share_gpu(llf_ctx *ctx);
-
 // Set up the CG of K x = b (fixed entries of x0 prescribed; host arrays of
 // K's DoF count) on ctx's stream, with a local preconditioner (none, Jacobi,
 // block Jacobi).  Synchronises ctx's stream.  K must outlive the system.

@@ -176,7 +176,7 @@ void destroy_job_objects(llf_ctx *ctx, Job &j) {
 void prep_main(llf_server *s) {
   llf_ctx *ctx = nullptr;
   int crc = llf_ctx_create(s->device, &ctx);
-  if (crc == LLF_OK) llf_engine::share_gpu(ctx);
+  if (crc == LLF_OK) llf_ctx_share_gpu(ctx, 1);
   for (;;) {
     std::unique_ptr<Request> req = take_request(s);
     if (!req) break;
@@ -227,7 +227,7 @@ void engine_main(llf_server *s) {
   llf_ctx *ctx = nullptr;
   llf_engine::Engine *eng = nullptr;
   int crc = llf_ctx_create(s->device, &ctx);
-  if (crc == LLF_OK) llf_engine::share_gpu(ctx);
+  if (crc == LLF_OK) llf_ctx_share_gpu(ctx, 1);
   if (crc == LLF_OK) crc = llf_engine::create(ctx, s->max_systems, (int64_t)1 << 20, &eng);
   std::string cerr = crc == LLF_OK ? "" : (ctx ? llf_last_error(ctx) : "engine has no CUDA context");
   std::deque<std::unique_ptr<Job>> pending;
@@ -334,7 +334,7 @@ void engine_main(llf_server *s) {
 void worker_main(llf_server *s) {
   llf_ctx *ctx = nullptr;
   int crc = llf_ctx_create(s->device, &ctx);
-  if (crc == LLF_OK) llf_engine::share_gpu(ctx);
+  if (crc == LLF_OK) llf_ctx_share_gpu(ctx, 1);
   for (;;) {
     std::unique_ptr<Request> req = take_request(s);
     if (!req) break;

@@ -3075,8 +3075,6 @@ __global__ void __launch_bounds__(CG_THREADS) k_eng_update(EngTab T, unsigned *c
 
 namespace llf_engine {
 
-void share_gpu(llf_ctx *ctx) { ctx->shares_gpu = true; }
-
 struct System {
   const llf_matrix *K = nullptr;
   int P = 1, precond = 0;

@@ -78,3 +78,16 @@ def test_meeting_points_only_where_the_loop_may_run(llf):
         solve()
         count.append(ctx.allocs() - a)
     assert count[0] == count[1] + 1
+
+
+def test_contexts_that_share_the_gpu_take_the_launches(llf):
+    ctx, solve = _solve(llf, llf.structured_box_mesh(n=12, order=1), "Solid")
+    want = solve()
+    ctx.share_gpu()
+    try:
+        assert _forms(ctx, solve) == {LAUNCHES}
+        got = solve()
+    finally:
+        ctx.share_gpu(False)
+    assert _forms(ctx, solve) == {HALO}
+    assert np.array_equal(got[0], want[0]) and got[1:] == want[1:]
