@@ -5,8 +5,8 @@
 // P*nadj[nptr[B] + k/P] + k%P.  The assembled operators are symmetric bit
 // for bit (element blocks are mirrored, per-entry sums run over the same
 // elements in the same order), so y = A x is computed column-wise as
-// y_c = sum_k A[row_k, c] x[row_k] — one warp per column, no atomics, a fixed
-// shuffle tree per column: results are identical run to run.
+// y_c = sum_k A[row_k, c] x[row_k] — SPMV_G lanes per column node, no atomics,
+// a fixed shuffle tree per column: results are identical run to run.
 //
 // PCG restates IterativeSolvers.cg (0.9.4) as called by solveDisplacement /
 // solveTemperature / solveField (src/linear.jl:3827-3833): x0 = 0 on the
@@ -45,9 +45,10 @@ constexpr int CHUNK = 768;  // most DoFs per reduction chunk
 constexpr int CHUNK_PER_THREAD = CHUNK / CG_THREADS;  // a chunk's DoFs per thread of its block
 static_assert(CHUNK % CG_THREADS == 0, "a chunk is whole rounds of a block");
 // DoFs per chunk of a system of n DoFs (a multiple of every pdim: chunks hold
-// whole nodes): small systems are cut into chunks for every SM, down to 192
-// DoFs, whose sums still cost less than their products.  A function of the
-// system alone, so that its sums do not depend on what else is in a batch.
+// whole nodes): small systems are cut into 148 chunks, for nearly all of the
+// 152 SMs, down to 192 DoFs, whose sums still cost less than their products.
+// A function of the system alone, so that its sums depend neither on what else
+// is in a batch nor on the device.
 constexpr int64_t CHUNKS_WANTED = 148;
 __host__ __device__ inline int chunk_dofs(int64_t n) {
   const int64_t c = ((n + CHUNKS_WANTED - 1) / CHUNKS_WANTED + 5) / 6 * 6;
@@ -1235,7 +1236,10 @@ k_cg_resident(Seg S, const double *__restrict__ nz, const int64_t *__restrict__ 
         }
         z[k] = fx[k] ? 0.0 : zi;
         sC[i] = z[k];
-        // every chunk has read the z of the iteration before (its u.c has come)
+        // every chunk has read the z of the iteration before: what it read is
+        // part of the u.c that it sent and that alpha, and so this z, was formed
+        // with (a z that it could read early would depend on itself; where the
+        // u.c does not depend on a value, for rows of fixed DoFs, no result does)
         if (HALO) zg[b + i] = z[k];
       }
     }
@@ -2531,6 +2535,9 @@ int pcg_outcome(llf_ctx *ctx, int nseg, const SegState *hst, int64_t *iters, dou
 // array until the process exits.  Regions are 256-byte aligned.
 constexpr int64_t NA_N = LLF_NOALLOC_MAX_DOFS;
 constexpr int64_t NA_CH = (NA_N + CHUNK - 1) / CHUNK;
+// chunk_count(n) for n <= NA_N: at most CHUNKS_WANTED chunks of fewer than
+// CHUNK DoFs, else whole ones
+static_assert(NA_CH >= CHUNKS_WANTED, "the chunk arrays hold the chunks of every system of up to NA_N DoFs");
 constexpr size_t na_round(size_t b) { return (b + 255) / 256 * 256; }
 constexpr size_t NA_VEC = na_round(sizeof(double) * NA_N);
 constexpr size_t NA_OFF_PINV = 5 * NA_VEC;                       // r, z, u, c, xw
