@@ -8,12 +8,13 @@
 //   k_elem_packed elements of up to 384 node pairs: as many per CTA as fill
 //                 its threads (one hex27, eight hex8), after k_affine_coeff
 //                 has formed the affine ones' coefficients;
-//   k_elem_affine larger elements of meshes whose elements are all affine:
-//                 one CTA per element at a time (persistent), the node-pair
-//                 blocks formed from the reference pair tables into a
-//                 shared-memory image of the element matrix, which one bulk
-//                 store writes out;
-//   k_elem_fp64   other meshes: one CTA per element at a time, element node
+//   k_elem_affine conduction of tet35, mass of tet35 and hex64 on meshes whose
+//                 elements are all affine (larger elements whose matrix and
+//                 table fit in shared memory): one CTA per element at a time
+//                 (persistent), the entries formed from the reference pair
+//                 tables into a shared-memory image of the element matrix,
+//                 which one bulk store writes out;
+//   k_elem_fp64   other elements: one CTA per element at a time, element node
 //                 coordinates gathered into shared memory, the reference
 //                 shape gradients staged in shared memory for the CTA's
 //                 lifetime (read from global memory for elements whose tables
@@ -425,9 +426,9 @@ k_elem_fp64(ElemArgs A) {
   }
 }
 
-// Affine-element kernel with staged stores, for meshes whose elements are
-// all affine (k_affine_geometry counted no other): one CTA per element at a
-// time (grid-stride, persistent).  The pair table (the parts of R_ab, or
+// Affine-element kernel with staged stores for conduction and mass in 3D, on
+// meshes whose elements are all affine (k_affine_geometry counted no other):
+// one CTA per element at a time (grid-stride, persistent).  The pair table (the parts of R_ab, or
 // Mref_ab) is copied into shared memory once per CTA by a bulk copy
 // (cp.async.bulk completing on an mbarrier; a bounded wait).  Each element
 // matrix is built in a shared-memory image of its Kf run (the same layout,
@@ -462,12 +463,11 @@ __device__ __forceinline__ bool bar_wait(uint64_t *bar, unsigned parity) {
 
 constexpr int AFFK_MAX_THREADS = 256;
 
-template <int KIND, int DIM>
+template <int KIND>
 __global__ void __launch_bounds__(AFFK_MAX_THREADS)
 k_elem_affine(ElemArgs A, int tab_n) {
   extern __shared__ __align__(128) double smem_a[];
-  constexpr int BS = (KIND == KIND_ELASTIC) ? DIM * DIM : 1;
-  constexpr int P = (KIND == KIND_ELASTIC) ? DIM : 1;
+  static_assert(KIND != KIND_ELASTIC, "no elastic element beyond k_elem_packed's fits");
   const int64_t kelems = (int64_t)A.npe * A.colstride;
   const unsigned ke_bytes = (unsigned)(kelems * 8);
   double *sKe = smem_a;
@@ -504,22 +504,21 @@ k_elem_affine(ElemArgs A, int tab_n) {
     const int mat = A.emat ? A.emat[e] : 0;
     if (mat < 0) continue;  // uniform across the CTA
     const double c1 = A.c1[mat];
-    const double c2 = (KIND == KIND_ELASTIC) ? A.c2[mat] : 0.0;
     const bool aligned = A.aflag[e] == 2;
     if ((int)(threadIdx.x >> 5) == (int)((blockIdx.x + iter) % (unsigned)nwarps)) {
       const int lane = threadIdx.x & 31;
       if (aligned)
-        affine_stage_aligned<DIM>(A.ageo + (size_t)e * 10, c1, c2, sAff, A.status, lane);
+        affine_stage_aligned<3>(A.ageo + (size_t)e * 10, c1, 0.0, sAff, A.status, lane);
       else
-        affine_stage<DIM>(A.ageo + (size_t)e * 10, c1, c2, sAff, A.status, lane);
+        affine_stage<3>(A.ageo + (size_t)e * 10, c1, 0.0, sAff, A.status, lane);
     }
     // the previous element's store has read the image
     if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     __syncthreads();
     if (aligned)
-      affine_pairs<KIND, DIM, P, BS, true, true>(A, sAff, sKe, sTab, sTab);
+      affine_pairs<KIND, 3, 1, 1, true, true>(A, sAff, sKe, sTab, sTab);
     else
-      affine_pairs<KIND, DIM, P, BS, false, true>(A, sAff, sKe, sTab, sTab);
+      affine_pairs<KIND, 3, 1, 1, false, true>(A, sAff, sKe, sTab, sTab);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1027,10 +1026,11 @@ int launch_elem(llf_ctx *ctx, const ElemArgs &a, size_t smem, unsigned grid) {
 }
 
 // The staged affine kernel when every element is affine and two CTAs fit on
-// an SM; *done = false
-// otherwise.  Threads: the node pairs in as few rounds of at most 256 as
-// possible, rounded up to whole warps (hex27: 378 pairs, 2 rounds of 192).
-template <int KIND, int DIM>
+// an SM (with the conduction table, tet35's 630 node pairs do and hex64's 2080
+// do not); *done = false otherwise.  Threads: the node pairs in as few rounds
+// of at most 256 as possible, rounded up to whole warps (tet35: 3 rounds of
+// 224).
+template <int KIND>
 int run_elem_affine(llf_ctx *ctx, const ElemArgs &a, bool *done) {
   *done = false;
   const int npairs = a.npairs;
@@ -1040,7 +1040,7 @@ int run_elem_affine(llf_ctx *ctx, const ElemArgs &a, bool *done) {
   if (smem > 110 * 1024) return LLF_OK;
   const int rounds = (npairs + AFFK_MAX_THREADS - 1) / AFFK_MAX_THREADS;
   const int threads = ((npairs + rounds - 1) / rounds + 31) / 32 * 32;
-  auto fn = k_elem_affine<KIND, DIM>;
+  auto fn = k_elem_affine<KIND>;
   if (smem > 48 * 1024)
     LLF_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
@@ -1124,7 +1124,8 @@ int run_elem(llf_ctx *ctx, ElemArgs a) {
   {
     bool done = false;
     int rc = run_elem_packed<KIND, DIM>(ctx, a, &done);
-    if (rc == LLF_OK && !done) rc = run_elem_affine<KIND, DIM>(ctx, a, &done);
+    if constexpr (KIND != KIND_ELASTIC && DIM == 3)
+      if (rc == LLF_OK && !done) rc = run_elem_affine<KIND>(ctx, a, &done);
     if (rc != LLF_OK || done) return rc;
   }
   const int npe = a.npe, nip = a.nip;

@@ -587,10 +587,16 @@ int run_colgather(llf_ctx *ctx, llf_pattern *pat, const int64_t *n2e_ptr, const 
 #define LLF_WIDE(NT, R) \
   return launch_wide<P, BV, T, NT, R>(ctx, pat, n2e_ptr, n2e, pos, npe, Kf, cs, init, nz, cnt, B0, nB, sp, first_marked)
   // longer: a CTA per column node, the rounds that use its threads and its
-  // registers best (measured with 64 to 576 threads)
-  if (nv <= 160 * 2) LLF_WIDE(160, 2);
-  if (nv <= 192 * 3) LLF_WIDE(192, 3);
-  if (nv <= 288 * 4) LLF_WIDE(288, 4);
+  // registers best (measured with 64 to 576 threads).  Each is instantiated for
+  // the columns that come to it: with two components scalars of hex64 and
+  // hex125 (128 and 250 values), with three scalars (tet35 105 to hex125 375)
+  // and blocks (tet35 315, hex64 576, hex125 1125)
+  if constexpr (P == 3 || (P == 2 && !BV))
+    if (nv <= 160 * 2) LLF_WIDE(160, 2);
+  if constexpr (P == 3)
+    if (nv <= 192 * 3) LLF_WIDE(192, 3);
+  if constexpr (P == 3 && BV)
+    if (nv <= 288 * 4) LLF_WIDE(288, 4);
   return llf_fail(ctx, LLF_ERR_LIMIT, "an element has too many nodes for the gather");
 #undef LLF_WIDE
 }
