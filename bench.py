@@ -48,11 +48,11 @@ def workload_name(n):
     return f"hooke3d-unit-cube-hex27-{n}x{n}x{n}"
 # ncu DRAM bytes (read + write) of one FP64 assembly of hex27 16^3 (19,320,201
 # structural nnz): k_affine_geometry 1.3 MB, k_affine_coeff 0.4 MB, k_elem_packed
-# 152.9 MB, k_colgather 338.2 MB (into the kept layout 420.2 MB), k_compact 417.5 MB
+# 152.9 MB, k_colgather 309.9 MB (into the kept layout 420.2 MB), k_compact 417.5 MB
 NNZ_16CUBE = 19320201
 KERNEL_DRAM_BYTES_16CUBE = {"k_affine_geometry": 1.324032e6, "k_affine_coeff": 0.353536e6,
                             "k_elem_packed": (1.539712 + 151.400576) * 1e6,
-                            "k_colgather": (224.209664 + 114.00704) * 1e6, "k_compact": (165.33248 + 252.210688) * 1e6,
+                            "k_colgather": (170.503424 + 83.71328 + 55.601664 + 0.082688) * 1e6, "k_compact": (165.33248 + 252.210688) * 1e6,
                             # the gather compacting into the pattern's kept stored layout (both launches)
                             "k_colgather_layout": (179.8208 + 177.19424 + 58.180224 + 5.301632) * 1e6}
 

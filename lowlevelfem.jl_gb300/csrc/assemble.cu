@@ -1073,15 +1073,16 @@ int packed_count(int npairs, size_t per_elem) {
 }
 
 // k_elem_packed for elements of at most PACK_PAIRS node pairs; *done = false
-// otherwise (from hex64's 2080 pairs on a thread has many pairs either way).  A mesh that would leave SMs idle puts
-// fewer elements in a CTA.
+// otherwise (from hex64's 2080 pairs on a thread has many pairs either way).  A
+// mesh that would leave SMs idle puts fewer elements in a CTA.
 template <int KIND, int DIM>
 int run_elem_packed(llf_ctx *ctx, const ElemArgs &a, bool *done) {
   *done = false;
   const bool quad = !a.all_affine || !a.aflag;
   // The mass matrix by points has one operation per pair and point and little
-  // shared memory; from 144 pairs on, an element per small CTA is as good
-  // (27,000 curved hex27: 1.012 against 1.038 ms here).
+  // shared memory; beyond 144 pairs an element per small CTA is as good on the
+  // whole (ms there and here: 14,400 curved quad25 0.340 and 0.397, 27,000 hex27
+  // 1.014 and 1.038, 10,368 tet20 0.595 and 0.556).
   if (a.npairs > (KIND == KIND_MASS && quad ? 144 : PACK_PAIRS)) return LLF_OK;
   const int gsw = (KIND == KIND_MASS) ? 1 : DIM;
   const size_t per_elem = sizeof(double) * ((size_t)a.npe * a.colstride + 2 * AFF_PACK<KIND, DIM> + 1 +

@@ -300,7 +300,9 @@ __device__ __forceinline__ void tile_order(const int64_t *__restrict__ nptr, int
 // KEPT of one or two components is left without: hex8 conduction, 357,911
 // nodes, 38 us and 41 with it.
 // Structural values, us: hex27 40^3 583, hex64 14^3 229, hex125 8^3 273, tet10
-// 24^3 86; KEPT 667, 328, 353, 99.  In node order 128 threads a block, so that
+// 24^3 86; KEPT 667, 328, 353, 99 (it takes two positions of a lane at a time
+// for rows of every length: four suited hex64, 259, and not tet10 16^3, 45
+// instead of 38; a matrix multiplied often gets its structural values).  In node order 128 threads a block, so that
 // more rows are under way beside a long one: 256 threads took 1.04 to 1.09
 // times as long for rows of three components.
 template <int P, bool KEPT, bool SORT, bool LONG>
